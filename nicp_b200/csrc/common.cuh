@@ -372,86 +372,6 @@ __device__ inline void d_eig3(const double *A, double *lam, double *U) {
   for (int r = 0; r < 3; r++) { U[r * 3 + 0] = v0[r]; U[r * 3 + 1] = v1[r]; U[r * 3 + 2] = v2[r]; }
 }
 
-// Solve A x = b for a symmetric 6x6 A given by its lower triangle: LDL^T
-// with symmetric diagonal pivoting.  Every index is a compile-time constant
-// (the pivot's row and column swaps are predicated per candidate), so the
-// factor stays in registers.
-__device__ __forceinline__ void d_ldlt_solve6(const double *A, const double *b, double *x) {
-  double M[6][6];
-  int perm[6];
-#pragma unroll
-  for (int i = 0; i < 6; i++) {
-    perm[i] = i;
-#pragma unroll
-    for (int j = 0; j < 6; j++) M[i][j] = (i >= j) ? A[i * 6 + j] : A[j * 6 + i];
-  }
-  double d[6];
-#pragma unroll
-  for (int k = 0; k < 6; k++) {
-    int piv = k;
-    double best = fabs(M[k][k]);
-#pragma unroll
-    for (int i = k + 1; i < 6; i++)
-      if (fabs(M[i][i]) > best) { best = fabs(M[i][i]); piv = i; }
-#pragma unroll
-    for (int i = k + 1; i < 6; i++) {
-      const bool sw = piv == i;
-#pragma unroll
-      for (int j = 0; j < 6; j++) {
-        const double a = M[k][j], c = M[i][j];
-        M[k][j] = sw ? c : a;
-        M[i][j] = sw ? a : c;
-      }
-#pragma unroll
-      for (int r = 0; r < 6; r++) {
-        const double a = M[r][k], c = M[r][i];
-        M[r][k] = sw ? c : a;
-        M[r][i] = sw ? a : c;
-      }
-      const int a = perm[k], c = perm[i];
-      perm[k] = sw ? c : a;
-      perm[i] = sw ? a : c;
-    }
-    d[k] = M[k][k];
-    double col[6];
-#pragma unroll
-    for (int i = k + 1; i < 6; i++) col[i] = M[i][k];
-#pragma unroll
-    for (int i = k + 1; i < 6; i++) M[i][k] = col[i] / d[k];
-#pragma unroll
-    for (int i = k + 1; i < 6; i++)
-#pragma unroll
-      for (int j = k + 1; j <= i; j++) {
-        M[i][j] = M[i][j] - M[i][k] * col[j];
-        M[j][i] = M[i][j];
-      }
-  }
-  double y[6];
-#pragma unroll
-  for (int i = 0; i < 6; i++) {
-    y[i] = b[0];
-#pragma unroll
-    for (int j = 1; j < 6; j++) y[i] = perm[i] == j ? b[j] : y[i];
-  }
-#pragma unroll
-  for (int i = 0; i < 6; i++)
-#pragma unroll
-    for (int j = 0; j < i; j++) y[i] = y[i] - M[i][j] * y[j];
-#pragma unroll
-  for (int i = 0; i < 6; i++) y[i] = y[i] / d[i];
-#pragma unroll
-  for (int i = 5; i >= 0; i--)
-#pragma unroll
-    for (int j = i + 1; j < 6; j++) y[i] = y[i] - M[j][i] * y[j];
-#pragma unroll
-  for (int j = 0; j < 6; j++) {  // x[perm[i]] = y[i]
-    double v = y[0];
-#pragma unroll
-    for (int i = 1; i < 6; i++) v = perm[i] == j ? y[i] : v;
-    x[j] = v;
-  }
-}
-
 // bm_se3.h:10-52 in FP64.
 __device__ inline void d_v2t(const double *x, double *T) {
   double qx = x[3], qy = x[4], qz = x[5];
@@ -469,8 +389,8 @@ __device__ inline void d_v2t(const double *x, double *T) {
   T[12] = 0; T[13] = 0; T[14] = 0; T[15] = 1;
 }
 
-// Shepperd's method, normalised, vector part with w >= 0.
-__device__ inline void d_t2v(const double *T, double *x) {
+// Shepperd's method: the quaternion q = (x, y, z, w) of T's rotation and its norm n.
+__device__ inline void d_quaternion(const double *T, double *q, double &n) {
   double R[3][3];
 #pragma unroll
   for (int i = 0; i < 3; i++)
@@ -515,11 +435,8 @@ __device__ inline void d_t2v(const double *T, double *x) {
       qy = (R[1][2] + R[2][1]) * s;
     }
   }
-  double n = sqrt(qx * qx + qy * qy + qz * qz + qw * qw);
-  qx /= n; qy /= n; qz /= n; qw /= n;
-  if (qw < 0) { qx = -qx; qy = -qy; qz = -qz; }
-  x[0] = T[3]; x[1] = T[7]; x[2] = T[11];
-  x[3] = qx; x[4] = qy; x[5] = qz;
+  n = sqrt(qx * qx + qy * qy + qz * qz + qw * qw);
+  q[0] = qx; q[1] = qy; q[2] = qz; q[3] = qw;
 }
 
 __device__ inline void d_mm4(const double *A, const double *B, double *C) {

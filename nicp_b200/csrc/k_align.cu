@@ -1060,108 +1060,287 @@ __global__ void k_init_pairs(const PairDev *__restrict__ pairs, int npairs, cons
   for (int k = 0; k < 12; k++) st->Tgate_used[k] = st->Tgate[k];
 }
 
+// ---- the 6x6 solve and the pose update, by one warp.
+// The chain of divisions, square roots and 4x4 products is short on work and
+// long on latency, so a lane owns an entry, independent divisions run in
+// different lanes and code stays short.  Every entry is formed by the same
+// operations in the same order as one thread would form it.
+struct SolveScratch {
+  double L[36];  // factor: row = unknown, column = step
+  double x[6];
+  double T[16], invT[16], Tstart[16], off[16], dT[16], A[16], B[16];
+};
+
+__device__ __forceinline__ int nibble(unsigned w, int i) { return (int)((w >> (4 * i)) & 15u); }
+// Lane that owns the unordered entry (i, j): the lower triangle row by row.
+__device__ __forceinline__ int tri(int i, int j) {
+  const int hi = max(i, j), lo = min(i, j);
+  return hi * (hi + 1) / 2 + lo;
+}
+
+// M x = b by LDL^T with symmetric diagonal pivoting (Golub & Van Loan 4.2);
+// lane tri(i, j) < 21 holds m = M_ij, lane i < 6 holds rhs = b_i; x to
+// s.x.  Unknowns are never moved: `perm` (position -> unknown) and `pos`
+// (unknown -> position) hold the order, six packed nibbles each, uniform in
+// the warp.  A step is a maximum over the remaining diagonal (one integer
+// reduction), three exchanges, one division and one FMA.
+__device__ __forceinline__ void warp_ldlt_solve6(double m, double rhs, SolveScratch &s, int lane) {
+  const unsigned kAll = 0xffffffffu;
+  unsigned perm = 0x543210u, pos = 0x543210u;
+  const int a = lane >= 21 ? 6 : lane >= 15 ? 5 : lane >= 10 ? 4 : lane >= 6 ? 3 : lane >= 3 ? 2 : lane >= 1 ? 1 : 0;
+  const int b = a == 6 ? 6 : lane - a * (a + 1) / 2;
+  double dpos = 1.0;  // lane i < 6: the pivot of position i
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    if (k < 5) {
+      // lane = position: the first of the largest remaining diagonal entries
+      const int u = nibble(perm, lane < 6 ? lane : 5);
+      const double dl = fabs(__shfl_sync(kAll, m, tri(u, u)));
+      const bool in = lane >= k && lane < 6;
+      const unsigned nan = __ballot_sync(kAll, in && dl != dl);
+      const unsigned hi = in && dl == dl ? (unsigned)__double2hiint(dl) : 0u;
+      const unsigned top = __reduce_max_sync(kAll, hi);
+      unsigned who = __ballot_sync(kAll, in && dl == dl && hi == top);
+      if (__popc(who) > 1) {  // equal upper words: the lower ones decide
+        const bool cand = (who >> lane) & 1u;
+        const unsigned lo = cand ? (unsigned)__double2loint(dl) : 0u;
+        const unsigned top_lo = __reduce_max_sync(kAll, lo);
+        who = __ballot_sync(kAll, cand && lo == top_lo);
+      }
+      // a NaN never beats another entry and is never beaten in its own place
+      const int piv = ((nan >> k) & 1u) || !who ? k : __ffs(who) - 1;
+      const unsigned uk = nibble(perm, k), up = nibble(perm, piv);
+      perm ^= ((uk ^ up) << (4 * k)) | ((uk ^ up) << (4 * piv));
+      if (uk != up) pos ^= ((unsigned)(k ^ piv) << (4 * uk)) | ((unsigned)(k ^ piv) << (4 * up));
+    }
+    const int u = nibble(perm, k);
+    const double d = __shfl_sync(kAll, m, tri(u, u));
+    if (lane == k) dpos = d;
+    if (k < 5) {
+      const int pa = nibble(pos, a), pb = nibble(pos, b);
+      const int hi = pa >= pb ? a : b, lo = pa >= pb ? b : a;
+      const double ch = __shfl_sync(kAll, m, tri(hi, u)), cl = __shfl_sync(kAll, m, tri(lo, u));
+      const bool left = a < 6 && pa > k && pb > k;
+      const double l = (left ? ch : d) / d;  // (a lane that is done divides d by itself)
+      if (left) m = m - l * cl;
+      if (left && a == b) s.L[a * 6 + k] = l;
+    }
+  }
+  __syncwarp();
+  // L y = b, lane = unknown
+  const int row = lane < 6 ? lane : 5, at = nibble(pos, row);
+  double y = rhs;
+#pragma unroll
+  for (int j = 0; j < 5; j++) {
+    const double yj = __shfl_sync(kAll, y, nibble(perm, j));
+    if (at > j) y = y - s.L[row * 6 + j] * yj;
+  }
+  y = y / __shfl_sync(kAll, dpos, at);
+  // L^T x = y, every lane the same, by position
+  double x[6], l[6][6];
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+    x[i] = __shfl_sync(kAll, y, nibble(perm, i));
+#pragma unroll
+    for (int j = 0; j < i; j++) l[i][j] = s.L[nibble(perm, i) * 6 + j];
+  }
+#pragma unroll
+  for (int i = 4; i >= 0; i--)
+#pragma unroll
+    for (int j = i + 1; j < 6; j++) x[i] = x[i] - l[j][i] * x[j];
+  if (lane == 0)
+#pragma unroll
+    for (int i = 0; i < 6; i++) s.x[nibble(perm, i)] = x[i];
+  __syncwarp();
+}
+
+// C = A B (rows 0..3), lane < 16 an entry; C is another array than A and B.
+__device__ __forceinline__ void warp_mm4(const double *A, const double *B, double *C, int lane) {
+  if (lane < 16) {
+    const double *r = A + (lane & 12), *c = B + (lane & 3);
+    C[lane] = r[0] * c[0] + r[1] * c[4] + r[2] * c[8] + r[3] * c[12];
+  }
+  __syncwarp();
+}
+// R = T^-1 of an isometry, R another array than T.
+__device__ __forceinline__ void warp_iso_inverse(const double *T, double *R, int lane) {
+  if (lane < 16) {
+    const int i = lane >> 2, j = lane & 3;
+    double v = lane == 15 ? 1.0 : 0.0;
+    if (i < 3) v = j < 3 ? T[j * 4 + i] : -(T[i] * T[3] + T[4 + i] * T[7] + T[8 + i] * T[11]);
+    R[lane] = v;
+  }
+  __syncwarp();
+}
+// v2t by every lane; lane 0 stores.
+__device__ __forceinline__ void warp_v2t(const double *x, double *T, int lane) {
+  double t[16];
+  d_v2t(x, t);
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < 16; k++) T[k] = t[k];
+  __syncwarp();
+}
+// t2v by every lane, the quaternion's four divisions in four lanes.
+__device__ __forceinline__ void warp_t2v(const double *T, double *x, int lane) {
+  double q[4], n;
+  d_quaternion(T, q, n);
+  const double v = (lane == 0 ? q[0] : lane == 1 ? q[1] : lane == 2 ? q[2] : q[3]) / n;
+  const bool flip = __shfl_sync(0xffffffffu, v, 3) < 0;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const double c = __shfl_sync(0xffffffffu, v, k);
+    x[3 + k] = flip ? -c : c;
+    x[k] = T[4 * k + 3];
+  }
+}
+
+// ---- the sum of a pair's tile partials: kSumGroups warps take the tiles
+// t = g, g + kSumGroups, ... each, then the groups are added; a fixed order,
+// whatever the batch.  (Four groups, as before, left one SM with 75 partials
+// a thread at 640x480: 4800 cycles of a 12500-cycle launch; 16 groups have
+// all their loads in flight at once.)
+constexpr int kSumGroups = 16, kSumThreads = 32 * kSumGroups;
+
+__device__ __forceinline__ void sum_tile_partials(const double *src, int nt, bool f32, double (*part)[32]) {
+  constexpr int kAhead = 8;
+  const int e = threadIdx.x & 31, g = threadIdx.x >> 5;
+  src += e;
+  double s = 0.0;
+  float s32 = 0.0f;
+  for (int t = g; t < nt; t += kSumGroups * kAhead) {
+    double v[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; q++) {
+      const int u = t + kSumGroups * q;
+      v[q] = u < nt ? __ldcg(src + (size_t)u * kPartialWords) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < kAhead; q++) {
+      if (f32) s32 += (float)v[q];  // precision study: the same order, in FP32
+      else s += v[q];
+    }
+  }
+  part[g][e] = f32 ? (double)s32 : s;
+  __syncthreads();
+}
+__device__ __forceinline__ double sum_groups(double (*part)[32], bool f32, int e) {
+  if (f32) {
+    float t = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kSumGroups; k++) t += (float)part[k][e];
+    return (double)t;
+  }
+  double q[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    q[k] = ((part[4 * k][e] + part[4 * k + 1][e]) + part[4 * k + 2][e]) + part[4 * k + 3][e];
+  return (q[0] + q[1]) + (q[2] + q[3]);
+}
+
 // mode: bit0 last inner iteration of the outer loop, bit1 reduce only (no
 // pose update: Linearizer results of a list pass), bit2 statistics pass
 // (reduce into Hstat only), kSolveCrossF32 sum the tile partials in FP32.
-__global__ void __launch_bounds__(128) k_solve(const PairDev *__restrict__ pairs, int npairs, float lambda, int mode,
-                                              double early_eps, int ignore_done) {
-  __shared__ double part[4][32];
-  __shared__ double tot[32];
+// The other warps only help to add the partials up; one of them writes the
+// sums out while warp 0 solves.
+__global__ void __launch_bounds__(kSumThreads) k_solve(const PairDev *__restrict__ pairs, int npairs, float lambda,
+                                                      int mode, double early_eps, int ignore_done) {
+  __shared__ double part[kSumGroups][32];
+  __shared__ SolveScratch sc;
   const PairDev &pd = pairs[blockIdx.x];
   PairState *st = pd.state;
+  const double *src = pd.partials;
+  const int P = pd.rows * pd.cols;
+  const int nt = (P + kCorrTilePixels - 1) / kCorrTilePixels;
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  if (g >= 2 && threadIdx.x < 64 + 48) {
+    const int q = threadIdx.x - 64;
+    const double *from = q < 16 ? st->invT : q < 32 ? st->Tstart : st->ref_offset;
+    double *to = q < 16 ? sc.invT : q < 32 ? sc.Tstart : sc.off;
+    to[q & 15] = from[q & 15];
+  }
+  const int iterations = st->iterations;
+  const float gate_used = lane < 12 ? st->Tgate[lane] : 0.0f;
+  double K[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    if (lane < 12) K[k] = (double)pd.K[(lane >> 2) * 3 + k];
   if (st->done && !ignore_done) return;
-  int P = pd.rows * pd.cols;
-  int nt = (P + kCorrTilePixels - 1) / kCorrTilePixels;
-  int e = threadIdx.x & 31, g = threadIdx.x >> 5;
-  if (mode & kSolveCrossF32) {
-    // precision study: the same fixed order, in FP32
-    float s = 0.0f;
-    for (int t = g; t < nt; t += 4) s += (float)pd.partials[(size_t)t * kPartialWords + e];
-    part[g][e] = (double)s;
-    __syncthreads();
-    if (threadIdx.x < 32)
-      tot[e] = (double)((((float)part[0][e] + (float)part[1][e]) + (float)part[2][e]) + (float)part[3][e]);
-  } else {
-    // the fixed order t = g, g + 4, ..., with eight loads in flight
-    double s = 0.0;
-    int t = g;
-    for (; t + 28 < nt; t += 32) {
-      double v[8];
+  sum_tile_partials(src, nt, (mode & kSolveCrossF32) != 0, part);
+  const double tot = sum_groups(part, (mode & kSolveCrossF32) != 0, lane);
+  // H's entry (i, j) in the sums: 0..5 Htt lower, 6..14 Htr row by row, 15..20 Hrr lower
+  auto element = [](int i, int j) {
+    const int hi = max(i, j), lo = min(i, j);
+    return hi < 3 ? tri(hi, lo) : lo >= 3 ? 15 + tri(hi - 3, lo - 3) : 6 + lo * 3 + hi - 3;
+  };
+  if (g == 1) {
+    double *H = (mode & 4) ? st->Hstat : st->H;
 #pragma unroll
-      for (int q = 0; q < 8; q++) v[q] = pd.partials[(size_t)(t + 4 * q) * kPartialWords + e];
-#pragma unroll
-      for (int q = 0; q < 8; q++) s += v[q];
+    for (int r = 0; r < 2; r++) {
+      const int k = min(lane + 32 * r, 35), i = k / 6, j = k - 6 * i;
+      const double h = __shfl_sync(0xffffffffu, tot, element(i, j));
+      if (lane + 32 * r < 36) H[k] = h;
     }
-    for (; t < nt; t += 4) s += pd.partials[(size_t)t * kPartialWords + e];
-    part[g][e] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) tot[e] = ((part[0][e] + part[1][e]) + part[2][e]) + part[3][e];
-  }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  // (every index below is a compile-time constant: H, b and A stay in registers)
-  constexpr int li[6][2] = {{0, 0}, {1, 0}, {1, 1}, {2, 0}, {2, 1}, {2, 2}};
-  double H[36], b[6];
-#pragma unroll
-  for (int q = 0; q < 6; q++) {
-    const int i = li[q][0], j = li[q][1];
-    H[i * 6 + j] = H[j * 6 + i] = tot[q];
-    H[(3 + i) * 6 + 3 + j] = H[(3 + j) * 6 + 3 + i] = tot[15 + q];
-  }
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-      H[i * 6 + 3 + j] = tot[6 + i * 3 + j];
-      H[(3 + j) * 6 + i] = tot[6 + i * 3 + j];
+    if (!(mode & 4)) {
+      if (lane >= 21 && lane < 27) st->b[lane - 21] = tot;
+      if (lane == 27) st->error = (float)tot;
+      if (lane == 28) st->inliers = (int)tot;
+      if (lane == 29) st->candidates = (int)tot;
+      if (lane == 30) st->num_corr = (int)tot;
     }
-#pragma unroll
-  for (int i = 0; i < 3; i++) { b[i] = tot[21 + i]; b[3 + i] = tot[24 + i]; }
-  if (mode & 4) {
-#pragma unroll
-    for (int k = 0; k < 36; k++) st->Hstat[k] = H[k];
+  }
+  if (g != 0 || (mode & 6)) return;
+  // H += lambda I; dx = H^-1 (-b); invT = v2t(dx) invT  (alignerprojective.cpp:72-95)
+  {
+    const int a = lane >= 15 ? 5 : lane >= 10 ? 4 : lane >= 6 ? 3 : lane >= 3 ? 2 : lane >= 1 ? 1 : 0;
+    const int b = min(lane - a * (a + 1) / 2, 5);
+    double m = __shfl_sync(0xffffffffu, tot, element(a, b));
+    if (a == b) m = m + (double)lambda;
+    const double rhs = -__shfl_sync(0xffffffffu, tot, 21 + (lane < 6 ? lane : 5));
+    warp_ldlt_solve6(m, rhs, sc, lane);
+  }
+  warp_v2t(sc.x, sc.dT, lane);
+  warp_mm4(sc.dT, sc.invT, sc.A, lane);  // the new invT
+  if (lane >= 12 && lane < 16) sc.A[lane] = lane == 15 ? 1.0 : 0.0;
+  __syncwarp();
+  if (!(mode & 1)) {
+    if (lane < 16) st->invT[lane] = sc.A[lane];
+    if (lane < 12) st->Tlin[lane] = (float)sc.A[lane];
     return;
   }
-#pragma unroll
-  for (int k = 0; k < 36; k++) st->H[k] = H[k];
-#pragma unroll
-  for (int k = 0; k < 6; k++) st->b[k] = b[k];
-  st->error = (float)tot[27];
-  st->inliers = (int)tot[28];
-  st->candidates = (int)tot[29];
-  st->num_corr = (int)tot[30];
-  if (mode & 2) return;
-  // H += lambda I; dx = H^-1 (-b); invT = v2t(dx) invT  (alignerprojective.cpp:72-95)
-  double A[36], nb[6], dx[6];
-#pragma unroll
-  for (int k = 0; k < 36; k++) A[k] = H[k];
-#pragma unroll
-  for (int i = 0; i < 6; i++) { A[i * 6 + i] += (double)lambda; nb[i] = -b[i]; }
-  d_ldlt_solve6(A, nb, dx);
-  double dT[16], nT[16];
-  d_v2t(dx, dT);
-  d_mm4(dT, st->invT, nT);
-  for (int k = 0; k < 16; k++) st->invT[k] = nT[k];
-  st->invT[12] = 0; st->invT[13] = 0; st->invT[14] = 0; st->invT[15] = 1;
-  float12_of(st->invT, st->Tlin);
-  if (!(mode & 1)) return;
   // T = invT^-1, renormalised through t2v/v2t (alignerprojective.cpp:98-100)
-  double T[16], x[6];
-  d_iso_inverse(st->invT, T);
-  d_t2v(T, x);
-  d_v2t(x, st->T);
-  st->iterations += 1;
-  for (int k = 0; k < 12; k++) st->Tgate_used[k] = st->Tgate[k];
+  double v[6];
+  warp_iso_inverse(sc.A, sc.B, lane);
+  warp_t2v(sc.B, v, lane);
+  warp_v2t(v, sc.T, lane);
+  if (lane == 0) st->iterations = iterations + 1;
+  if (lane < 12) st->Tgate_used[lane] = gate_used;
   if (early_eps > 0) {
-    double Si[16], D[16], dv[6];
-    d_iso_inverse(st->Tstart, Si);
-    d_mm4(st->T, Si, D);
-    d_t2v(D, dv);
+    warp_iso_inverse(sc.Tstart, sc.A, lane);
+    warp_mm4(sc.T, sc.A, sc.B, lane);
+    warp_t2v(sc.B, v, lane);
     double m = 0;
-    for (int k = 0; k < 6; k++) m = fmax(m, fabs(dv[k]));
-    if (m < early_eps) st->done = 1;
+#pragma unroll
+    for (int k = 0; k < 6; k++) m = fmax(m, fabs(v[k]));
+    if (lane == 0 && m < early_eps) st->done = 1;
+    __syncwarp();
   }
-  begin_outer(pd, st);
+  // the next outer iteration starts from T (as begin_outer)
+  warp_mm4(sc.T, sc.off, sc.A, lane);
+  warp_iso_inverse(sc.A, sc.B, lane);  // the projector's inverse pose
+  warp_iso_inverse(sc.T, sc.A, lane);  // invT
+  if (lane < 16) {
+    st->T[lane] = sc.T[lane];
+    st->Tstart[lane] = sc.T[lane];
+    st->invT[lane] = sc.A[lane];
+  }
+  if (lane < 12) {
+    const int j = lane & 3;
+    st->KRt[lane] = (float)(K[0] * sc.B[j] + K[1] * sc.B[4 + j] + K[2] * sc.B[8 + j]);
+    const float f = (float)sc.A[lane];
+    st->Tgate[lane] = f;
+    st->Tlin[lane] = f;
+  }
 }
 
 // ------------------------------------------------------------ launchers
@@ -1290,7 +1469,7 @@ void launch_init_pairs(const PairDev *d_pairs, int npairs, const double *d_guess
 void launch_solve(const PairDev *d_pairs, int npairs, float lambda, int mode, double early_eps, int ignore_done,
                   cudaStream_t s, Profiler *prof) {
   prof->begin(NICP_K_SOLVE, s);
-  k_solve<<<npairs, 128, 0, s>>>(d_pairs, npairs, lambda, mode, early_eps, ignore_done);
+  k_solve<<<npairs, kSumThreads, 0, s>>>(d_pairs, npairs, lambda, mode, early_eps, ignore_done);
   prof->end(NICP_K_SOLVE, s);
 }
 
@@ -1331,17 +1510,12 @@ __global__ void __launch_bounds__(kCorrThreads) k_lin_noalloc(NoAllocLinArgs a, 
 
 // Sums the tile partials in the same fixed order as k_solve and writes
 // H (36, row-major), b (6), error, inliers to out.
-__global__ void __launch_bounds__(128) k_lin_noalloc_sum(int ntiles, const double *__restrict__ partials,
-                                                         double *__restrict__ out) {
-  __shared__ double part[4][32];
+__global__ void __launch_bounds__(kSumThreads) k_lin_noalloc_sum(int ntiles, const double *__restrict__ partials,
+                                                                 double *__restrict__ out) {
+  __shared__ double part[kSumGroups][32];
   __shared__ double tot[32];
-  const int e = threadIdx.x & 31, g = threadIdx.x >> 5;
-  double s = 0.0;
-  const int nt = min(ntiles, kNoAllocMaxTiles);
-  for (int t = g; t < nt; t += 4) s += partials[(size_t)t * kPartialWords + e];
-  part[g][e] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) tot[e] = ((part[0][e] + part[1][e]) + part[2][e]) + part[3][e];
+  sum_tile_partials(partials, min(ntiles, kNoAllocMaxTiles), false, part);
+  if (threadIdx.x < 32) tot[threadIdx.x] = sum_groups(part, false, threadIdx.x);
   __syncthreads();
   if (threadIdx.x != 0) return;
   const int li[6][2] = {{0, 0}, {1, 0}, {1, 1}, {2, 0}, {2, 1}, {2, 2}};
@@ -1390,7 +1564,7 @@ int lin_noalloc(const NoAllocLinArgs &args, double *out_dev, cudaStream_t s) {
   if (!partials) return NICP_ECUDA;
   const int ntiles = std::max(1, (args.num_pairs + kCorrTilePixels - 1) / kCorrTilePixels);
   k_lin_noalloc<<<ntiles, kCorrThreads, 0, s>>>(args, partials);
-  k_lin_noalloc_sum<<<1, 128, 0, s>>>(ntiles, partials, out_dev);
+  k_lin_noalloc_sum<<<1, kSumThreads, 0, s>>>(ntiles, partials, out_dev);
   return cudaGetLastError() == cudaSuccess ? NICP_OK : NICP_ECUDA;
 }
 
