@@ -1342,7 +1342,7 @@ extern "C" int nicp_linearize(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_c
   const PairDev *dpd = (const PairDev *)(ctx->ws + pl.o_pairs);
   launch_lin_list(dpd, 1, pl.total_tiles, lin_params(*prm), std::max(1, parity_threads), 0,
                   (const float *)(ctx->ws + pl.o_krt), s, &ctx->prof);
-  launch_solve(dpd, 1, 0.0f, 2 | (prm->cross_block_f32 ? kSolveCrossF32 : 0), 0.0, 1, s, &ctx->prof);
+  launch_solve(dpd, 1, 0.0f, 2 | (prm->cross_block_f32 ? kSolveCrossF32 : 0), 0.0, 1, false, s, &ctx->prof);
   CK(ctx, cudaGetLastError());
   char *pd_host;
   if ((rc = pin_down(ctx, sizeof(PairState), &pd_host))) return rc;
@@ -1417,8 +1417,8 @@ extern "C" int nicp_project(nicp_ctx *ctx, const nicp_cloud *cloud, const nicp_c
   CK(ctx, cudaEventRecord(ctx->pin_up_ev, s));
   CK(ctx, cudaMemsetAsync(ctx->ws + pl.o_zbuf, 0xff, pl.zbuf_bytes, s));
   const PairDev *dpd = (const PairDev *)(ctx->ws + pl.o_pairs);
-  launch_zbuffer(dpd, 1, pl.max_pt_tiles, 0, (const float *)(ctx->ws + pl.o_krt), kZbufDefaultPPT, s, &ctx->prof);
-  launch_resolve(dpd, 1, pl.max_tiles, 0, (float *)(ctx->ws + o_depth), 0, s, &ctx->prof);
+  launch_zbuffer(dpd, 1, pl.max_pt_tiles, 0, (const float *)(ctx->ws + pl.o_krt), kZbufDefaultPPT, false, s, &ctx->prof);
+  launch_resolve(dpd, 1, pl.max_tiles, 0, (float *)(ctx->ws + o_depth), 0, false, s, &ctx->prof);
   CK(ctx, cudaGetLastError());
   if (index_out) CK(ctx, cudaMemcpyAsync(index_out, ctx->ws + pl.o_cur[0], 4 * P, cudaMemcpyDeviceToHost, s));
   if (depth_out) CK(ctx, cudaMemcpyAsync(depth_out, ctx->ws + o_depth, 4 * P, cudaMemcpyDeviceToHost, s));
@@ -1666,7 +1666,7 @@ extern "C" int nicp_align_nn(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cl
   LinParams lp = lin_params(*lin);
   const int xb = lin->cross_block_f32 ? kSolveCrossF32 : 0;
   launch_init_pairs(dpd, 1, (const double *)(ws + pl.o_guess), (const double *)(ws + pl.o_guess + 128), nullptr, 0,
-                    s, &ctx->prof);
+                    false, s, &ctx->prof);
   NNQuery q = nn_query(ctx, pl, ref, cur, normal_scaling, *corr, nullptr, (const PairState *)(ws + pl.o_st));
   for (int i = 0; i < prm->outer_iterations; i++) {
     // correspondences with the state's T^-1 (alignernn.cpp:40-45)
@@ -1675,13 +1675,13 @@ extern "C" int nicp_align_nn(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cl
       return fail(ctx, NICP_ECUDA, "nearest-neighbour query failed");
     for (int k = 0; k < prm->inner_iterations; k++) {
       launch_lin_list(dpd, 1, pl.tiles, lp, 1, 1, nullptr, s, &ctx->prof);
-      launch_solve(dpd, 1, prm->lambda, ((k == prm->inner_iterations - 1) ? 1 : 0) | xb, prm->early_exit_eps, 0, s,
-                   &ctx->prof);
+      launch_solve(dpd, 1, prm->lambda, ((k == prm->inner_iterations - 1) ? 1 : 0) | xb, prm->early_exit_eps, 0, false,
+                   s, &ctx->prof);
     }
   }
   if (prm->compute_statistics) {
     launch_lin_list(dpd, 1, pl.tiles, lp, 1, 2, nullptr, s, &ctx->prof);
-    launch_solve(dpd, 1, 0.0f, 4 | xb, 0.0, 1, s, &ctx->prof);
+    launch_solve(dpd, 1, 0.0f, 4 | xb, 0.0, 1, false, s, &ctx->prof);
   }
   CK(ctx, cudaGetLastError());
   PairState st;
@@ -1858,8 +1858,8 @@ extern "C" int nicp_merge(nicp_ctx *ctx, nicp_cloud *cloud, const nicp_camera *c
   CK(ctx, cudaMemsetAsync(ctx->ws + pl.o_zbuf, 0xff, pl.zbuf_bytes, s));
   const PairDev *dpd = (const PairDev *)(ctx->ws + pl.o_pairs);
   // the serial z-buffer of PinholePointProjector::project, all points kept
-  launch_zbuffer(dpd, 1, pl.max_pt_tiles, 0, (const float *)(ctx->ws + pl.o_krt), kZbufDefaultPPT, s, &ctx->prof);
-  launch_resolve(dpd, 1, pl.max_tiles, 0, (float *)(ex + o_depth), 0, s, &ctx->prof);
+  launch_zbuffer(dpd, 1, pl.max_pt_tiles, 0, (const float *)(ctx->ws + pl.o_krt), kZbufDefaultPPT, false, s, &ctx->prof);
+  launch_resolve(dpd, 1, pl.max_tiles, 0, (float *)(ex + o_depth), 0, false, s, &ctx->prof);
   MergeArgs a{};
   a.n = n;
   a.count = cloud->count;
@@ -1935,31 +1935,33 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) 
   int outer = p.outer_iterations, inner = p.inner_iterations;
   bool stats = p.compute_statistics != 0;
   const int xb = a.lin->cross_block_f32 ? kSolveCrossF32 : 0;
+  // (list mode's kernels and the general fused kernel are not part of a chain)
+  const bool chained = pl.structured && few_tiles(pl.n, pl.max_tiles);
   cudaMemsetAsync(ctx->ws + pl.o_zbuf, 0xff, pl.zbuf_bytes, s);
   int *tile_pair = (int *)(ctx->ws + pl.o_tile_pair);
   launch_init_pairs(dpd, pl.n, (const double *)(ctx->ws + pl.o_guess), (const double *)(ctx->ws + pl.o_roff),
-                    tile_pair, pl.max_tiles, s, &ctx->prof);
+                    tile_pair, pl.max_tiles, chained, s, &ctx->prof);
   // current cloud, seen from its sensor offset, projected once (alignerprojective.cpp:36-39)
   const nicp_ctx::Launch &L = ctx->launch;
-  launch_zbuffer(dpd, pl.n, pl.max_pt_tiles, 0, (const float *)(ctx->ws + pl.o_krt), L.zb_ppt, s, &ctx->prof);
+  launch_zbuffer(dpd, pl.n, pl.max_pt_tiles, 0, (const float *)(ctx->ws + pl.o_krt), L.zb_ppt, chained, s, &ctx->prof);
   // outside list (parity) mode, current pixels whose point has no normal are
   // dropped from the index image: the gates would reject them anyway
-  launch_resolve(dpd, pl.n, pl.max_tiles, 0, nullptr, (pl.list_mode || cp.demoted) ? 0 : 1, s, &ctx->prof);
+  launch_resolve(dpd, pl.n, pl.max_tiles, 0, nullptr, (pl.list_mode || cp.demoted) ? 0 : 1, chained, s, &ctx->prof);
   for (int i = 0; i < outer; i++) {
-    launch_zbuffer(dpd, pl.n, pl.max_pt_tiles, 1, nullptr, L.zb_ppt, s, &ctx->prof);
+    launch_zbuffer(dpd, pl.n, pl.max_pt_tiles, 1, nullptr, L.zb_ppt, chained, s, &ctx->prof);
     if (pl.list_mode) {
-      launch_resolve(dpd, pl.n, pl.max_tiles, 1, nullptr, 0, s, &ctx->prof);
+      launch_resolve(dpd, pl.n, pl.max_tiles, 1, nullptr, 0, false, s, &ctx->prof);
       launch_corr_list(dpd, pl.n, pl.total_tiles, cp, 1, nullptr, s, &ctx->prof);
       for (int k = 0; k < inner; k++) {
         launch_lin_list(dpd, pl.n, pl.total_tiles, lp, std::max(1, a.corr->parity_threads), 1, nullptr, s, &ctx->prof);
-        launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, s, &ctx->prof);
+        launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, chained, s, &ctx->prof);
       }
     } else {
       for (int k = 0; k < inner; k++) {
         int flags = (k == 0) ? (1 | 2 | (pl.keep_ref ? 4 : 0)) : 0;
-        launch_corr_lin(dpd, pl.n, pl.total_tiles, cp, lp, flags, pl.structured, L.corr_ctas, tile_pair, s,
+        launch_corr_lin(dpd, pl.n, pl.total_tiles, pl.max_tiles, cp, lp, flags, pl.structured, L.corr_ctas, tile_pair, s,
                         &ctx->prof);
-        launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, s, &ctx->prof);
+        launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, chained, s, &ctx->prof);
       }
     }
   }
@@ -1969,8 +1971,8 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) 
     if (pl.list_mode)
       launch_lin_list(dpd, pl.n, pl.total_tiles, lp, std::max(1, a.corr->parity_threads), 2, nullptr, s, &ctx->prof);
     else
-      launch_corr_lin(dpd, pl.n, pl.total_tiles, cp, lp, 8, pl.structured, L.corr_ctas, tile_pair, s, &ctx->prof);
-    launch_solve(dpd, pl.n, 0.0f, 4 | xb, 0.0, 1, s, &ctx->prof);
+      launch_corr_lin(dpd, pl.n, pl.total_tiles, pl.max_tiles, cp, lp, 8, pl.structured, L.corr_ctas, tile_pair, s, &ctx->prof);
+    launch_solve(dpd, pl.n, 0.0f, 4 | xb, 0.0, 1, chained, s, &ctx->prof);
   }
 }
 

@@ -145,6 +145,18 @@ struct LinParams {
   int demoted;
 };
 
+// ---- launches chained without a drain between them (launch in
+// kernels.hpp).  A chained kernel's CTAs may start while the kernel before it
+// still runs: what they read before chain_wait() must have been written at
+// least two kernels earlier (chain_wait() returns when the kernel before has
+// completed, and a kernel lets the next one start only after its own wait).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain() {
+  chain_wait();
+  chain_next();
+}
+
 // ------------------------------------------------------------ float helpers
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }

@@ -62,21 +62,24 @@ __global__ void __launch_bounds__(kPointsPerCta / PPT)
   if (pi >= npairs) return;
   const PairDev &pd = pairs[pi];
   const PairState *st = pd.state;
-  if (mode == 1 && st->done) return;
+  // the clouds are older than the loop: the points are fetched while the
+  // kernel before (the solve that sets KRt and done) finishes
   const int i0 = blockIdx.x * kPointsPerCta + threadIdx.x;
   const float4 *pts = mode ? pd.ref_pts : pd.cur_pts;
   const int n = mode ? *pd.ref_count : *pd.cur_count;
-  if (i0 >= n) return;
-  float K[12];
-  const float *src = mode ? st->KRt : explicit_KRt + 12 * pi;
-#pragma unroll
-  for (int k = 0; k < 12; k++) K[k] = src[k];
   float4 p[PPT];
 #pragma unroll
   for (int k = 0; k < PPT; k++) {
     int i = i0 + k * kThreads;
     p[k] = (i < n) ? pts[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
+  chain();
+  if (mode == 1 && st->done) return;
+  if (i0 >= n) return;
+  float K[12];
+  const float *src = mode ? st->KRt : explicit_KRt + 12 * pi;
+#pragma unroll
+  for (int k = 0; k < 12; k++) K[k] = src[k];
 #pragma unroll
   for (int k = 0; k < PPT; k++) {
     int i = i0 + k * kThreads;
@@ -111,6 +114,7 @@ __global__ void k_resolve(const PairDev *__restrict__ pairs, int npairs, int to_
   const int P = pd.rows * pd.cols;
   const int pix0 = blockIdx.x * kCorrTilePixels + threadIdx.x;
   int32_t *dst = to_ref ? pd.ref_index : pd.cur_index;
+  chain();
   unsigned long long z[kCorrTilePixels / kCorrThreads];
 #pragma unroll
   for (int k = 0; k < kCorrTilePixels / kCorrThreads; k++) {
@@ -329,8 +333,20 @@ __device__ __forceinline__ void lin_terms(const LinParams &lp, const float *T12,
 // transform.  Every accumulator update is one fused chain of FMAs; the
 // robust kernel's weight ks (linearizer.cpp:83-89) is folded into the
 // weights and residual terms only for the pixels beyond the chi2 bound.
-__device__ __forceinline__ void lin_terms_structured_xf(const LinParams &lp, const float *omd, float3 rp, float3 rn,
-                                                       float4 cpt, float4 cn, Acc &acc) {
+// A pixel's part is what the sums need of it (PixelTerms); two disjoint sets
+// of accumulators take it up (add_pose_terms, add_rotation_terms), so that
+// k_corr_tile can give them to different warps.
+struct PixelTerms {
+  float ux, uy, uz, be;   // current normal, beta of Omega_p
+  float a, b, c, al;      // moved reference point, alpha of Omega_p
+  float an, bn, cn, aln;  // moved reference normal, alpha of Omega_n
+  float ep0, ep1, ep2, ben;  // Omega_p times the point residual, beta of Omega_n
+  float en0, en1, en2, le;   // Omega_n times the normal residual, chi2
+};
+
+// False when the pixel adds nothing (an outlier without the robust kernel).
+__device__ __forceinline__ bool pixel_terms(const LinParams &lp, const float *omd, float3 rp, float3 rn, float4 cpt,
+                                            float4 cn, PixelTerms &o) {
   float alp = 0.0f, bep = 0.0f, aln = 0.0f, ben = 0.0f;
   if (point_has_normal(cpt.w)) {
     const int cls = (int)cpt.w - 1;
@@ -354,54 +370,77 @@ __device__ __forceinline__ void lin_terms_structured_xf(const LinParams &lp, con
   float en0 = fmaf(bv, ux, aln * ne0), en1 = fmaf(bv, uy, aln * ne1), en2 = fmaf(bv, uz, aln * ne2);
   float le = fmaf(ne2, en2, fmaf(ne1, en1, fmaf(ne0, en0, fmaf(pe2, ep2, fmaf(pe1, ep1, pe0 * ep0)))));
   if (le > lp.max_chi2) {
-    if (!lp.robust) return;
+    if (!lp.robust) return false;
     const float ks = lp.max_chi2 / le;
     le *= ks;
     alp *= ks; bep *= ks; aln *= ks; ben *= ks;
     ep0 *= ks; ep1 *= ks; ep2 *= ks;
     en0 *= ks; en1 *= ks; en2 *= ks;
   }
-  acc.v[27] += le;
-  acc.cnt += Acc::kInlier;
-  const float a = rp.x, b = rp.y, c = rp.z;
-  const float an = rn.x, bn = rn.y, cn2 = rn.z;
+  o.ux = ux; o.uy = uy; o.uz = uz; o.be = bep;
+  o.a = rp.x; o.b = rp.y; o.c = rp.z; o.al = alp;
+  o.an = rn.x; o.bn = rn.y; o.cn = rn.z; o.aln = aln;
+  o.ep0 = ep0; o.ep1 = ep1; o.ep2 = ep2; o.ben = ben;
+  o.en0 = en0; o.en1 = en1; o.en2 = en2; o.le = le;
+  return true;
+}
+
+// Htt, Htr, bt and br (v[0..14], v[21..26])
+__device__ __forceinline__ void add_pose_terms(const PixelTerms &p, float *v) {
   // Htt += Omega_p
-  const float t0 = bep * ux, t1 = bep * uy, t2 = bep * uz;
-  acc.v[0] = fmaf(t0, ux, acc.v[0] + alp);
-  acc.v[1] = fmaf(t0, uy, acc.v[1]);
-  acc.v[2] = fmaf(t1, uy, acc.v[2] + alp);
-  acc.v[3] = fmaf(t0, uz, acc.v[3]);
-  acc.v[4] = fmaf(t1, uz, acc.v[4]);
-  acc.v[5] = fmaf(t2, uz, acc.v[5] + alp);
+  const float t0 = p.be * p.ux, t1 = p.be * p.uy, t2 = p.be * p.uz;
+  v[0] = fmaf(t0, p.ux, v[0] + p.al);
+  v[1] = fmaf(t0, p.uy, v[1]);
+  v[2] = fmaf(t1, p.uy, v[2] + p.al);
+  v[3] = fmaf(t0, p.uz, v[3]);
+  v[4] = fmaf(t1, p.uz, v[4]);
+  v[5] = fmaf(t2, p.uz, v[5] + p.al);
   // Htr += Omega_p S = alp S + bep u wp^T, S = [[0, c, -b], [-c, 0, a], [b, -a, 0]]
-  const float wp0 = fmaf(b, uz, -c * uy), wp1 = fmaf(c, ux, -a * uz), wp2 = fmaf(a, uy, -b * ux);
-  const float wn0 = fmaf(bn, uz, -cn2 * uy), wn1 = fmaf(cn2, ux, -an * uz), wn2 = fmaf(an, uy, -bn * ux);
-  acc.v[6] = fmaf(t0, wp0, acc.v[6]);
-  acc.v[7] = fmaf(t0, wp1, fmaf(alp, c, acc.v[7]));
-  acc.v[8] = fmaf(t0, wp2, fmaf(-alp, b, acc.v[8]));
-  acc.v[9] = fmaf(t1, wp0, fmaf(-alp, c, acc.v[9]));
-  acc.v[10] = fmaf(t1, wp1, acc.v[10]);
-  acc.v[11] = fmaf(t1, wp2, fmaf(alp, a, acc.v[11]));
-  acc.v[12] = fmaf(t2, wp0, fmaf(alp, b, acc.v[12]));
-  acc.v[13] = fmaf(t2, wp1, fmaf(-alp, a, acc.v[13]));
-  acc.v[14] = fmaf(t2, wp2, acc.v[14]);
-  // Hrr += S^T Omega_p S + Sn^T Omega_n Sn
-  //      = alp (|v|^2 I - v v^T) + aln (|vn|^2 I - vn vn^T) + bep wp wp^T + ben wn wn^T
-  const float qa = alp * a, qb = alp * b, qc = alp * c;
-  const float qan = aln * an, qbn = aln * bn, qcn = aln * cn2;
-  const float pw0 = bep * wp0, pw1 = bep * wp1, pw2 = bep * wp2;
-  const float nw0 = ben * wn0, nw1 = ben * wn1, nw2 = ben * wn2;
-  acc.v[15] = fmaf(nw0, wn0, fmaf(pw0, wp0, fmaf(qcn, cn2, fmaf(qbn, bn, fmaf(qc, c, fmaf(qb, b, acc.v[15]))))));
-  acc.v[16] = fmaf(nw1, wn0, fmaf(pw1, wp0, fmaf(-qbn, an, fmaf(-qb, a, acc.v[16]))));
-  acc.v[17] = fmaf(nw1, wn1, fmaf(pw1, wp1, fmaf(qcn, cn2, fmaf(qan, an, fmaf(qc, c, fmaf(qa, a, acc.v[17]))))));
-  acc.v[18] = fmaf(nw2, wn0, fmaf(pw2, wp0, fmaf(-qcn, an, fmaf(-qc, a, acc.v[18]))));
-  acc.v[19] = fmaf(nw2, wn1, fmaf(pw2, wp1, fmaf(-qcn, bn, fmaf(-qc, b, acc.v[19]))));
-  acc.v[20] = fmaf(nw2, wn2, fmaf(pw2, wp2, fmaf(qbn, bn, fmaf(qan, an, fmaf(qb, b, fmaf(qa, a, acc.v[20]))))));
+  const float wp0 = fmaf(p.b, p.uz, -p.c * p.uy), wp1 = fmaf(p.c, p.ux, -p.a * p.uz),
+              wp2 = fmaf(p.a, p.uy, -p.b * p.ux);
+  v[6] = fmaf(t0, wp0, v[6]);
+  v[7] = fmaf(t0, wp1, fmaf(p.al, p.c, v[7]));
+  v[8] = fmaf(t0, wp2, fmaf(-p.al, p.b, v[8]));
+  v[9] = fmaf(t1, wp0, fmaf(-p.al, p.c, v[9]));
+  v[10] = fmaf(t1, wp1, v[10]);
+  v[11] = fmaf(t1, wp2, fmaf(p.al, p.a, v[11]));
+  v[12] = fmaf(t2, wp0, fmaf(p.al, p.b, v[12]));
+  v[13] = fmaf(t2, wp1, fmaf(-p.al, p.a, v[13]));
+  v[14] = fmaf(t2, wp2, v[14]);
   // bt += ep; br += Sp^T ep + Sn^T en (S^T e = v x e)
-  acc.v[21] += ep0; acc.v[22] += ep1; acc.v[23] += ep2;
-  acc.v[24] = fmaf(bn, en2, fmaf(-cn2, en1, fmaf(b, ep2, fmaf(-c, ep1, acc.v[24]))));
-  acc.v[25] = fmaf(cn2, en0, fmaf(-an, en2, fmaf(c, ep0, fmaf(-a, ep2, acc.v[25]))));
-  acc.v[26] = fmaf(an, en1, fmaf(-bn, en0, fmaf(a, ep1, fmaf(-b, ep0, acc.v[26]))));
+  v[21] += p.ep0; v[22] += p.ep1; v[23] += p.ep2;
+  v[24] = fmaf(p.bn, p.en2, fmaf(-p.cn, p.en1, fmaf(p.b, p.ep2, fmaf(-p.c, p.ep1, v[24]))));
+  v[25] = fmaf(p.cn, p.en0, fmaf(-p.an, p.en2, fmaf(p.c, p.ep0, fmaf(-p.a, p.ep2, v[25]))));
+  v[26] = fmaf(p.an, p.en1, fmaf(-p.bn, p.en0, fmaf(p.a, p.ep1, fmaf(-p.b, p.ep0, v[26]))));
+}
+
+// Hrr and chi2 (v[15..20], v[27]):
+// Hrr += S^T Omega_p S + Sn^T Omega_n Sn
+//      = alp (|v|^2 I - v v^T) + aln (|vn|^2 I - vn vn^T) + bep wp wp^T + ben wn wn^T
+__device__ __forceinline__ void add_rotation_terms(const PixelTerms &p, float *v) {
+  v[27] += p.le;
+  const float a = p.a, b = p.b, c = p.c, an = p.an, bn = p.bn, cn2 = p.cn;
+  const float wp0 = fmaf(b, p.uz, -c * p.uy), wp1 = fmaf(c, p.ux, -a * p.uz), wp2 = fmaf(a, p.uy, -b * p.ux);
+  const float wn0 = fmaf(bn, p.uz, -cn2 * p.uy), wn1 = fmaf(cn2, p.ux, -an * p.uz), wn2 = fmaf(an, p.uy, -bn * p.ux);
+  const float qa = p.al * a, qb = p.al * b, qc = p.al * c;
+  const float qan = p.aln * an, qbn = p.aln * bn, qcn = p.aln * cn2;
+  const float pw0 = p.be * wp0, pw1 = p.be * wp1, pw2 = p.be * wp2;
+  const float nw0 = p.ben * wn0, nw1 = p.ben * wn1, nw2 = p.ben * wn2;
+  v[15] = fmaf(nw0, wn0, fmaf(pw0, wp0, fmaf(qcn, cn2, fmaf(qbn, bn, fmaf(qc, c, fmaf(qb, b, v[15]))))));
+  v[16] = fmaf(nw1, wn0, fmaf(pw1, wp0, fmaf(-qbn, an, fmaf(-qb, a, v[16]))));
+  v[17] = fmaf(nw1, wn1, fmaf(pw1, wp1, fmaf(qcn, cn2, fmaf(qan, an, fmaf(qc, c, fmaf(qa, a, v[17]))))));
+  v[18] = fmaf(nw2, wn0, fmaf(pw2, wp0, fmaf(-qcn, an, fmaf(-qc, a, v[18]))));
+  v[19] = fmaf(nw2, wn1, fmaf(pw2, wp1, fmaf(-qcn, bn, fmaf(-qc, b, v[19]))));
+  v[20] = fmaf(nw2, wn2, fmaf(pw2, wp2, fmaf(qbn, bn, fmaf(qan, an, fmaf(qb, b, fmaf(qa, a, v[20]))))));
+}
+
+__device__ __forceinline__ void lin_terms_structured_xf(const LinParams &lp, const float *omd, float3 rp, float3 rn,
+                                                       float4 cpt, float4 cn, Acc &acc) {
+  PixelTerms p;
+  if (!pixel_terms(lp, omd, rp, rn, cpt, cn, p)) return;
+  acc.cnt += Acc::kInlier;
+  add_pose_terms(p, acc.v);
+  add_rotation_terms(p, acc.v);
 }
 
 __device__ __forceinline__ void lin_terms_structured(const LinParams &lp, const float *T12, const float *omd,
@@ -829,6 +868,190 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
   cp_async_wait<0>();
 }
 
+// ---- the same pass for few tiles: one CTA per tile, everything in flight.
+// With one tile per CTA the pipeline above has nothing to overlap: a launch
+// of 19 to 300 tiles took 9 to 11 us, the latency of one tile -- eight pixels
+// one after the other in each of 128 threads, their indices and points
+// fetched sub-tile by sub-tile.  Here 256 threads take a tile: all indices,
+// then all gathers are issued at once; a thread gates and forms the terms of
+// four pixels (PixelTerms, left in place of the gathered points), and the
+// sums of a slot -- the slot t, t + 128, ... of the thread t above -- are
+// taken over by two warps, one for each set of accumulators.  Every sum has
+// the terms and the order of k_corr_lin, so both give the same bits.  Loops
+// stay rolled: each instruction runs once or twice per launch, and fetching
+// them is a good part of its time.
+constexpr int kTileThreads = 256;
+constexpr int kTileRows = kCorrTilePixels / kFusedThreads;  // pixels of a slot: 8
+constexpr int kTileHalf = kCorrTilePixels / 2;
+constexpr int kTileCtas = 3;
+struct TileSmem {
+  float4 px[2][4][kTileHalf];  // per half tile: points and normals of both clouds, then four parts of the terms
+  float4 last[kTileHalf];      // the fifth part of the half at hand; then the sums' rows
+};
+
+// Grid (tiles of the largest pair image, pairs).
+__global__ void __launch_bounds__(kTileThreads, kTileCtas)
+    k_corr_tile(const PairDev *__restrict__ pairs, CorrParams cp, LinParams lp, int flags) {
+  extern __shared__ __align__(16) unsigned char tile_smem_raw[];
+  TileSmem &sm = *reinterpret_cast<TileSmem *>(tile_smem_raw);
+  __shared__ float sT[32];
+  __shared__ unsigned counts[kTileThreads / 32];
+  __shared__ double wsum[4][32];
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const bool stats_pass = flags & 8;
+  const bool drop_no_normal = !cp.demoted;
+  const PairDev &pd = pairs[blockIdx.y];
+  const PairState *st = pd.state;
+  const int rows = pd.rows, cols = pd.cols, P = rows * cols;
+  const int p0 = (int)blockIdx.x * kCorrTilePixels + t;
+  if ((int)blockIdx.x * kCorrTilePixels >= P) return;
+  const int nref = *pd.ref_count, ncur = *pd.cur_count;
+  const float4 *ref_pts = pd.ref_pts, *ref_nrm = pd.ref_nrm, *cur_pts = pd.cur_pts, *cur_nrm = pd.cur_nrm;
+  unsigned long long *zbuf = pd.zbuf;
+  int32_t *ref_index = pd.ref_index;
+  int ci[4], ri[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int p = p0 + k * kTileThreads;
+    ci[k] = p < P ? pd.cur_index[p] : -1;  // written before the loop
+  }
+  if (t >= 32 && t < 40) sT[24 + t - 32] = pd.cur_omd[t - 32];
+  chain();
+  // one round trip: the pair's flag and transforms, the pixels' indices
+  const int done = __ldcg(&st->done);
+  unsigned long long z[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int p = p0 + k * kTileThreads;
+    z[k] = ~0ull;
+    if (p < P) z[k] = (flags & 1) ? __ldcg(zbuf + p) : (unsigned long long)(unsigned)__ldcg(ref_index + p);
+  }
+  bool same_t = true;
+  if (t < 12) {
+    const float a = __ldcg((stats_pass ? st->Tgate_used : st->Tgate) + t), b = __ldcg(st->Tlin + t);
+    sT[t] = a;
+    sT[12 + t] = b;
+    same_t = a == b;
+  }
+  if (!stats_pass && done) return;
+  unsigned cnt = 0;
+  unsigned valid = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int p = p0 + k * kTileThreads;
+    ri[k] = (int)(unsigned)z[k];
+    if (flags & 1) {
+      // (an empty word decodes to an index beyond every cloud, or to -1)
+      const unsigned lo = (unsigned)z[k];
+      ri[k] = (drop_no_normal && (lo & 1u)) ? -1 : (int)(lo >> 1);
+      if (p < P && (flags & 2)) __stcs(zbuf + p, ~0ull);
+      if (p < P && (flags & 4)) ref_index[p] = ri[k];
+    }
+    bool ok = p < P && (unsigned)ri[k] < (unsigned)nref && (unsigned)ci[k] < (unsigned)ncur;
+    if (ok && cp.row_limit_threads > 1) ok = p / cols < (rows / cp.row_limit_threads) * cp.row_limit_threads;
+    if (ok) {
+      const int at = t + (k & 1) * kTileThreads;
+      cp_async16(&sm.px[k >> 1][0][at], ref_pts + ri[k]);
+      cp_async16(&sm.px[k >> 1][1][at], ref_nrm + ri[k]);
+      cp_async16(&sm.px[k >> 1][2][at], cur_pts + ci[k]);
+      cp_async16(&sm.px[k >> 1][3][at], cur_nrm + ci[k]);
+      cnt += Acc::kCandidate;
+      valid |= 1u << k;
+    }
+    if (k & 1) cp_async_commit();
+  }
+  float v[28];
+#pragma unroll
+  for (int k = 0; k < 28; k++) v[k] = 0.0f;
+  const int group = wid & 3;       // slots 32 group .. 32 group + 31
+  const bool rotation = wid >= 4;  // the set of accumulators (uniform in the warp)
+  const bool same = __syncthreads_and(same_t) != 0;  // and the constants are visible
+  cp_async_wait<1>();
+#pragma unroll 1
+  for (int h = 0; h < 2; h++) {
+    // gates and terms of a thread's two pixels (each reads what it copied itself)
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+      const int at = t + k * kTileThreads;
+      PixelTerms o = {};
+      if ((valid >> (2 * h + k)) & 1u) {
+        const float4 rp0 = sm.px[h][0][at], rn0 = sm.px[h][1][at], cpt = sm.px[h][2][at], cn = sm.px[h][3][at];
+        float3 rp, rn;
+        if (gate_t(cp, sT, rp0, rn0, cpt, cn, rp, rn)) {
+          cnt += Acc::kAccepted;
+          if (!same || cp.demoted) {
+            rp = xform_point_g(sT + 12, rp0);
+            rn = xform_normal_g(sT + 12, rn0);
+          }
+          PixelTerms q;
+          if (pixel_terms(lp, sT + 24, rp, rn, cpt, cn, q)) {
+            cnt += Acc::kInlier;
+            o = q;
+          }
+        }
+      }
+      sm.px[h][0][at] = make_float4(o.ux, o.uy, o.uz, o.be);
+      sm.px[h][1][at] = make_float4(o.a, o.b, o.c, o.al);
+      sm.px[h][2][at] = make_float4(o.an, o.bn, o.cn, o.aln);
+      sm.px[h][3][at] = make_float4(o.ep0, o.ep1, o.ep2, o.ben);
+      sm.last[at] = make_float4(o.en0, o.en1, o.en2, o.le);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int m = 0; m < kTileRows / 2; m++) {
+      const int at = m * kFusedThreads + 32 * group + lane;
+      const float4 r0 = sm.px[h][0][at], r1 = sm.px[h][1][at], r2 = sm.px[h][2][at], r3 = sm.px[h][3][at],
+                   r4 = sm.last[at];
+      const PixelTerms o = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y,
+                            r2.z, r2.w, r3.x, r3.y, r3.z, r3.w, r4.x, r4.y, r4.z, r4.w};
+      if (rotation) add_rotation_terms(o, v);
+      else add_pose_terms(o, v);
+    }
+    cp_async_wait<0>();
+    __syncthreads();  // sm.last has been read
+  }
+  cnt = __reduce_add_sync(0xffffffffu, cnt);  // (10 bits each: at most 128 pixels a warp)
+  if (lane == 0) counts[wid] = cnt;
+  // rows of 32 slots per group and element; lane L adds row L in FP64, in
+  // block_reduce_store_staged's order
+  float *row0 = reinterpret_cast<float *>(sm.px) + group * 28 * 32;
+#pragma unroll
+  for (int k = 0; k < 28; k++) {
+    const bool rot = (k >= 15 && k <= 20) || k == 27;
+    if (rot == rotation) row0[32 * k + lane] = v[k];
+  }
+  __syncthreads();
+  if (wid < 4) {
+    double d = 0.0;
+    if (lane < 28) {
+      const float4 *r4 = reinterpret_cast<const float4 *>(row0 + 32 * lane);
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const float4 x = r4[(q + lane) & 7];
+        d += (double)x.x;
+        d += (double)x.y;
+        d += (double)x.z;
+        d += (double)x.w;
+      }
+    }
+    wsum[wid][lane] = d;
+  }
+  __syncthreads();
+  if (wid == 0) {
+    double d = 0.0;
+    if (lane < 28) {
+#pragma unroll
+      for (int w = 0; w < 4; w++) d += wsum[w][lane];
+    } else if (lane < 31) {
+      int n = 0;
+#pragma unroll
+      for (int w = 0; w < kTileThreads / 32; w++) n += (int)((counts[w] >> (10 * (lane - 28))) & 1023u);
+      d = (double)n;
+    }
+    pd.partials[(size_t)blockIdx.x * kPartialWords + lane] = d * acc_scale(lane);
+  }
+}
+
 // ------------------------------------------------------------ list mode
 // CorrespondenceFinderProjective::_computeMulti for reference pixel p
 // (correspondencefinderprojective.cpp:150-240): the best current point of
@@ -1253,6 +1476,7 @@ __global__ void __launch_bounds__(kSumThreads) k_solve(const PairDev *__restrict
   const int P = pd.rows * pd.cols;
   const int nt = (P + kCorrTilePixels - 1) / kCorrTilePixels;
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  // (the pose is older than the linearization that this launch waits for)
   if (g >= 2 && threadIdx.x < 64 + 48) {
     const int q = threadIdx.x - 64;
     const double *from = q < 16 ? st->invT : q < 32 ? st->Tstart : st->ref_offset;
@@ -1265,6 +1489,7 @@ __global__ void __launch_bounds__(kSumThreads) k_solve(const PairDev *__restrict
 #pragma unroll
   for (int k = 0; k < 3; k++)
     if (lane < 12) K[k] = (double)pd.K[(lane >> 2) * 3 + k];
+  chain();
   if (st->done && !ignore_done) return;
   sum_tile_partials(src, nt, (mode & kSolveCrossF32) != 0, part);
   const double tot = sum_groups(part, (mode & kSolveCrossF32) != 0, lane);
@@ -1343,32 +1568,72 @@ __global__ void __launch_bounds__(kSumThreads) k_solve(const PairDev *__restrict
   }
 }
 
+// tile_pair[tile] = the pair whose pixel image holds the tile (grid: tiles
+// of a pair, pair), so that the persistent fused kernel finds a tile's pair
+// with one load instead of a search.
+__global__ void k_tile_pairs(const PairDev *__restrict__ pairs, int npairs, int *__restrict__ tile_pair, int pair0) {
+  const int pi = pair0 + (int)blockIdx.y;
+  if (pi >= npairs) return;
+  const PairDev &pd = pairs[pi];
+  chain();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int ntiles = (pd.rows * pd.cols + kCorrTilePixels - 1) / kCorrTilePixels;
+  if (t < ntiles) tile_pair[pd.tile_base + t] = pi;
+}
+
 // ------------------------------------------------------------ launchers
+// An SM changes its split of shared memory and L1 only while it is empty.
+// The loop's kernels are chained, so all of them ask for the split of the
+// fused kernel (its gather stages): otherwise its CTAs find SMs still set up
+// for the projection's small need and fewer of them fit.  Once per device
+// (std::call_once: host threads on other contexts wait rather than race).
+static void configure_loop() {
+  constexpr int kMaxDevices = 64;
+  static std::once_flag once[kMaxDevices];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  auto set = [] {
+    auto most_shared = [](auto *kernel) {
+      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    };
+    most_shared(k_zbuffer<4>);
+    most_shared(k_solve);
+    most_shared(k_corr_tile);
+    cudaFuncSetAttribute(k_corr_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem));
+  };
+  if (dev >= 0 && dev < kMaxDevices)
+    std::call_once(once[dev], set);
+  else
+    set();
+}
+
 void launch_zbuffer(const PairDev *d_pairs, int npairs, int max_pt_tiles, int mode, const float *explicit_KRt,
-                    int ppt, cudaStream_t s, Profiler *prof) {
+                    int ppt, bool chained, cudaStream_t s, Profiler *prof) {
   if (max_pt_tiles <= 0 || npairs <= 0) return;
+  configure_loop();
   prof->begin(NICP_K_ZBUFFER, s);
   const int kMaxGridY = 65535;
   for (int p0 = 0; p0 < npairs; p0 += kMaxGridY) {
     const dim3 g(max_pt_tiles, std::min(kMaxGridY, npairs - p0));
     switch (ppt) {
-      case 1: k_zbuffer<1><<<g, kPointsPerCta, 0, s>>>(d_pairs, npairs, mode, explicit_KRt, p0); break;
-      case 2: k_zbuffer<2><<<g, kPointsPerCta / 2, 0, s>>>(d_pairs, npairs, mode, explicit_KRt, p0); break;
-      case 8: k_zbuffer<8><<<g, kPointsPerCta / 8, 0, s>>>(d_pairs, npairs, mode, explicit_KRt, p0); break;
-      default: k_zbuffer<4><<<g, kPointsPerCta / 4, 0, s>>>(d_pairs, npairs, mode, explicit_KRt, p0); break;
+      case 1: launch(chained, k_zbuffer<1>, g, kPointsPerCta, 0, s, d_pairs, npairs, mode, explicit_KRt, p0); break;
+      case 2: launch(chained, k_zbuffer<2>, g, kPointsPerCta / 2, 0, s, d_pairs, npairs, mode, explicit_KRt, p0); break;
+      case 8: launch(chained, k_zbuffer<8>, g, kPointsPerCta / 8, 0, s, d_pairs, npairs, mode, explicit_KRt, p0); break;
+      default: launch(chained, k_zbuffer<4>, g, kPointsPerCta / 4, 0, s, d_pairs, npairs, mode, explicit_KRt, p0); break;
     }
   }
   prof->end(NICP_K_ZBUFFER, s);
 }
 
 void launch_resolve(const PairDev *d_pairs, int npairs, int max_tiles, int to_ref, float *depth_out,
-                    int drop_no_normal, cudaStream_t s, Profiler *prof) {
+                    int drop_no_normal, bool chained, cudaStream_t s, Profiler *prof) {
   if (max_tiles <= 0 || npairs <= 0) return;
+  configure_loop();
   prof->begin(NICP_K_RESOLVE, s);
   const int kMaxGridY = 65535;
   for (int p0 = 0; p0 < npairs; p0 += kMaxGridY)
-    k_resolve<<<dim3(max_tiles, std::min(kMaxGridY, npairs - p0)), kCorrThreads, 0, s>>>(d_pairs, npairs, to_ref,
-                                                                                        depth_out, drop_no_normal, p0);
+    launch(chained, k_resolve, dim3(max_tiles, std::min(kMaxGridY, npairs - p0)), kCorrThreads, 0, s, d_pairs, npairs,
+                   to_ref, depth_out, drop_no_normal, p0);
   prof->end(NICP_K_RESOLVE, s);
 }
 
@@ -1410,12 +1675,27 @@ static int corr_lin_grid(int total_tiles, int ctas_per_sm) {
   return std::min(total_tiles, grid);
 }
 
-void launch_corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, const CorrParams &cp, const LinParams &lp,
-                     int flags, bool structured, int ctas_per_sm, const int *tile_pair, cudaStream_t s,
+// Three CTAs of k_corr_tile fit on an SM.  Up to there the pass takes less
+// than with k_corr_lin (19 tiles 9.3 -> 6.8 us, 300 tiles 11.3 -> 9.2 us after
+// the projection's end); at 900 tiles, two waves, it takes more (22.4 us
+// against 19.7), and over many tiles k_corr_lin's pipeline does 1.6 times the
+// tiles per second.
+bool few_tiles(int npairs, int max_tiles) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return false;
+  return npairs <= 65535 && (long long)max_tiles * npairs <= (long long)kTileCtas * sms;
+}
+
+void launch_corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, int max_tiles, const CorrParams &cp,
+                     const LinParams &lp, int flags, bool structured, int ctas_per_sm, const int *tile_pair, cudaStream_t s,
                      Profiler *prof) {
   if (total_tiles <= 0) return;
+  configure_loop();
   prof->begin(NICP_K_CORR_LIN, s);
-  if (structured) {
+  if (structured && few_tiles(npairs, max_tiles)) {
+    launch(true, k_corr_tile, dim3(max_tiles, npairs), kTileThreads, sizeof(TileSmem), s, d_pairs, cp, lp, flags);
+  } else if (structured) {
     int grid = corr_lin_grid<true>(total_tiles, ctas_per_sm);
     k_corr_lin<true><<<grid, kFusedThreads, corr_smem<true>(), s>>>(d_pairs, npairs, tile_pair, total_tiles, cp,
                                                                     lp, flags);
@@ -1442,34 +1722,24 @@ void launch_lin_list(const PairDev *d_pairs, int npairs, int total_tiles, const 
   prof->end(NICP_K_LIN_LIST, s);
 }
 
-// tile_pair[tile] = the pair whose pixel image holds the tile (grid: tiles
-// of a pair, pair), so that the persistent fused kernel finds a tile's pair
-// with one load instead of a search.
-__global__ void k_tile_pairs(const PairDev *__restrict__ pairs, int npairs, int *__restrict__ tile_pair, int pair0) {
-  const int pi = pair0 + (int)blockIdx.y;
-  if (pi >= npairs) return;
-  const PairDev &pd = pairs[pi];
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ntiles = (pd.rows * pd.cols + kCorrTilePixels - 1) / kCorrTilePixels;
-  if (t < ntiles) tile_pair[pd.tile_base + t] = pi;
-}
-
 void launch_init_pairs(const PairDev *d_pairs, int npairs, const double *d_guesses, const double *d_ref_offsets,
-                       int *tile_pair, int max_tiles, cudaStream_t s, Profiler *prof) {
+                       int *tile_pair, int max_tiles, bool chained, cudaStream_t s, Profiler *prof) {
+  configure_loop();
   prof->begin(NICP_K_SOLVE, s);
   k_init_pairs<<<(npairs + 63) / 64, 64, 0, s>>>(d_pairs, npairs, d_guesses, d_ref_offsets);
   const int kMaxGridY = 65535;
   if (tile_pair && max_tiles > 0)
     for (int p0 = 0; p0 < npairs; p0 += kMaxGridY)
-      k_tile_pairs<<<dim3((max_tiles + 255) / 256, std::min(kMaxGridY, npairs - p0)), 256, 0, s>>>(d_pairs, npairs,
-                                                                                                  tile_pair, p0);
+      launch(chained, k_tile_pairs, dim3((max_tiles + 255) / 256, std::min(kMaxGridY, npairs - p0)), 256, 0, s,
+                     d_pairs, npairs, tile_pair, p0);
   prof->end(NICP_K_SOLVE, s, tile_pair && max_tiles > 0 ? 2 : 1);
 }
 
 void launch_solve(const PairDev *d_pairs, int npairs, float lambda, int mode, double early_eps, int ignore_done,
-                  cudaStream_t s, Profiler *prof) {
+                  bool chained, cudaStream_t s, Profiler *prof) {
+  configure_loop();
   prof->begin(NICP_K_SOLVE, s);
-  k_solve<<<npairs, kSumThreads, 0, s>>>(d_pairs, npairs, lambda, mode, early_eps, ignore_done);
+  launch(chained, k_solve, npairs, kSumThreads, 0, s, d_pairs, npairs, lambda, mode, early_eps, ignore_done);
   prof->end(NICP_K_SOLVE, s);
 }
 

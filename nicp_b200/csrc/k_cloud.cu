@@ -87,6 +87,7 @@ __device__ __forceinline__ int block_sum_int(int v, int *smem) {
 __global__ void __launch_bounds__(256) k_unproject_count(const FrameDev *__restrict__ frames,
                                                          const int *__restrict__ frame_of) {
   __shared__ int red[32];
+  chain();
   int fi = frame_of[blockIdx.x];
   const FrameDev &f = frames[fi];
   int tile = blockIdx.x - f.tile_base;
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(256) k_unproject_write(const FrameDev *__restr
   const int P = f.rows * f.cols;
   const int ntiles = (P + kUnprojTilePixels - 1) / kUnprojTilePixels;
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  chain();
   // points numbered before this tile
   int before = 0;
   for (int q = t; q < tile; q += blockDim.x) before += f.tile_counts[q];
@@ -456,6 +458,7 @@ __global__ void __launch_bounds__(kRowThreads) k_moments_band_totals(const Frame
   const int r0 = b * kBandRows, nr = min(f.rows - r0, kBandRows);
   A *tot = static_cast<A *>(f.band_tot) + (size_t)b * 10 * cols;
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  chain();
   A carry[10];
 #pragma unroll
   for (int m = 0; m < 10; m++) carry[m] = A(0);
@@ -546,6 +549,7 @@ __global__ void __launch_bounds__(128) k_moments_band_carry(const FrameDev *__re
   if (q >= (int)stride) return;
   const int nb = (f.rows + kBandRows - 1) / kBandRows;
   A *tot = static_cast<A *>(f.band_tot) + q;
+  chain();
   A acc = A(0);
   for (int b0 = 0; b0 < nb; b0 += kAhead) {
     A v[kAhead];
@@ -942,10 +946,9 @@ void launch_depth_scale(const uint16_t *u16, const float *f32, size_t pitch_elem
 
 void launch_unproject(const FrameDev *d_frames, int nframes, int total_tiles, const int *frame_of_tile, cudaStream_t s,
                       Profiler *prof) {
-  (void)nframes;
   prof->begin(NICP_K_UNPROJECT, s);
   k_unproject_count<<<total_tiles, 256, 0, s>>>(d_frames, frame_of_tile);
-  k_unproject_write<<<total_tiles, 256, 0, s>>>(d_frames, frame_of_tile);
+  launch(moments_row_path(nframes), k_unproject_write, total_tiles, 256, 0, s, d_frames, frame_of_tile);
   prof->end(NICP_K_UNPROJECT, s, 2);
 }
 
@@ -971,6 +974,7 @@ __global__ void __launch_bounds__(kRowThreads) k_moments_rowpre(const FrameDev *
   const int cols = f.cols;
   const size_t P = (size_t)f.rows * cols;
   A *Rp = static_cast<A *>(f.rowpre) + (size_t)r * cols;
+  chain();
   A carry[10];
 #pragma unroll
   for (int m = 0; m < 10; m++) carry[m] = A(0);
@@ -1002,6 +1006,7 @@ __global__ void __launch_bounds__(128) k_moments_colsum(const FrameDev *__restri
   const int r1 = min(f.rows, r0 + kBandRows);
   const int m = q / cols, c = q - m * cols;
   const size_t P = (size_t)f.rows * cols;
+  chain();
   A s = static_cast<const A *>(f.band_tot)[(size_t)b * 10 * cols + q];
   const A *Rp = static_cast<const A *>(f.rowpre) + m * P + c;
   A v[kBandRows];
@@ -1042,14 +1047,15 @@ template <class M>
 static void launch_bands(const FrameDev *d_frames, int nframes, int total_bands, int total_carry_ctas, int max_bands,
                          const int *frame_of_band, const int *frame_of_carry, cudaStream_t s, Profiler *prof) {
   configure_bands<M>();
+  const bool chained = moments_row_path(nframes);
   prof->begin(NICP_K_MOMENTS_BANDS, s);
-  k_moments_band_totals<M><<<total_bands, kRowThreads, band_smem_bytes<M>(), s>>>(d_frames, frame_of_band);
-  k_moments_band_carry<M><<<total_carry_ctas, 128, 0, s>>>(d_frames, frame_of_carry);
+  launch(chained, k_moments_band_totals<M>, total_bands, kRowThreads, band_smem_bytes<M>(), s, d_frames, frame_of_band);
+  launch(chained, k_moments_band_carry<M>, total_carry_ctas, 128, 0, s, d_frames, frame_of_carry);
   prof->end(NICP_K_MOMENTS_BANDS, s, 2);
   prof->begin(NICP_K_MOMENTS_SWEEP, s);
   if (moments_row_path(nframes) && max_bands <= 65535) {  // (grid y of the column sums)
-    k_moments_rowpre<M><<<dim3(total_bands, kBandRows), kRowThreads, 0, s>>>(d_frames, frame_of_band);
-    k_moments_colsum<M><<<dim3(total_carry_ctas, max_bands), 128, 0, s>>>(d_frames, frame_of_carry);
+    launch(chained, k_moments_rowpre<M>, dim3(total_bands, kBandRows), kRowThreads, 0, s, d_frames, frame_of_band);
+    launch(chained, k_moments_colsum<M>, dim3(total_carry_ctas, max_bands), 128, 0, s, d_frames, frame_of_carry);
     prof->end(NICP_K_MOMENTS_SWEEP, s, 2);
   } else {
     k_moments_band_sweep<M><<<dim3(max_bands, nframes), kRowThreads, band_smem_bytes<M>(), s>>>(d_frames, nframes);

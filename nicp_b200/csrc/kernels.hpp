@@ -9,6 +9,31 @@
 
 namespace nicp {
 
+// Launches a kernel; with `chained`, its CTAs may be placed while the kernel
+// before it on the stream finishes (programmatic dependent launch; in a
+// captured graph, a programmatic edge), so that the start-up of a launch, 1 to
+// 2.5 us in a chain of kernels of 3 to 12 us, overlaps the tail of the one
+// before.  A chained kernel calls chain_wait() before it touches what that one
+// writes (common.cuh).  Only small grids are chained: CTAs of a grid that
+// fills the GPU are then placed where the kernel before happens to leave room
+// first, several on one SM, and a long-running grid stays that way (a build of
+// 9 frames: band sweep 110 us, chained 125; the fused kernel over 8 pairs 43
+// us, chained 52).
+template <typename... P, typename... A>
+inline void launch(bool chained, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = attr;
+  c.numAttrs = chained ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // Brackets kernel launches with CUDA events on the launching stream.  Events
 // recorded during stream capture become graph nodes and are re-recorded on
 // every replay of that graph.
@@ -62,6 +87,7 @@ struct Profiler {
 
 // frame_of_*: the frame of each CTA of the 1-D build grids (unprojection
 // tiles, 16-row bands, band-carry CTAs), filled on the host.
+// (A build of few frames -- moments_row_path -- chains its launches.)
 void launch_unproject(const FrameDev *d_frames, int nframes, int total_tiles, const int *frame_of_tile, cudaStream_t s,
                       Profiler *prof);
 void launch_depth_scale(const uint16_t *u16, const float *f32, size_t pitch_elems, int rows, int cols,
@@ -112,13 +138,17 @@ void solution_statistics(const double H36[36], const double T16[16], double *tra
 // Grid (max_pt_tiles, npairs): max_pt_tiles = the largest number of
 // 1024-point tiles of any pair's projected cloud.
 void launch_zbuffer(const PairDev *d_pairs, int npairs, int max_pt_tiles, int mode, const float *explicit_KRt,
-                    int ppt, cudaStream_t s, Profiler *prof);
+                    int ppt, bool chained, cudaStream_t s, Profiler *prof);
 // Grid (max_tiles, npairs): max_tiles = the largest number of 1024-pixel
 // tiles of any pair's image.
 void launch_resolve(const PairDev *d_pairs, int npairs, int max_tiles, int to_ref, float *depth_out,
-                    int drop_no_normal, cudaStream_t s, Profiler *prof);
-void launch_corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, const CorrParams &cp, const LinParams &lp,
-                     int flags, bool structured, int ctas_per_sm, const int *tile_pair, cudaStream_t s,
+                    int drop_no_normal, bool chained, cudaStream_t s, Profiler *prof);
+// A loop over so few pixel tiles (max_tiles of each of npairs pairs) that one
+// CTA per tile fits on the GPU at once: the fused pass then runs as
+// k_corr_tile and the loop's launches are chained.
+bool few_tiles(int npairs, int max_tiles);
+void launch_corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, int max_tiles, const CorrParams &cp,
+                     const LinParams &lp, int flags, bool structured, int ctas_per_sm, const int *tile_pair, cudaStream_t s,
                      Profiler *prof);
 void launch_corr_list(const PairDev *d_pairs, int npairs, int total_tiles, const CorrParams &cp, int use_state_T,
                       const float *explicit_T, cudaStream_t s, Profiler *prof);
@@ -127,9 +157,9 @@ void launch_lin_list(const PairDev *d_pairs, int npairs, int total_tiles, const 
 // Initialises the pair states and, when tile_pair is given, the tile -> pair
 // table of the fused kernel (total pixel tiles entries).
 void launch_init_pairs(const PairDev *d_pairs, int npairs, const double *d_guesses, const double *d_ref_offsets,
-                       int *tile_pair, int max_tiles, cudaStream_t s, Profiler *prof);
+                       int *tile_pair, int max_tiles, bool chained, cudaStream_t s, Profiler *prof);
 void launch_solve(const PairDev *d_pairs, int npairs, float lambda, int mode, double early_eps, int ignore_done,
-                  cudaStream_t s, Profiler *prof);
+                  bool chained, cudaStream_t s, Profiler *prof);
 
 // Inputs of the scratch-free linearizer, passed by value to the kernel.
 struct NoAllocLinArgs {
