@@ -1341,7 +1341,7 @@ extern "C" int nicp_linearize(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_c
     CK(ctx, cudaMemcpyAsync(ctx->ws + pl.o_list[0], pairs, 8 * (size_t)num_pairs, cudaMemcpyHostToDevice, s));
   const PairDev *dpd = (const PairDev *)(ctx->ws + pl.o_pairs);
   launch_lin_list(dpd, 1, pl.total_tiles, lin_params(*prm), std::max(1, parity_threads), 0,
-                  (const float *)(ctx->ws + pl.o_krt), s, &ctx->prof);
+                  (const float *)(ctx->ws + pl.o_krt), false, s, &ctx->prof);
   launch_solve(dpd, 1, 0.0f, 2 | (prm->cross_block_f32 ? kSolveCrossF32 : 0), 0.0, 1, false, s, &ctx->prof);
   CK(ctx, cudaGetLastError());
   char *pd_host;
@@ -1476,44 +1476,57 @@ static int cloud_counts2(nicp_cloud *c, int out[2]);
 
 namespace {
 // Workspace of one NN alignment: the grid over the current cloud, the match
-// / flag / position arrays over the reference points, the pair list, FP64
+// and candidate arrays over the reference points, the pair list, FP64
 // partials, the pair descriptor and state.
 struct NNPlan {
   int nr = 0, nc = 0, tiles = 0;
   NNGrid grid{};
-  size_t o_keys, o_skeys, o_idx, o_sidx, o_feat, o_sfeat, o_cstart, o_cend, o_temp, temp_bytes;
-  size_t o_match, o_flag, o_pos, o_pairs, o_np, o_part, o_pd, o_st, o_guess, o_roff;
+  size_t o_cells, o_first, o_cell_of, o_rank, o_feat, o_temp, temp_bytes;
+  size_t o_match, o_near, blocks, o_far, o_nfar, o_pairs, o_np, o_part, o_pd, o_st, o_guess, o_roff;
 };
 
-// Bounding box of the current cloud (host), then the grid: cell h =
-// cbrt(volume / points) (about one cell per point of a surface patch; at
-// least 1 mm), at most 2^24 cells.
-int nn_plan(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cloud *cur, float radius, NNPlan &pl) {
+// The current cloud's bounding box (device; with the clouds' counts in one
+// read-back), then the grid: cell h = kNNCell cbrt(volume / points), at least
+// 1 mm, at most 2^24 cells.  The points lie on surfaces: at 320x240 a point's
+// cell holds about 20.  0.35 / 0.5 / 0.7 / 1.0 / 1.4 measured 1.31 / 1.19 /
+// 1.10 / 1.37 / 1.49 ms per 10-iteration alignment there.
+constexpr double kNNCell = 0.7;
+int nn_plan(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cloud *cur, NNPlan &pl) {
   int rc;
-  int cr[2], cc[2];
-  if ((rc = cloud_counts2(const_cast<nicp_cloud *>(ref), cr)) || (rc = cloud_counts2(const_cast<nicp_cloud *>(cur), cc)))
-    return rc;
-  pl.nr = cr[0];
-  pl.nc = cc[0];
-  std::vector<float4> pts(std::max(pl.nc, 1));
-  if (pl.nc > 0) {
-    CK(ctx, cudaMemcpyAsync(pts.data(), cur->pts, 16 * (size_t)pl.nc, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(ctx, cudaStreamSynchronize(ctx->stream));
+  struct Head {
+    unsigned box[6];
+    int ref[2], cur[2];
+  };
+  Layout B;
+  const size_t o_box = B.take(sizeof(Head::box));
+  if ((rc = ensure_ws(ctx, B.off))) return rc;
+  char *pin;
+  if ((rc = pin_down(ctx, sizeof(Head), &pin))) return rc;
+  Head *head = (Head *)pin;
+  std::memset(head, 0, sizeof(Head));
+  cudaStream_t s = ctx->stream;
+  if (cur->mem) {
+    if (launch_nn_bounds(cur->pts, cur->count, cur->capacity, (unsigned *)(ctx->ws + o_box), s))
+      return fail(ctx, NICP_ECUDA, "bounding box");
+    CK(ctx, cudaMemcpyAsync(head->box, ctx->ws + o_box, sizeof(head->box), cudaMemcpyDeviceToHost, s));
+    CK(ctx, cudaMemcpyAsync(head->cur, cur->count, sizeof(head->cur), cudaMemcpyDeviceToHost, s));
   }
+  if (ref->mem) CK(ctx, cudaMemcpyAsync(head->ref, ref->count, sizeof(head->ref), cudaMemcpyDeviceToHost, s));
+  CK(ctx, cudaStreamSynchronize(s));
+  pl.nr = head->ref[0];
+  pl.nc = head->cur[0];
   float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
-  for (int j = 0; j < pl.nc; j++) {
-    const float v[3] = {pts[j].x, pts[j].y, pts[j].z};
+  if (pl.nc > 0 && head->box[0] <= head->box[3])  // (no finite point: an empty box)
     for (int a = 0; a < 3; a++) {
-      if (j == 0 || v[a] < lo[a]) lo[a] = v[a];
-      if (j == 0 || v[a] > hi[a]) hi[a] = v[a];
+      lo[a] = nn_key_float(head->box[a]);
+      hi[a] = nn_key_float(head->box[3 + a]);
     }
-  }
   double ext[3], vol = 1.0;
   for (int a = 0; a < 3; a++) {
     ext[a] = std::max(1e-3, (double)hi[a] - lo[a]);
     vol *= ext[a];
   }
-  double h = std::max(1e-3, std::cbrt(vol / std::max(pl.nc, 1)));
+  double h = std::max(1e-3, kNNCell * std::cbrt(vol / std::max(pl.nc, 1)));
   for (;;) {
     double cells = 1.0;
     for (int a = 0; a < 3; a++) cells *= std::floor(ext[a] / h) + 1;
@@ -1526,18 +1539,24 @@ int nn_plan(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cloud *cur, float r
   for (int a = 0; a < 3; a++) {
     g.origin[a] = lo[a];
     g.dim[a] = (int)std::floor(ext[a] / h) + 1;
+    // a coordinate's cell comes from three float roundings relative to the
+    // axis (and to the coordinates themselves, for a cloud far from zero)
+    g.slack[a] = (float)(h * (1e-3 + 1e-6 * g.dim[a]) + 5e-7 * std::max(std::fabs(lo[a]), std::fabs(hi[a])));
   }
-  g.max_shell = (int)std::ceil(radius / h) + 1;
   const size_t ncells = (size_t)g.dim[0] * g.dim[1] * g.dim[2];
   const size_t NC = std::max(pl.nc, 1), NR = std::max(pl.nr, 1);
   pl.tiles = (int)((NR + kCorrTilePixels - 1) / kCorrTilePixels);
-  pl.temp_bytes = std::max(nn_temp_bytes((int)NC), nn_temp_bytes((int)NR));
+  pl.temp_bytes = nn_temp_bytes(ncells);
   Layout L;
-  pl.o_keys = L.take(4 * NC); pl.o_skeys = L.take(4 * NC); pl.o_idx = L.take(4 * NC); pl.o_sidx = L.take(4 * NC);
-  pl.o_feat = L.take(24 * NC); pl.o_sfeat = L.take(24 * NC);
-  pl.o_cstart = L.take(4 * ncells); pl.o_cend = L.take(4 * ncells);
+  pl.o_cells = L.take(4 * (ncells + 1));
+  pl.o_first = L.take(4 * (ncells + 1));
+  pl.o_cell_of = L.take(4 * NC); pl.o_rank = L.take(4 * NC);
+  pl.o_feat = L.take(32 * NC);
   pl.o_temp = L.take(pl.temp_bytes);
-  pl.o_match = L.take(4 * NR); pl.o_flag = L.take(4 * NR); pl.o_pos = L.take(4 * NR);
+  pl.o_match = L.take(4 * NR); pl.o_near = L.take(4 * NR);
+  pl.o_far = L.take(4 * NR);
+  pl.blocks = (NR + kNNBlock - 1) / kNNBlock;
+  pl.o_nfar = L.take(4 * (1 + 2 * pl.blocks));
   pl.o_pairs = L.take(8 * NR); pl.o_np = L.take(4);
   pl.o_part = L.take(8 * kPartialWords * (size_t)pl.tiles);
   pl.o_pd = L.take(sizeof(PairDev)); pl.o_st = L.take(sizeof(PairState));
@@ -1553,13 +1572,13 @@ int nn_build(nicp_ctx *ctx, const NNPlan &pl, const nicp_cloud *cur, float nscal
   b.cur_nrm = cur->nrm;
   b.nscale = nscale;
   b.grid = pl.grid;
-  const size_t ncells = (size_t)pl.grid.dim[0] * pl.grid.dim[1] * pl.grid.dim[2];
-  b.key_bits = 1;
-  while (b.key_bits < 32 && ((size_t)1 << b.key_bits) < ncells) b.key_bits++;
-  b.keys = (unsigned *)(ws + pl.o_keys); b.skeys = (unsigned *)(ws + pl.o_skeys);
-  b.idx = (unsigned *)(ws + pl.o_idx); b.sidx = (unsigned *)(ws + pl.o_sidx);
-  b.feat6 = (float *)(ws + pl.o_feat); b.sfeat6 = (float *)(ws + pl.o_sfeat);
-  b.cstart = (int *)(ws + pl.o_cstart); b.cend = (int *)(ws + pl.o_cend);
+  b.cells = (int *)(ws + pl.o_cells);
+  b.first = (int *)(ws + pl.o_first);
+  b.cell_of = (int *)(ws + pl.o_cell_of);
+  b.rank = (int *)(ws + pl.o_rank);
+  b.feat = (float4 *)(ws + pl.o_feat);
+  b.far_count = (int *)(ws + pl.o_nfar);
+  b.zero_bytes = 4 * (1 + 2 * pl.blocks);
   b.temp = ws + pl.o_temp;
   b.temp_bytes = pl.temp_bytes;
   if (launch_nn_build(b, ctx->stream)) return fail(ctx, NICP_ECUDA, "nearest-neighbour index build failed");
@@ -1571,6 +1590,7 @@ NNQuery nn_query(nicp_ctx *ctx, const NNPlan &pl, const nicp_cloud *ref, const n
   char *ws = ctx->ws;
   NNQuery q{};
   q.nr = pl.nr;
+  q.nc = pl.nc;
   q.ref_pts = ref->pts; q.ref_nrm = ref->nrm;
   q.cur_pts = cur->pts; q.cur_nrm = cur->nrm;
   q.Tg = Tg;
@@ -1579,10 +1599,16 @@ NNQuery nn_query(nicp_ctx *ctx, const NNPlan &pl, const nicp_cloud *ref, const n
   q.sq = cp.inlier_distance_threshold * cp.inlier_distance_threshold;
   q.cos_thr = cp.inlier_normal_angular_threshold;
   q.demoted = cp.demoted_to_gicp;
+  q.seeded = 0;
   q.grid = pl.grid;
-  q.cstart = (const int *)(ws + pl.o_cstart); q.cend = (const int *)(ws + pl.o_cend);
-  q.sfeat6 = (const float *)(ws + pl.o_sfeat); q.sidx = (const unsigned *)(ws + pl.o_sidx);
+  q.first = (const int *)(ws + pl.o_first);
+  q.feat = (const float4 *)(ws + pl.o_feat);
   q.match = (int *)(ws + pl.o_match);
+  q.near = (int *)(ws + pl.o_near);
+  q.far = (int *)(ws + pl.o_far);
+  q.far_count = (int *)(ws + pl.o_nfar);
+  q.block_hits = q.far_count + 1;
+  q.next_hits = q.block_hits + pl.blocks;
   return q;
 }
 }  // namespace
@@ -1594,7 +1620,7 @@ extern "C" int nicp_correspond_nn(nicp_ctx *ctx, const nicp_cloud *ref, const ni
   NICP_ON_DEVICE(ctx);
   if (!ctx || !ref || !cur || !T16 || !corr || !num_pairs) return NICP_EINVAL;
   NNPlan pl;
-  int rc = nn_plan(ctx, ref, cur, corr->inlier_distance_threshold, pl);
+  int rc = nn_plan(ctx, ref, cur, pl);
   if (rc) return rc;
   *num_pairs = 0;
   if (pl.nr == 0 || pl.nc == 0) return NICP_OK;
@@ -1606,8 +1632,7 @@ extern "C" int nicp_correspond_nn(nicp_ctx *ctx, const nicp_cloud *ref, const ni
   CK(ctx, cudaMemcpyAsync(ctx->ws + pl.o_guess, pin, 48, cudaMemcpyHostToDevice, s));
   CK(ctx, cudaEventRecord(ctx->pin_up_ev, s));
   NNQuery q = nn_query(ctx, pl, ref, cur, normal_scaling, *corr, (const float *)(ctx->ws + pl.o_guess), nullptr);
-  if (launch_nn_correspond(q, (int *)(ctx->ws + pl.o_flag), (int *)(ctx->ws + pl.o_pos), ctx->ws + pl.o_temp,
-                           pl.temp_bytes, (int32_t *)(ctx->ws + pl.o_pairs), (int *)(ctx->ws + pl.o_np), s))
+  if (launch_nn_correspond(q, (int32_t *)(ctx->ws + pl.o_pairs), (int *)(ctx->ws + pl.o_np), false, s))
     return fail(ctx, NICP_ECUDA, "nearest-neighbour query failed");
   int K = 0;
   CK(ctx, cudaMemcpyAsync(&K, ctx->ws + pl.o_np, 4, cudaMemcpyDeviceToHost, s));
@@ -1631,7 +1656,7 @@ extern "C" int nicp_align_nn(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cl
   if (!ref->mem || !cur->mem || ref->ctx != ctx || cur->ctx != ctx)
     return fail(ctx, NICP_EINVAL, "both clouds must be built on this context");
   NNPlan pl;
-  int rc = nn_plan(ctx, ref, cur, corr->inlier_distance_threshold, pl);
+  int rc = nn_plan(ctx, ref, cur, pl);
   if (rc) return rc;
   if ((rc = nn_build(ctx, pl, cur, normal_scaling))) return rc;
   char *ws = ctx->ws;
@@ -1670,18 +1695,19 @@ extern "C" int nicp_align_nn(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cl
   NNQuery q = nn_query(ctx, pl, ref, cur, normal_scaling, *corr, nullptr, (const PairState *)(ws + pl.o_st));
   for (int i = 0; i < prm->outer_iterations; i++) {
     // correspondences with the state's T^-1 (alignernn.cpp:40-45)
-    if (launch_nn_correspond(q, (int *)(ws + pl.o_flag), (int *)(ws + pl.o_pos), ws + pl.o_temp, pl.temp_bytes,
-                             d.pairs, d.num_pairs, s))
+    if (launch_nn_correspond(q, d.pairs, d.num_pairs, i > 0, s))
       return fail(ctx, NICP_ECUDA, "nearest-neighbour query failed");
+    q.seeded = 1;
+    std::swap(q.block_hits, q.next_hits);
     for (int k = 0; k < prm->inner_iterations; k++) {
-      launch_lin_list(dpd, 1, pl.tiles, lp, 1, 1, nullptr, s, &ctx->prof);
-      launch_solve(dpd, 1, prm->lambda, ((k == prm->inner_iterations - 1) ? 1 : 0) | xb, prm->early_exit_eps, 0, false,
+      launch_lin_list(dpd, 1, pl.tiles, lp, 1, 1, nullptr, true, s, &ctx->prof);
+      launch_solve(dpd, 1, prm->lambda, ((k == prm->inner_iterations - 1) ? 1 : 0) | xb, prm->early_exit_eps, 0, true,
                    s, &ctx->prof);
     }
   }
   if (prm->compute_statistics) {
-    launch_lin_list(dpd, 1, pl.tiles, lp, 1, 2, nullptr, s, &ctx->prof);
-    launch_solve(dpd, 1, 0.0f, 4 | xb, 0.0, 1, false, s, &ctx->prof);
+    launch_lin_list(dpd, 1, pl.tiles, lp, 1, 2, nullptr, true, s, &ctx->prof);
+    launch_solve(dpd, 1, 0.0f, 4 | xb, 0.0, 1, true, s, &ctx->prof);
   }
   CK(ctx, cudaGetLastError());
   PairState st;
@@ -1953,7 +1979,7 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) 
       launch_resolve(dpd, pl.n, pl.max_tiles, 1, nullptr, 0, false, s, &ctx->prof);
       launch_corr_list(dpd, pl.n, pl.total_tiles, cp, 1, nullptr, s, &ctx->prof);
       for (int k = 0; k < inner; k++) {
-        launch_lin_list(dpd, pl.n, pl.total_tiles, lp, std::max(1, a.corr->parity_threads), 1, nullptr, s, &ctx->prof);
+        launch_lin_list(dpd, pl.n, pl.total_tiles, lp, std::max(1, a.corr->parity_threads), 1, nullptr, false, s, &ctx->prof);
         launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, chained, s, &ctx->prof);
       }
     } else {
@@ -1969,7 +1995,7 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) 
     // Aligner::_computeStatistics: one more linearization at the final pose
     // with the last correspondences (aligner.cpp:90-95)
     if (pl.list_mode)
-      launch_lin_list(dpd, pl.n, pl.total_tiles, lp, std::max(1, a.corr->parity_threads), 2, nullptr, s, &ctx->prof);
+      launch_lin_list(dpd, pl.n, pl.total_tiles, lp, std::max(1, a.corr->parity_threads), 2, nullptr, false, s, &ctx->prof);
     else
       launch_corr_lin(dpd, pl.n, pl.total_tiles, pl.max_tiles, cp, lp, 8, pl.structured, L.corr_ctas, tile_pair, s, &ctx->prof);
     launch_solve(dpd, pl.n, 0.0f, 4 | xb, 0.0, 1, chained, s, &ctx->prof);

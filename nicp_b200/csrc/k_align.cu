@@ -1209,6 +1209,7 @@ __global__ void __launch_bounds__(kCorrThreads) k_lin_list(const PairDev *__rest
                                                            const float *__restrict__ explicit_T) {
   int pi = find_pair(pairs, npairs, blockIdx.x);
   const PairDev &pd = pairs[pi];
+  chain();
   if (use_state_T == 1 && pd.state->done) return;
   int tile = blockIdx.x - pd.tile_base;
   int K = *pd.num_pairs;
@@ -1716,9 +1717,10 @@ void launch_corr_list(const PairDev *d_pairs, int npairs, int total_tiles, const
 }
 
 void launch_lin_list(const PairDev *d_pairs, int npairs, int total_tiles, const LinParams &lp, int parity_threads,
-                     int use_state_T, const float *explicit_T, cudaStream_t s, Profiler *prof) {
+                     int use_state_T, const float *explicit_T, bool chained, cudaStream_t s, Profiler *prof) {
   prof->begin(NICP_K_LIN_LIST, s);
-  k_lin_list<<<total_tiles, kCorrThreads, 0, s>>>(d_pairs, npairs, lp, parity_threads, use_state_T, explicit_T);
+  launch(chained, k_lin_list, total_tiles, kCorrThreads, 0, s, d_pairs, npairs, lp, parity_threads, use_state_T,
+         explicit_T);
   prof->end(NICP_K_LIN_LIST, s);
 }
 

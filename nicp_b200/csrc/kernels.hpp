@@ -153,7 +153,7 @@ void launch_corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, int ma
 void launch_corr_list(const PairDev *d_pairs, int npairs, int total_tiles, const CorrParams &cp, int use_state_T,
                       const float *explicit_T, cudaStream_t s, Profiler *prof);
 void launch_lin_list(const PairDev *d_pairs, int npairs, int total_tiles, const LinParams &lp, int parity_threads,
-                     int use_state_T, const float *explicit_T, cudaStream_t s, Profiler *prof);
+                     int use_state_T, const float *explicit_T, bool chained, cudaStream_t s, Profiler *prof);
 // Initialises the pair states and, when tile_pair is given, the tile -> pair
 // table of the fused kernel (total pixel tiles entries).
 void launch_init_pairs(const PairDev *d_pairs, int npairs, const double *d_guesses, const double *d_ref_offsets,
@@ -202,39 +202,49 @@ struct MergeArgs {
 struct NNGrid {
   float origin[3];
   float h, inv_h;
+  float slack[3];  // per axis: how far a point may lie outside its cell by rounding
   int dim[3];
-  int max_shell;  // shells needed to cover the radius
 };
 struct NNBuild {
   int nc;
   const float4 *cur_pts, *cur_nrm;
   float nscale;
   NNGrid grid;
-  int key_bits;
-  unsigned *keys, *skeys, *idx, *sidx;
-  float *feat6, *sfeat6;
-  int *cstart, *cend;
+  int *cells;          // points per cell (and one more entry)
+  int *first;          // first point of each cell in `feat`, and their number
+  int *cell_of, *rank; // per point
+  float4 *feat;        // two per point: (x, y, z, index), scaled normal
+  int *far_count;      // the query's counters, zero_bytes of them
+  size_t zero_bytes;
   void *temp;
   size_t temp_bytes;
 };
+constexpr int kNNBlock = 128;  // reference points and threads per compaction CTA
 struct NNQuery {
-  int nr;
+  int nr, nc;
   const float4 *ref_pts, *ref_nrm;
   const float4 *cur_pts, *cur_nrm;
   const float *Tg;          // rows 0..2 of the transform, or null: the pair state's Tgate
   const PairState *state;
   float nscale, sq, cos_thr;
   int demoted;
+  int seeded;               // near[] holds the candidates of another transform of the same clouds
   NNGrid grid;
-  const int *cstart, *cend;
-  const float *sfeat6;
-  const unsigned *sidx;
-  int *match;
+  const int *first;
+  const float4 *feat;
+  int *match;               // current index or -1
+  int *near;                // place in feat of the nearest point within the radius, or -1
+  int *far, *far_count;     // points left to the wide search, their number (0 before a query)
+  int *block_hits;          // matches per kNNBlock points (0 before a query)
+  int *next_hits;           // the same for the next query: zeroed by this one
 };
-size_t nn_temp_bytes(int n);
+// Keys of the bounding box (minima, then maxima; nn_key_float) of the finite
+// points; box: 6 words.
+int launch_nn_bounds(const float4 *pts, const int *count, int capacity, unsigned *box, cudaStream_t s);
+float nn_key_float(unsigned key);
+size_t nn_temp_bytes(size_t cells);
 int launch_nn_build(const NNBuild &b, cudaStream_t s);
-int launch_nn_correspond(const NNQuery &q, int *flag, int *pos, void *temp, size_t temp_bytes, int32_t *pairs,
-                         int *num_pairs, cudaStream_t s);
+int launch_nn_correspond(const NNQuery &q, int32_t *pairs, int *num_pairs, bool chained, cudaStream_t s);
 
 size_t merge_scan_temp_bytes(int n);
 int launch_merge(const MergeArgs &a, cudaStream_t s);
