@@ -869,7 +869,7 @@ static int build_frames(nicp_ctx *ctx, int n, const FrameIn *fin, const nicp_cam
   char *pin;
   if ((rc = pin_up(ctx, frames_bytes, &pin))) return rc;
   int *tab_all = reinterpret_cast<int *>(pin + sizeof(FrameDev) * n);
-  struct Grid { int tiles, bands, carryctas, max_bands, max_pixels; };
+  struct Grid { int tiles, bands, carryctas, max_bands, max_pixels, max_rows, max_cols; };
   std::vector<Grid> grids(chunks.size());
   for (size_t ci = 0; ci < chunks.size(); ci++) {
     const int i0 = chunks[ci].first, nf = chunks[ci].second - i0;
@@ -887,7 +887,7 @@ static int build_frames(nicp_ctx *ctx, int n, const FrameIn *fin, const nicp_cam
     }
     FrameDev *fd = reinterpret_cast<FrameDev *>(pin) + i0;
     int *tab_t = tab_all + tab_off[ci], *tab_b = tab_t + tab_tiles[ci], *tab_k = tab_b + tab_bands[ci];
-    int tiles = 0, bands = 0, carryctas = 0, max_bands = 0, max_pixels = 0;
+    int tiles = 0, bands = 0, carryctas = 0, max_bands = 0, max_pixels = 0, max_rows = 0, max_cols = 0;
     for (int k = 0; k < nf; k++) {
       const FrameIn &f = fin[i0 + k];
       const nicp_camera &cam = cams[i0 + k];
@@ -910,6 +910,8 @@ static int build_frames(nicp_ctx *ctx, int n, const FrameIn *fin, const nicp_cam
       bands += (f.rows + nb_rows - 1) / nb_rows;
       max_bands = std::max(max_bands, (f.rows + nb_rows - 1) / nb_rows);
       max_pixels = std::max(max_pixels, (int)P);
+      max_rows = std::max(max_rows, f.rows);
+      max_cols = std::max(max_cols, f.cols);
       carryctas += (10 * f.cols + 127) / 128;
       d.depth_scale = prm->depth_scale;
       d.min_d = cam.min_distance;
@@ -961,7 +963,7 @@ static int build_frames(nicp_ctx *ctx, int n, const FrameIn *fin, const nicp_cam
       d.band_tot = unproject_only ? nullptr : (void *)(ctx->ws + o_band[k]);
       d.rowpre = o_rowpre[k] ? (void *)(ctx->ws + o_rowpre[k]) : nullptr;
     }
-    grids[ci] = {tiles, bands, carryctas, max_bands, max_pixels};
+    grids[ci] = {tiles, bands, carryctas, max_bands, max_pixels, max_rows, max_cols};
   }
   FrameDev *dfr_all = (FrameDev *)(ctx->ws + o_frames_all);
   CK(ctx, cudaMemcpyAsync(dfr_all, pin, frames_bytes, cudaMemcpyHostToDevice, s));
@@ -1019,9 +1021,14 @@ static int build_frames(nicp_ctx *ctx, int n, const FrameIn *fin, const nicp_cam
       return fail_staged(e, "cudaStreamWaitEvent");
     const FrameDev *dfr = dfr_all + i0;
     const int *ft = dtab_all + tab_off[ci], *fb = ft + tab_tiles[ci], *fk = fb + tab_bands[ci];
-    launch_unproject(dfr, nf, g.tiles, ft, s, &ctx->prof);
+    const bool few = !unproject_only && moments_row_path(nf);
+    if (few)
+      launch_build_few(prm->moments_precision, dfr, nf, g.max_rows, g.max_cols, g.max_pixels, s, &ctx->prof);
+    else
+      launch_unproject(dfr, nf, g.tiles, ft, s, &ctx->prof);
     if (!unproject_only) {
-      launch_moments(prm->moments_precision, dfr, nf, g.bands, g.carryctas, g.max_bands, fb, fk, s, &ctx->prof);
+      if (!few)
+        launch_moments(prm->moments_precision, dfr, nf, g.bands, g.carryctas, g.max_bands, fb, fk, s, &ctx->prof);
       // only the smallest eigenpair is needed unless Stats are kept or an
       // information matrix has distinct second and third diagonal entries
       const bool lean = !prm->keep_stats && prm->pim_flat[1] == prm->pim_flat[2] &&

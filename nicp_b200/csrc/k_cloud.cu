@@ -87,7 +87,6 @@ __device__ __forceinline__ int block_sum_int(int v, int *smem) {
 __global__ void __launch_bounds__(256) k_unproject_count(const FrameDev *__restrict__ frames,
                                                          const int *__restrict__ frame_of) {
   __shared__ int red[32];
-  chain();
   int fi = frame_of[blockIdx.x];
   const FrameDev &f = frames[fi];
   int tile = blockIdx.x - f.tile_base;
@@ -144,22 +143,13 @@ __device__ __forceinline__ void write_gaussian(const FrameDev &f, float4 *g, flo
 // row-major: within the tile, pixel order is (round, warp, lane) order.
 constexpr int kUnprojRounds = kUnprojTilePixels / 256;
 
-__global__ void __launch_bounds__(256) k_unproject_write(const FrameDev *__restrict__ frames,
-                                                         const int *__restrict__ frame_of) {
-  __shared__ int red[32];
+// One tile of a frame by 256 threads; before: points numbered before it.
+__device__ __forceinline__ void unproject_tile(const FrameDev &f, int tile, int before) {
   __shared__ int rcnt[kUnprojRounds * 8];  // valid pixels per (round, warp), then their exclusive prefix
   __shared__ int wtot[4];
-  int fi = frame_of[blockIdx.x];
-  const FrameDev &f = frames[fi];
-  const int tile = blockIdx.x - f.tile_base;
   const int P = f.rows * f.cols;
   const int ntiles = (P + kUnprojTilePixels - 1) / kUnprojTilePixels;
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  chain();
-  // points numbered before this tile
-  int before = 0;
-  for (int q = t; q < tile; q += blockDim.x) before += f.tile_counts[q];
-  before = block_sum_int(before, red);
   const int base = tile * kUnprojTilePixels + t;
   // The tile's depths come in with 128-bit loads (thread t: bytes 16 t,
   // 16 (t + 256), ... of the tile) into shared memory, from where thread t
@@ -256,6 +246,17 @@ __global__ void __launch_bounds__(256) k_unproject_write(const FrameDev *__restr
     }
     if (p < P) f.index[p] = out;
   }
+}
+
+__global__ void __launch_bounds__(256) k_unproject_write(const FrameDev *__restrict__ frames,
+                                                         const int *__restrict__ frame_of) {
+  __shared__ int red[32];
+  const FrameDev &f = frames[frame_of[blockIdx.x]];
+  const int tile = blockIdx.x - f.tile_base;
+  // points numbered before this tile
+  int before = 0;
+  for (int q = threadIdx.x; q < tile; q += blockDim.x) before += f.tile_counts[q];
+  unproject_tile(f, tile, block_sum_int(before, red));
 }
 
 // ------------------------------------------------------------ moments
@@ -458,7 +459,6 @@ __global__ void __launch_bounds__(kRowThreads) k_moments_band_totals(const Frame
   const int r0 = b * kBandRows, nr = min(f.rows - r0, kBandRows);
   A *tot = static_cast<A *>(f.band_tot) + (size_t)b * 10 * cols;
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  chain();
   A carry[10];
 #pragma unroll
   for (int m = 0; m < 10; m++) carry[m] = A(0);
@@ -549,7 +549,6 @@ __global__ void __launch_bounds__(128) k_moments_band_carry(const FrameDev *__re
   if (q >= (int)stride) return;
   const int nb = (f.rows + kBandRows - 1) / kBandRows;
   A *tot = static_cast<A *>(f.band_tot) + q;
-  chain();
   A acc = A(0);
   for (int b0 = 0; b0 < nb; b0 += kAhead) {
     A v[kAhead];
@@ -946,78 +945,299 @@ void launch_depth_scale(const uint16_t *u16, const float *f32, size_t pitch_elem
 
 void launch_unproject(const FrameDev *d_frames, int nframes, int total_tiles, const int *frame_of_tile, cudaStream_t s,
                       Profiler *prof) {
+  (void)nframes;
   prof->begin(NICP_K_UNPROJECT, s);
   k_unproject_count<<<total_tiles, 256, 0, s>>>(d_frames, frame_of_tile);
-  launch(moments_row_path(nframes), k_unproject_write, total_tiles, 256, 0, s, d_frames, frame_of_tile);
+  k_unproject_write<<<total_tiles, 256, 0, s>>>(d_frames, frame_of_tile);
   prof->end(NICP_K_UNPROJECT, s, 2);
 }
 
-// ---- few-frame path (no more than kRowPathFrames frames per launch).  The
-// sweep walks a band's 16 rows in sequence, which on a single frame leaves
-// the GPU nearly idle.  Here the row prefixes R of every row are computed in
-// parallel (one CTA per image row, row_chunk_scan) into `rowpre`, then one
-// thread per (band, plane, column) adds them down the band onto the band's
-// carry: the sweep's additions in the sweep's order, so the planes are
-// bitwise those of the sweep and results do not depend on how frames are
-// batched.
+// ---- few-frame path (no more than kRowPathFrames frames per launch).  A
+// single frame leaves the kernels above nearly idle: the sweep walks a band's
+// 16 rows in sequence, and every launch waits for the one before.  Here a
+// build is three launches, each with everything that can run at once:
+//   k_build_rows    band totals (a CTA of 640 threads per band, a column per
+//                   thread, then the row scan of two moments per 128
+//                   threads), and the row prefixes R of five image rows per
+//                   CTA into `rowpre`
+//   k_build_planes  the unprojection's tiles (a tile's first number comes
+//                   from the row prefixes of plane 0), and per (band, plane
+//                   pair, column) the band's carry -- the totals above it,
+//                   added in k_moments_band_carry's order -- with R added down
+//                   the band
+//   k_stats
+// Every sum has the sweep's terms in the sweep's order, so the planes are
+// bitwise the sweep's and results do not depend on how frames are batched.
+// 640x480, from the first launch to the end of the planes: 84 us as seven
+// launches (band totals 24, row prefixes 22 with 8-byte stores 40 bytes apart,
+// column sums 12), now 30.
 constexpr int kRowPathFrames = 2;
+constexpr int kFewRows = 5;                              // image rows per CTA of k_build_rows
+constexpr int kFewThreads = kFewRows * kRowThreads;      // 640: also a column each
+static_assert(kFewThreads == kChunkPix, "a band CTA has a thread per column of a chunk");
+static_assert(2 * kFewRows == 10, "two moments per 128 threads");
 
-template <class M>
-__global__ void __launch_bounds__(kRowThreads) k_moments_rowpre(const FrameDev *__restrict__ frames,
-                                                                const int *__restrict__ frame_of) {
-  typedef typename MomAcc<M>::T A;
-  __shared__ A wtot[kRowThreads / 32][10];
-  const int fi = frame_of[blockIdx.x];
-  const FrameDev &f = frames[fi];
-  const int r = ((int)blockIdx.x - f.band_base) * kBandRows + (int)blockIdx.y;
-  if (r >= f.rows) return;  // the whole CTA
-  const int cols = f.cols;
-  const size_t P = (size_t)f.rows * cols;
-  A *Rp = static_cast<A *>(f.rowpre) + (size_t)r * cols;
-  chain();
-  A carry[10];
-#pragma unroll
-  for (int m = 0; m < 10; m++) carry[m] = A(0);
-  for (int x0 = 0; x0 < cols; x0 += kChunkPix) {
-    unsigned w[kRowPix];
-    load_row_raw(f, r, x0 + threadIdx.x * kRowPix, w);
-    float d[kRowPix];
-#pragma unroll
-    for (int k = 0; k < kRowPix; k++) d[k] = depth_from_raw(f, w[k]);
-    row_chunk_scan<M>(f, r, x0, d, carry, wtot, [&](int, int c, const A *acc) {
-      if (c < cols) {
-#pragma unroll
-        for (int m = 0; m < 10; m++) Rp[m * P + c] = acc[m];
-      }
-    });
+// Moment m (a compile-time constant) of a point as point_moments forms it.
+__device__ __forceinline__ double moment_of(int m, float4 p, double v) {
+  const double x = p.x, y = p.y, z = p.z;
+  switch (m) {
+    case 0: return v;
+    case 1: return v * x;
+    case 2: return v * y;
+    case 3: return v * z;
+    case 4: return v * x * x;
+    case 5: return v * x * y;
+    case 6: return v * x * z;
+    case 7: return v * y * y;
+    case 8: return v * y * z;
+    default: return v * z * z;
+  }
+}
+__device__ __forceinline__ float moment_of(int m, float4 p, float v) {
+  switch (m) {
+    case 0: return v;
+    case 1: return v * p.x;
+    case 2: return v * p.y;
+    case 3: return v * p.z;
+    case 4: return v * fm(p.x, p.x);
+    case 5: return v * fm(p.x, p.y);
+    case 6: return v * fm(p.x, p.z);
+    case 7: return v * fm(p.y, p.y);
+    case 8: return v * fm(p.y, p.z);
+    default: return v * fm(p.z, p.z);
   }
 }
 
+// Row prefix of the image row r by 128 threads (their barrier: `bar`).
 template <class M>
-__global__ void __launch_bounds__(128) k_moments_colsum(const FrameDev *__restrict__ frames,
-                                                        const int *__restrict__ frame_of) {
+__device__ __forceinline__ void row_prefix(const FrameDev &f, int r, int bar, typename MomAcc<M>::T (*stage)[kChunkPix],
+                                           typename MomAcc<M>::T (*wtot)[10], typename MomAcc<M>::T *carry) {
   typedef typename MomAcc<M>::T A;
-  const int fi = frame_of[blockIdx.x];
-  const FrameDev &f = frames[fi];
+  auto sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kRowThreads) : "memory"); };
+  const int u = threadIdx.x % kRowThreads, lane = u & 31, w = u >> 5;
   const int cols = f.cols;
-  const int q = ((int)blockIdx.x - f.col_base) * 128 + (int)threadIdx.x;  // plane * cols + column
-  const int b = blockIdx.y, r0 = b * kBandRows;
-  if (q >= 10 * cols || r0 >= f.rows) return;
-  const int r1 = min(f.rows, r0 + kBandRows);
-  const int m = q / cols, c = q - m * cols;
   const size_t P = (size_t)f.rows * cols;
-  chain();
-  A s = static_cast<const A *>(f.band_tot)[(size_t)b * 10 * cols + q];
-  const A *Rp = static_cast<const A *>(f.rowpre) + m * P + c;
-  A v[kBandRows];
+  A *Rp = static_cast<A *>(f.rowpre) + (size_t)r * cols;
+  for (int x0 = 0; x0 < cols; x0 += kChunkPix) {
+    const int c0 = x0 + u * kRowPix;
+    unsigned raw[kRowPix];
+    load_row_raw(f, r, c0, raw);
+    float4 pt[kRowPix];
+    A v[kRowPix];
 #pragma unroll
-  for (int k = 0; k < kBandRows; k++) v[k] = r0 + k < r1 ? Rp[(size_t)(r0 + k) * cols] : A(0);
-#pragma unroll
-  for (int k = 0; k < kBandRows; k++) {
-    if (r0 + k < r1) {
-      s = s + v[k];
-      M::store(f.moments, P, m, (size_t)(r0 + k) * cols + c, (double)s);
+    for (int k = 0; k < kRowPix; k++) {
+      const float d = depth_from_raw(f, raw[k]);
+      const bool valid = c0 + k < cols && depth_valid(d, f.min_d, f.max_d);
+      pt[k] = valid ? unproject_pixel(f.iKRt, c0 + k, r, d) : make_float4(0, 0, 0, 0);
+      v[k] = valid ? A(1) : A(0);
     }
+#pragma unroll
+    for (int m0 = 0; m0 < 10; m0 += 5) {
+      A acc[5];
+#pragma unroll
+      for (int m = 0; m < 5; m++) {
+        A sum = A(0);
+#pragma unroll
+        for (int k = 0; k < kRowPix; k++) sum = sum + moment_of(m0 + m, pt[k], v[k]);
+        A inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const A y = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc = inc + y;
+        }
+        if (lane == 31) wtot[w][m0 + m] = inc;
+        acc[m] = inc - sum;
+      }
+      sync();
+#pragma unroll
+      for (int m = 0; m < 5; m++) {
+        const A left = x0 ? carry[m0 + m] : A(0);
+        A off = left + acc[m], tot = A(0);
+#pragma unroll
+        for (int q = 0; q < kRowThreads / 32; q++) {
+          const A t = wtot[q][m0 + m];
+          if (q < w) off = off + t;
+          tot = tot + t;
+        }
+        acc[m] = off;
+        if (x0 + kChunkPix < cols) {  // (uniform: the chunk to the right needs it)
+          sync();
+          if (u == 0) carry[m0 + m] = left + tot;
+        }
+      }
+      // the values, staged so that consecutive threads store consecutive columns
+#pragma unroll
+      for (int m = 0; m < 5; m++) {
+        A a = acc[m];
+        A *row = stage[(m0 + m) & 1];
+#pragma unroll
+        for (int k = 0; k < kRowPix; k++) {
+          a = a + moment_of(m0 + m, pt[k], v[k]);
+          row[u * kRowPix + k] = a;
+        }
+        sync();
+#pragma unroll
+        for (int j = 0; j < kRowPix; j++) {
+          const int c = x0 + j * kRowThreads + u;
+          if (c < cols) Rp[(size_t)(m0 + m) * P + c] = row[j * kRowThreads + u];
+        }
+      }
+    }
+    sync();  // wtot, carry and the stages have been read
+  }
+}
+
+// Grid (max_bands band CTAs, then row CTAs; frame).
+template <class M>
+__global__ void __launch_bounds__(kFewThreads, 1) k_build_rows(const FrameDev *__restrict__ frames, int max_bands) {
+  typedef typename MomAcc<M>::T A;
+  extern __shared__ __align__(16) unsigned char band_raw[];
+  __shared__ A wtot[kFewRows][kRowThreads / 32][10];
+  __shared__ A carries[kFewRows][10];
+  const FrameDev &f = frames[blockIdx.y];
+  const int t = threadIdx.x, g = t / kRowThreads;
+  chain_next();
+  if ((int)blockIdx.x >= max_bands) {
+    const int r = ((int)blockIdx.x - max_bands) * kFewRows + g;
+    if (r < f.rows)  // (the 128 threads of a row have a barrier of their own)
+      row_prefix<M>(f, r, 1 + g, reinterpret_cast<A (*)[kChunkPix]>(band_raw) + 2 * g, wtot[g], carries[g]);
+    return;
+  }
+  const int b = blockIdx.x, cols = f.cols, r0 = b * kBandRows, nr = min(f.rows - r0, kBandRows);
+  if (b == 0 && t == 0) f.count[1] = 0;  // points with a normal, counted by k_stats
+  if (nr <= 0) return;
+  A(*cs)[kChunkPix] = reinterpret_cast<A (*)[kChunkPix]>(band_raw);
+  A *tot = static_cast<A *>(f.band_tot) + (size_t)b * 10 * cols;
+  const int u = t % kRowThreads, lane = t & 31, w = u >> 5;
+  A carry[2] = {A(0), A(0)};
+  for (int x0 = 0; x0 < cols; x0 += kChunkPix) {
+    const int c = x0 + t;
+    A acc[10];
+#pragma unroll
+    for (int m = 0; m < 10; m++) acc[m] = A(0);
+    if (c < cols) {
+      unsigned raw[kBandRows];
+#pragma unroll
+      for (int i = 0; i < kBandRows; i++) raw[i] = i < nr ? depth_raw(f, (r0 + i) * cols + c) : 0u;
+#pragma unroll
+      for (int i = 0; i < kBandRows; i++) {
+        const float d = depth_from_raw(f, raw[i]);
+        const bool valid = i < nr && depth_valid(d, f.min_d, f.max_d);
+        const float4 p = valid ? unproject_pixel(f.iKRt, c, r0 + i, d) : make_float4(0, 0, 0, 0);
+        A mk[10];
+        point_moments(p, valid, mk);
+#pragma unroll
+        for (int m = 0; m < 10; m++) acc[m] = acc[m] + mk[m];
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 10; m++) cs[m][t] = acc[m];
+    __syncthreads();
+    // inclusive prefix along x of the moments 2g and 2g + 1, in place (thread
+    // u: entries u kRowPix .. u kRowPix + kRowPix - 1)
+    A loc[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const A *row = cs[2 * g + q] + u * kRowPix;
+      A sum = A(0);
+#pragma unroll
+      for (int k = 0; k < kRowPix; k++) sum = sum + row[k];
+      A inc = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const A y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc = inc + y;
+      }
+      if (lane == 31) wtot[g][w][q] = inc;
+      loc[q] = inc - sum;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      A *row = cs[2 * g + q] + u * kRowPix;
+      A off = carry[q] + loc[q], all = A(0);
+#pragma unroll
+      for (int k = 0; k < kRowThreads / 32; k++) {
+        const A x = wtot[g][k][q];
+        if (k < w) off = off + x;
+        all = all + x;
+      }
+      carry[q] = carry[q] + all;
+#pragma unroll
+      for (int k = 0; k < kRowPix; k++) {
+        off = off + row[k];
+        row[k] = off;
+      }
+    }
+    __syncthreads();
+    if (c < cols)
+#pragma unroll
+      for (int m = 0; m < 10; m++) tot[(size_t)m * cols + c] = cs[m][t];
+    __syncthreads();  // the copy-out has read cs before the next chunk overwrites it
+  }
+}
+
+// Grid (max_tiles unprojection tiles, then ncol CTAs of 256 plane-pair columns
+// for each of max_bands bands; frame).
+template <class M>
+__global__ void __launch_bounds__(256) k_build_planes(const FrameDev *__restrict__ frames, int max_tiles, int ncol) {
+  typedef typename MomAcc<M>::T A;
+  __shared__ int red[32];
+  const FrameDev &f = frames[blockIdx.y];
+  const int rows = f.rows, cols = f.cols;
+  const size_t P = (size_t)rows * cols;
+  chain();
+  const A *R = static_cast<const A *>(f.rowpre);
+  if ((int)blockIdx.x < max_tiles) {
+    const size_t p0 = (size_t)blockIdx.x * kUnprojTilePixels;
+    if (p0 >= P) return;
+    // plane 0 counts the points of a row from its left end
+    const int tr = (int)(p0 / cols), tc = (int)(p0 - (size_t)tr * cols);
+    int before = 0;
+    for (int q = threadIdx.x; q < tr; q += 256) before += (int)R[(size_t)q * cols + cols - 1];
+    if (threadIdx.x == 0 && tc > 0) before += (int)R[(size_t)tr * cols + tc - 1];
+    unproject_tile(f, blockIdx.x, block_sum_int(before, red));
+    return;
+  }
+  const int at = (int)blockIdx.x - max_tiles, b = at / ncol, q = (at - b * ncol) * 256 + (int)threadIdx.x;
+  const int r0 = b * kBandRows, k = q / cols, c = q - k * cols;
+  if (k >= 5 || r0 >= rows) return;
+  const size_t stride = (size_t)10 * cols;
+  const A *tot = static_cast<const A *>(f.band_tot) + (size_t)2 * k * cols + c;
+  A s0 = A(0), s1 = A(0);
+  constexpr int kAhead = 8;
+  for (int b0 = 0; b0 < b; b0 += kAhead) {
+    A v0[kAhead], v1[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; i++) {
+      const A *x = tot + (size_t)min(b0 + i, b - 1) * stride;
+      v0[i] = x[0];
+      v1[i] = x[cols];
+    }
+#pragma unroll
+    for (int i = 0; i < kAhead; i++)
+      if (b0 + i < b) {
+        s0 = s0 + v0[i];
+        s1 = s1 + v1[i];
+      }
+  }
+  const A *Rp = R + (size_t)2 * k * P + c;
+#pragma unroll
+  for (int h = 0; h < kBandRows; h += kAhead) {
+    A v0[kAhead], v1[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; i++) {
+      const size_t x = (size_t)min(r0 + h + i, rows - 1) * cols;
+      v0[i] = Rp[x];
+      v1[i] = Rp[P + x];
+    }
+#pragma unroll
+    for (int i = 0; i < kAhead; i++)
+      if (r0 + h + i < rows) {
+        s0 = s0 + v0[i];
+        s1 = s1 + v1[i];
+        M::store2(f.moments, P, k, (size_t)(r0 + h + i) * cols + c, (double)s0, (double)s1);
+      }
   }
 }
 
@@ -1036,6 +1256,7 @@ static void configure_bands() {
   auto set = [] {
     cudaFuncSetAttribute(k_moments_band_totals<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, band_smem_bytes<M>());
     cudaFuncSetAttribute(k_moments_band_sweep<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, band_smem_bytes<M>());
+    cudaFuncSetAttribute(k_build_rows<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, band_smem_bytes<M>());
   };
   if (dev >= 0 && dev < kMaxDevices)
     std::call_once(once[dev], set);
@@ -1047,20 +1268,36 @@ template <class M>
 static void launch_bands(const FrameDev *d_frames, int nframes, int total_bands, int total_carry_ctas, int max_bands,
                          const int *frame_of_band, const int *frame_of_carry, cudaStream_t s, Profiler *prof) {
   configure_bands<M>();
-  const bool chained = moments_row_path(nframes);
   prof->begin(NICP_K_MOMENTS_BANDS, s);
-  launch(chained, k_moments_band_totals<M>, total_bands, kRowThreads, band_smem_bytes<M>(), s, d_frames, frame_of_band);
-  launch(chained, k_moments_band_carry<M>, total_carry_ctas, 128, 0, s, d_frames, frame_of_carry);
+  k_moments_band_totals<M><<<total_bands, kRowThreads, band_smem_bytes<M>(), s>>>(d_frames, frame_of_band);
+  k_moments_band_carry<M><<<total_carry_ctas, 128, 0, s>>>(d_frames, frame_of_carry);
   prof->end(NICP_K_MOMENTS_BANDS, s, 2);
   prof->begin(NICP_K_MOMENTS_SWEEP, s);
-  if (moments_row_path(nframes) && max_bands <= 65535) {  // (grid y of the column sums)
-    launch(chained, k_moments_rowpre<M>, dim3(total_bands, kBandRows), kRowThreads, 0, s, d_frames, frame_of_band);
-    launch(chained, k_moments_colsum<M>, dim3(total_carry_ctas, max_bands), 128, 0, s, d_frames, frame_of_carry);
-    prof->end(NICP_K_MOMENTS_SWEEP, s, 2);
-  } else {
-    k_moments_band_sweep<M><<<dim3(max_bands, nframes), kRowThreads, band_smem_bytes<M>(), s>>>(d_frames, nframes);
-    prof->end(NICP_K_MOMENTS_SWEEP, s);
-  }
+  k_moments_band_sweep<M><<<dim3(max_bands, nframes), kRowThreads, band_smem_bytes<M>(), s>>>(d_frames, nframes);
+  prof->end(NICP_K_MOMENTS_SWEEP, s);
+}
+
+template <class M>
+static void launch_few(const FrameDev *d_frames, int nframes, int max_rows, int max_cols, int max_pixels, cudaStream_t s,
+                       Profiler *prof) {
+  configure_bands<M>();
+  const int bands = (max_rows + kBandRows - 1) / kBandRows, row_ctas = (max_rows + kFewRows - 1) / kFewRows;
+  prof->begin(NICP_K_MOMENTS_BANDS, s);
+  k_build_rows<M><<<dim3(bands + row_ctas, nframes), kFewThreads, band_smem_bytes<M>(), s>>>(d_frames, bands);
+  prof->end(NICP_K_MOMENTS_BANDS, s);
+  const int tiles = (max_pixels + kUnprojTilePixels - 1) / kUnprojTilePixels;
+  const int ncol = (int)((5 * (long long)max_cols + 255) / 256);
+  prof->begin(NICP_K_MOMENTS_SWEEP, s);
+  launch(true, k_build_planes<M>, dim3(tiles + ncol * bands, nframes), 256, 0, s, d_frames, tiles, ncol);
+  prof->end(NICP_K_MOMENTS_SWEEP, s);
+}
+
+void launch_build_few(int precision, const FrameDev *d_frames, int nframes, int max_rows, int max_cols, int max_pixels,
+                      cudaStream_t s, Profiler *prof) {
+  if (precision == NICP_MOMENTS_F32) launch_few<MomF32>(d_frames, nframes, max_rows, max_cols, max_pixels, s, prof);
+  else if (precision == NICP_MOMENTS_TWOFLOAT)
+    launch_few<MomTwoFloat>(d_frames, nframes, max_rows, max_cols, max_pixels, s, prof);
+  else launch_few<MomF64>(d_frames, nframes, max_rows, max_cols, max_pixels, s, prof);
 }
 
 int moment_band_rows() { return kBandRows; }

@@ -87,7 +87,6 @@ struct Profiler {
 
 // frame_of_*: the frame of each CTA of the 1-D build grids (unprojection
 // tiles, 16-row bands, band-carry CTAs), filled on the host.
-// (A build of few frames -- moments_row_path -- chains its launches.)
 void launch_unproject(const FrameDev *d_frames, int nframes, int total_tiles, const int *frame_of_tile, cudaStream_t s,
                       Profiler *prof);
 void launch_depth_scale(const uint16_t *u16, const float *f32, size_t pitch_elems, int rows, int cols,
@@ -95,10 +94,14 @@ void launch_depth_scale(const uint16_t *u16, const float *f32, size_t pitch_elem
 // Integral image over 16-row bands (moment_band_rows()): total_bands band
 // CTAs, total_carry_ctas = sum over frames of ceil(10 cols / 128).
 int moment_band_rows();
-// Few-frame launches (moments_row_path) compute every row prefix in parallel
+// Few-frame builds (moments_row_path) compute every row prefix in parallel
 // into FrameDev::rowpre (10 planes of moment_acc_bytes per pixel) instead of
-// sweeping the bands; the planes are bitwise the same.
+// sweeping the bands, and unproject beside it: launch_build_few takes the place
+// of launch_unproject and launch_moments (counted as moments); the planes are
+// bitwise the same.
 bool moments_row_path(int nframes);
+void launch_build_few(int precision, const FrameDev *d_frames, int nframes, int max_rows, int max_cols, int max_pixels,
+                      cudaStream_t s, Profiler *prof);
 size_t moment_acc_bytes(int precision);
 // Resident band-sweep CTAs per SM (one per 16-row band and frame): frame
 // chunks of whole waves of them leave no half-empty last wave.
