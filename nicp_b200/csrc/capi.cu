@@ -1179,7 +1179,7 @@ struct PairPlan {
   bool structured = false;  // every current cloud has structured Omegas (k_corr_lin<true>)
   int total_tiles = 0, max_pt_tiles = 0;  // max_pt_tiles: 1024-point tiles of the largest projected cloud
   int max_tiles = 0;                      // pixel tiles of the largest pair image
-  size_t o_pairs = 0, o_states = 0, o_krt = 0, o_guess = 0, o_roff = 0, o_zbuf = 0, zbuf_bytes = 0;
+  size_t o_pairs = 0, o_states = 0, o_krt = 0, o_zbuf = 0, zbuf_bytes = 0;
   size_t o_tile_pair = 0;  // int per pixel tile: its pair
   std::vector<size_t> o_cur, o_ref, o_part, o_list, o_ltc, o_np;
   std::vector<int> P, tiles;
@@ -1196,8 +1196,6 @@ static int plan_pairs(nicp_ctx *ctx, int n, const nicp_camera *cams, const nicp_
   pl.o_pairs = L.take(sizeof(PairDev) * n);
   pl.o_states = L.take(sizeof(PairState) * n);
   pl.o_krt = L.take(48 * (size_t)n);
-  pl.o_guess = L.take(128 * (size_t)n);
-  pl.o_roff = L.take(128 * (size_t)n);
   size_t ztot = 0;
   pl.P.resize(n);
   pl.tiles.resize(n);
@@ -1489,7 +1487,7 @@ struct NNPlan {
   int nr = 0, nc = 0, tiles = 0;
   NNGrid grid{};
   size_t o_cells, o_first, o_cell_of, o_rank, o_feat, o_temp, temp_bytes;
-  size_t o_match, o_near, blocks, o_far, o_nfar, o_pairs, o_np, o_part, o_pd, o_st, o_guess, o_roff;
+  size_t o_match, o_near, blocks, o_far, o_nfar, o_pairs, o_np, o_part, o_pd, o_st, o_guess;
 };
 
 // The current cloud's bounding box (device; with the clouds' counts in one
@@ -1567,7 +1565,7 @@ int nn_plan(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cloud *cur, NNPlan 
   pl.o_pairs = L.take(8 * NR); pl.o_np = L.take(4);
   pl.o_part = L.take(8 * kPartialWords * (size_t)pl.tiles);
   pl.o_pd = L.take(sizeof(PairDev)); pl.o_st = L.take(sizeof(PairState));
-  pl.o_guess = L.take(128); pl.o_roff = L.take(128);
+  pl.o_guess = L.take(48);
   return ensure_ws(ctx, L.off);
 }
 
@@ -1691,14 +1689,17 @@ extern "C" int nicp_align_nn(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cl
   for (int k = 0; k < 16; k++) gs[k] = G.a[k];
   double *ro = gs + 16;
   for (int k = 0; k < 16; k++) ro[k] = (k % 5 == 0) ? 1.0 : 0.0;
-  CK(ctx, cudaMemcpyAsync(ws + pl.o_pd, pin, sizeof(PairDev), cudaMemcpyHostToDevice, s));
-  CK(ctx, cudaMemcpyAsync(ws + pl.o_guess, gs, 256, cudaMemcpyHostToDevice, s));
-  CK(ctx, cudaEventRecord(ctx->pin_up_ev, s));
   const PairDev *dpd = (const PairDev *)(ws + pl.o_pd);
   LinParams lp = lin_params(*lin);
   const int xb = lin->cross_block_f32 ? kSolveCrossF32 : 0;
-  launch_init_pairs(dpd, 1, (const double *)(ws + pl.o_guess), (const double *)(ws + pl.o_guess + 128), nullptr, 0,
-                    false, s, &ctx->prof);
+  BeginArgs begin{};
+  begin.pairs = &d;
+  begin.guess = gs;
+  begin.roff = ro;
+  begin.npairs = 1;
+  begin.dev_pairs = (PairDev *)(ws + pl.o_pd);
+  launch_begin_loop(begin, s, &ctx->prof);
+  CK(ctx, cudaEventRecord(ctx->pin_up_ev, s));
   NNQuery q = nn_query(ctx, pl, ref, cur, normal_scaling, *corr, nullptr, (const PairState *)(ws + pl.o_st));
   for (int i = 0; i < prm->outer_iterations; i++) {
     // correspondences with the state's T^-1 (alignernn.cpp:40-45)
@@ -1716,10 +1717,12 @@ extern "C" int nicp_align_nn(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cl
     launch_lin_list(dpd, 1, pl.tiles, lp, 1, 2, nullptr, true, s, &ctx->prof);
     launch_solve(dpd, 1, 0.0f, 4 | xb, 0.0, 1, true, s, &ctx->prof);
   }
+  char *res;
+  if ((rc = pin_down(ctx, sizeof(PairState), &res))) return rc;
+  launch_publish((const PairState *)(ws + pl.o_st), (PairState *)res, 1, true, s, &ctx->prof);
   CK(ctx, cudaGetLastError());
-  PairState st;
-  CK(ctx, cudaMemcpyAsync(&st, ws + pl.o_st, sizeof(PairState), cudaMemcpyDeviceToHost, s));
   CK(ctx, cudaStreamSynchronize(s));
+  const PairState &st = *(const PairState *)res;
   std::memcpy(out->T, st.T, sizeof(out->T));
   out->error = st.error;
   out->inliers = st.inliers;
@@ -1955,6 +1958,8 @@ struct AlignCall {
   const nicp_align_params *prm;
   bool graph;
   bool foreign_clouds = false;  // clouds of another context on the same device (the server's workers)
+  BeginArgs begin{};             // the loop's input and its results, in the context's pinned memory
+  PairState *results = nullptr;
 };
 }  // namespace
 
@@ -1970,13 +1975,19 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) 
   const int xb = a.lin->cross_block_f32 ? kSolveCrossF32 : 0;
   // (list mode's kernels and the general fused kernel are not part of a chain)
   const bool chained = pl.structured && few_tiles(pl.n, pl.max_tiles);
-  cudaMemsetAsync(ctx->ws + pl.o_zbuf, 0xff, pl.zbuf_bytes, s);
   int *tile_pair = (int *)(ctx->ws + pl.o_tile_pair);
-  launch_init_pairs(dpd, pl.n, (const double *)(ctx->ws + pl.o_guess), (const double *)(ctx->ws + pl.o_roff),
-                    tile_pair, pl.max_tiles, chained, s, &ctx->prof);
+  BeginArgs begin = a.begin;
+  begin.npairs = pl.n;
+  begin.dev_pairs = (PairDev *)(ctx->ws + pl.o_pairs);
+  begin.dev_krt = (float *)(ctx->ws + pl.o_krt);
+  begin.tile_pair = tile_pair;
+  begin.zbuf = (uint4 *)(ctx->ws + pl.o_zbuf);
+  begin.zbuf16 = pl.zbuf_bytes / 16;  // (a multiple of 256 bytes)
+  launch_begin_loop(begin, s, &ctx->prof);
   // current cloud, seen from its sensor offset, projected once (alignerprojective.cpp:36-39)
   const nicp_ctx::Launch &L = ctx->launch;
-  launch_zbuffer(dpd, pl.n, pl.max_pt_tiles, 0, (const float *)(ctx->ws + pl.o_krt), L.zb_ppt, chained, s, &ctx->prof);
+  // (not chained: its CTAs read the descriptors that the launch before writes)
+  launch_zbuffer(dpd, pl.n, pl.max_pt_tiles, 0, (const float *)(ctx->ws + pl.o_krt), L.zb_ppt, false, s, &ctx->prof);
   // outside list (parity) mode, current pixels whose point has no normal are
   // dropped from the index image: the gates would reject them anyway
   launch_resolve(dpd, pl.n, pl.max_tiles, 0, nullptr, (pl.list_mode || cp.demoted) ? 0 : 1, chained, s, &ctx->prof);
@@ -2007,12 +2018,15 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) 
       launch_corr_lin(dpd, pl.n, pl.total_tiles, pl.max_tiles, cp, lp, 8, pl.structured, L.corr_ctas, tile_pair, s, &ctx->prof);
     launch_solve(dpd, pl.n, 0.0f, 4 | xb, 0.0, 1, chained, s, &ctx->prof);
   }
+  launch_publish((const PairState *)(ctx->ws + pl.o_states), a.results, pl.n, chained, s, &ctx->prof);
 }
 
 static std::string graph_key(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) {
   std::string k;
   auto put = [&](const void *p, size_t n) { k.append((const char *)p, n); };
   put(&ctx->ws, sizeof(ctx->ws));
+  put(&a.begin, sizeof(a.begin));  // (baked into the graph)
+  put(&a.results, sizeof(a.results));
   put(&pl.n, sizeof(int));
   put(&pl.keep_ref, 1);
   put(&pl.list_mode, 1);
@@ -2100,7 +2114,7 @@ static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
   return rc;
 }
 
-static int align_impl(nicp_ctx *ctx, const AlignCall &a, nicp_align_result *out) {
+static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
   if (!ctx || a.n < 0 || !a.cams || !a.corr || !a.lin || !a.prm || (a.n > 0 && (!a.refs || !a.curs || !out)))
     return NICP_EINVAL;
   if (a.n == 0) return NICP_OK;
@@ -2158,11 +2172,13 @@ static int align_impl(nicp_ctx *ctx, const AlignCall &a, nicp_align_result *out)
     }
   }
   cudaStream_t s = ctx->stream;
-  CK(ctx, cudaMemcpyAsync(ctx->ws + pl.o_pairs, pd, sizeof(PairDev) * a.n, cudaMemcpyHostToDevice, s));
-  CK(ctx, cudaMemcpyAsync(ctx->ws + pl.o_krt, krt, 48 * (size_t)a.n, cudaMemcpyHostToDevice, s));
-  CK(ctx, cudaMemcpyAsync(ctx->ws + pl.o_guess, gs, 128 * (size_t)a.n, cudaMemcpyHostToDevice, s));
-  CK(ctx, cudaMemcpyAsync(ctx->ws + pl.o_roff, ro, 128 * (size_t)a.n, cudaMemcpyHostToDevice, s));
-  CK(ctx, cudaEventRecord(ctx->pin_up_ev, s));
+  char *res;
+  if ((rc = pin_down(ctx, sizeof(PairState) * a.n, &res))) return rc;
+  a.begin.pairs = pd;
+  a.begin.krt = krt;
+  a.begin.guess = gs;
+  a.begin.roff = ro;
+  a.results = (PairState *)res;
   ctx->h2d_bytes += (sizeof(PairDev) + 48 + 256) * (unsigned long long)a.n;
   ctx->launch = nicp_ctx::Launch();
   ctx->launch.zb_ppt = default_zb_ppt(ctx, pl);
@@ -2217,9 +2233,7 @@ static int align_impl(nicp_ctx *ctx, const AlignCall &a, nicp_align_result *out)
     enqueue_loop(ctx, pl, a);
   }
   CK(ctx, cudaGetLastError());
-  char *res;
-  if ((rc = pin_down(ctx, sizeof(PairState) * a.n, &res))) return rc;
-  CK(ctx, cudaMemcpyAsync(res, ctx->ws + pl.o_states, sizeof(PairState) * a.n, cudaMemcpyDeviceToHost, s));
+  CK(ctx, cudaEventRecord(ctx->pin_up_ev, s));  // (the loop reads its input from pinned memory)
   ctx->d2h_bytes += sizeof(PairState) * (unsigned long long)a.n;
   CK(ctx, cudaStreamSynchronize(s));
   const PairState *st = (const PairState *)res;

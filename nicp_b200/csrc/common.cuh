@@ -451,24 +451,4 @@ __device__ inline void d_quaternion(const double *T, double *q, double &n) {
   q[0] = qx; q[1] = qy; q[2] = qz; q[3] = qw;
 }
 
-__device__ inline void d_mm4(const double *A, const double *B, double *C) {
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-      C[i * 4 + j] = A[i * 4 + 0] * B[0 * 4 + j] + A[i * 4 + 1] * B[1 * 4 + j] + A[i * 4 + 2] * B[2 * 4 + j] +
-                     A[i * 4 + 3] * B[3 * 4 + j];
-}
-
-__device__ inline void d_iso_inverse(const double *T, double *R) {
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++) R[i * 4 + j] = T[j * 4 + i];
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-    R[i * 4 + 3] = -(R[i * 4 + 0] * T[3] + R[i * 4 + 1] * T[7] + R[i * 4 + 2] * T[11]);
-  R[12] = 0; R[13] = 0; R[14] = 0; R[15] = 1;
-}
-
 }  // namespace nicp

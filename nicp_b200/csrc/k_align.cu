@@ -1237,53 +1237,6 @@ __global__ void __launch_bounds__(kCorrThreads) k_lin_list(const PairDev *__rest
 }
 
 // ------------------------------------------------------------ solve
-__device__ inline void float12_of(const double *T, float *o) {
-  for (int i = 0; i < 3; i++)
-    for (int j = 0; j < 4; j++) o[i * 4 + j] = (float)T[i * 4 + j];
-}
-
-// KRt of the projector placed at X (pinholepointprojector.cpp:16-31), in FP64.
-__device__ inline void krt_of(const float *K, const double *X, float *o) {
-  double t[16];
-  d_iso_inverse(X, t);
-  for (int i = 0; i < 3; i++) {
-    for (int j = 0; j < 3; j++)
-      o[i * 4 + j] = (float)((double)K[i * 3 + 0] * t[0 * 4 + j] + (double)K[i * 3 + 1] * t[1 * 4 + j] +
-                             (double)K[i * 3 + 2] * t[2 * 4 + j]);
-    o[i * 4 + 3] = (float)((double)K[i * 3 + 0] * t[3] + (double)K[i * 3 + 1] * t[7] + (double)K[i * 3 + 2] * t[11]);
-  }
-}
-
-// Prepares the matrices of an outer iteration from st->T.
-__device__ inline void begin_outer(const PairDev &pd, PairState *st) {
-  for (int k = 0; k < 16; k++) st->Tstart[k] = st->T[k];
-  double X[16];
-  d_mm4(st->T, st->ref_offset, X);
-  krt_of(pd.K, X, st->KRt);
-  d_iso_inverse(st->T, st->invT);
-  float12_of(st->invT, st->Tgate);
-  float12_of(st->invT, st->Tlin);
-}
-
-__global__ void k_init_pairs(const PairDev *__restrict__ pairs, int npairs, const double *__restrict__ guesses,
-                             const double *__restrict__ ref_offsets) {
-  int pi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pi >= npairs) return;
-  const PairDev &pd = pairs[pi];
-  PairState *st = pd.state;
-  for (int k = 0; k < 16; k++) {
-    st->T[k] = guesses[16 * pi + k];
-    st->ref_offset[k] = ref_offsets[16 * pi + k];
-  }
-  st->T[12] = 0; st->T[13] = 0; st->T[14] = 0; st->T[15] = 1;
-  st->error = 0; st->inliers = 0; st->num_corr = 0; st->candidates = 0;
-  st->iterations = 0; st->done = 0; st->status = 0;
-  for (int k = 0; k < 36; k++) st->H[k] = 0;
-  for (int k = 0; k < 6; k++) st->b[k] = 0;
-  begin_outer(pd, st);
-  for (int k = 0; k < 12; k++) st->Tgate_used[k] = st->Tgate[k];
-}
-
 // ---- the 6x6 solve and the pose update, by one warp.
 // The chain of divisions, square roots and 4x4 products is short on work and
 // long on latency, so a lane owns an entry, independent divisions run in
@@ -1419,6 +1372,28 @@ __device__ __forceinline__ void warp_t2v(const double *T, double *x, int lane) {
   }
 }
 
+// The matrices of an outer iteration that starts from sc.T (rows 0..3 of the
+// pose), by one warp: T and its inverse, the projector's KRt for the pose
+// T ref_offset (pinholepointprojector.cpp:16-31), the float transforms of the
+// gates and the linearizer.  K: lane < 12 the row lane / 4 of the camera matrix.
+__device__ __forceinline__ void warp_begin_outer(PairState *st, SolveScratch &sc, const double K[3], int lane) {
+  warp_mm4(sc.T, sc.off, sc.A, lane);
+  warp_iso_inverse(sc.A, sc.B, lane);  // the projector's inverse pose
+  warp_iso_inverse(sc.T, sc.A, lane);  // invT
+  if (lane < 16) {
+    st->T[lane] = sc.T[lane];
+    st->Tstart[lane] = sc.T[lane];
+    st->invT[lane] = sc.A[lane];
+  }
+  if (lane < 12) {
+    const int j = lane & 3;
+    st->KRt[lane] = (float)(K[0] * sc.B[j] + K[1] * sc.B[4 + j] + K[2] * sc.B[8 + j]);
+    const float f = (float)sc.A[lane];
+    st->Tgate[lane] = f;
+    st->Tlin[lane] = f;
+  }
+}
+
 // ---- the sum of a pair's tile partials: kSumGroups warps take the tiles
 // t = g, g + kSumGroups, ... each, then the groups are added; a fixed order,
 // whatever the batch.  (Four groups, as before, left one SM with 75 partials
@@ -1551,36 +1526,65 @@ __global__ void __launch_bounds__(kSumThreads) k_solve(const PairDev *__restrict
     if (lane == 0 && m < early_eps) st->done = 1;
     __syncwarp();
   }
-  // the next outer iteration starts from T (as begin_outer)
-  warp_mm4(sc.T, sc.off, sc.A, lane);
-  warp_iso_inverse(sc.A, sc.B, lane);  // the projector's inverse pose
-  warp_iso_inverse(sc.T, sc.A, lane);  // invT
-  if (lane < 16) {
-    st->T[lane] = sc.T[lane];
-    st->Tstart[lane] = sc.T[lane];
-    st->invT[lane] = sc.A[lane];
-  }
-  if (lane < 12) {
-    const int j = lane & 3;
-    st->KRt[lane] = (float)(K[0] * sc.B[j] + K[1] * sc.B[4 + j] + K[2] * sc.B[8 + j]);
-    const float f = (float)sc.A[lane];
-    st->Tgate[lane] = f;
-    st->Tlin[lane] = f;
-  }
+  warp_begin_outer(st, sc, K, lane);  // the next outer iteration starts from T
 }
 
-// tile_pair[tile] = the pair whose pixel image holds the tile (grid: tiles
-// of a pair, pair), so that the persistent fused kernel finds a tile's pair
-// with one load instead of a search.
-__global__ void k_tile_pairs(const PairDev *__restrict__ pairs, int npairs, int *__restrict__ tile_pair, int pair0) {
-  const int pi = pair0 + (int)blockIdx.y;
-  if (pi >= npairs) return;
-  const PairDev &pd = pairs[pi];
-  chain();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ntiles = (pd.rows * pd.cols + kCorrTilePixels - 1) / kCorrTilePixels;
-  if (t < ntiles) tile_pair[pd.tile_base + t] = pi;
+// Everything a loop starts from, in one launch (four uploads, a memset and two
+// small kernels took 28 us in front of a 20 us iteration): the descriptors,
+// projection matrices and poses are read where the host wrote them (pinned
+// memory), the pairs' states initialised, the tile -> pair table filled
+// (tile_pair[tile] = the pair whose pixel image holds the tile, so that the
+// persistent fused kernel finds it with one load) and the z-buffers emptied.
+// CTA b: pairs b, b + gridDim.x, ..., and its share of the z-buffers.
+__global__ void __launch_bounds__(256) k_begin_loop(BeginArgs a) {
+  __shared__ SolveScratch sc;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  chain_next();
+  for (int pi = blockIdx.x; pi < a.npairs; pi += gridDim.x) {
+    const PairDev &src = a.pairs[pi];
+    if (wid == 0) {
+      PairState *st = src.state;
+      double K[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        if (lane < 12) K[k] = (double)src.K[(lane >> 2) * 3 + k];
+      __syncwarp();  // (the pair before is done with sc)
+      if (lane < 16) {
+        sc.T[lane] = lane < 12 ? a.guess[16 * (size_t)pi + lane] : lane == 15 ? 1.0 : 0.0;
+        const double r = a.roff[16 * (size_t)pi + lane];
+        sc.off[lane] = r;
+        st->ref_offset[lane] = r;
+      }
+      __syncwarp();
+      warp_begin_outer(st, sc, K, lane);
+      if (lane < 12) st->Tgate_used[lane] = st->Tgate[lane];
+      for (int k = lane; k < 36; k += 32) st->H[k] = 0.0;
+      if (lane < 6) st->b[lane] = 0.0;
+      if (lane == 0) {
+        st->error = 0;
+        st->inliers = st->num_corr = st->candidates = st->iterations = st->done = st->status = 0;
+      }
+    } else if (wid == 1) {
+      const unsigned *from = reinterpret_cast<const unsigned *>(&src);
+      unsigned *to = reinterpret_cast<unsigned *>(a.dev_pairs + pi);
+      for (int k = lane; k < (int)(sizeof(PairDev) / 4); k += 32) to[k] = from[k];
+      if (a.dev_krt && lane < 12) a.dev_krt[12 * (size_t)pi + lane] = a.krt[12 * (size_t)pi + lane];
+    } else if (a.tile_pair) {
+      const int ntiles = (src.rows * src.cols + kCorrTilePixels - 1) / kCorrTilePixels;
+      for (int k = t - 64; k < ntiles; k += 192) a.tile_pair[src.tile_base + k] = pi;
+    }
+  }
+  const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
+  for (size_t k = (size_t)blockIdx.x * 256 + t; k < a.zbuf16; k += (size_t)gridDim.x * 256) a.zbuf[k] = ones;
 }
+
+// The pairs' states to the host (pinned memory), chained to the loop's last solve.
+__global__ void __launch_bounds__(256) k_publish(const uint4 *__restrict__ states, uint4 *__restrict__ host, size_t n) {
+  chain();
+  for (size_t k = (size_t)blockIdx.x * 256 + threadIdx.x; k < n; k += (size_t)gridDim.x * 256)
+    host[k] = __ldcg(states + k);
+}
+static_assert(sizeof(PairState) % 16 == 0 && sizeof(PairDev) % 4 == 0, "copied by words");
 
 // ------------------------------------------------------------ launchers
 // An SM changes its split of shared memory and L1 only while it is empty.
@@ -1724,17 +1728,22 @@ void launch_lin_list(const PairDev *d_pairs, int npairs, int total_tiles, const 
   prof->end(NICP_K_LIN_LIST, s);
 }
 
-void launch_init_pairs(const PairDev *d_pairs, int npairs, const double *d_guesses, const double *d_ref_offsets,
-                       int *tile_pair, int max_tiles, bool chained, cudaStream_t s, Profiler *prof) {
+void launch_begin_loop(const BeginArgs &a, cudaStream_t s, Profiler *prof) {
   configure_loop();
   prof->begin(NICP_K_SOLVE, s);
-  k_init_pairs<<<(npairs + 63) / 64, 64, 0, s>>>(d_pairs, npairs, d_guesses, d_ref_offsets);
-  const int kMaxGridY = 65535;
-  if (tile_pair && max_tiles > 0)
-    for (int p0 = 0; p0 < npairs; p0 += kMaxGridY)
-      launch(chained, k_tile_pairs, dim3((max_tiles + 255) / 256, std::min(kMaxGridY, npairs - p0)), 256, 0, s,
-                     d_pairs, npairs, tile_pair, p0);
-  prof->end(NICP_K_SOLVE, s, tile_pair && max_tiles > 0 ? 2 : 1);
+  // a CTA per pair, and for the z-buffers 16 stores per thread up to eight CTAs per SM
+  const size_t want = std::max<size_t>(a.npairs, (a.zbuf16 + 16 * 256 - 1) / (16 * 256));
+  k_begin_loop<<<(unsigned)std::min<size_t>(want, 8 * 148), 256, 0, s>>>(a);
+  prof->end(NICP_K_SOLVE, s);
+}
+
+void launch_publish(const PairState *states, PairState *host, int npairs, bool chained, cudaStream_t s,
+                    Profiler *prof) {
+  prof->begin(NICP_K_SOLVE, s);
+  const size_t n = (size_t)npairs * (sizeof(PairState) / 16);
+  launch(chained, k_publish, (unsigned)std::min<size_t>((n + 255) / 256, 148), 256, 0, s, (const uint4 *)states,
+         (uint4 *)host, n);
+  prof->end(NICP_K_SOLVE, s);
 }
 
 void launch_solve(const PairDev *d_pairs, int npairs, float lambda, int mode, double early_eps, int ignore_done,

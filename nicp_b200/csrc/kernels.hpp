@@ -157,10 +157,25 @@ void launch_corr_list(const PairDev *d_pairs, int npairs, int total_tiles, const
                       const float *explicit_T, cudaStream_t s, Profiler *prof);
 void launch_lin_list(const PairDev *d_pairs, int npairs, int total_tiles, const LinParams &lp, int parity_threads,
                      int use_state_T, const float *explicit_T, bool chained, cudaStream_t s, Profiler *prof);
-// Initialises the pair states and, when tile_pair is given, the tile -> pair
-// table of the fused kernel (total pixel tiles entries).
-void launch_init_pairs(const PairDev *d_pairs, int npairs, const double *d_guesses, const double *d_ref_offsets,
-                       int *tile_pair, int max_tiles, bool chained, cudaStream_t s, Profiler *prof);
+// What a Gauss-Newton loop starts from: npairs descriptors, projection
+// matrices of the current clouds (12 floats each), poses and reference offsets
+// (16 doubles each) in pinned host memory, and where they go.  krt / dev_krt,
+// tile_pair and zbuf may be null.
+struct BeginArgs {
+  const PairDev *pairs;
+  const float *krt;
+  const double *guess, *roff;
+  int npairs;
+  PairDev *dev_pairs;
+  float *dev_krt;
+  int *tile_pair;  // tile -> pair table of the fused kernel (total pixel tiles entries)
+  uint4 *zbuf;     // the pairs' z-buffers, zbuf16 16-byte words
+  size_t zbuf16;
+};
+void launch_begin_loop(const BeginArgs &a, cudaStream_t s, Profiler *prof);
+// The pairs' states to pinned host memory.
+void launch_publish(const PairState *states, PairState *host, int npairs, bool chained, cudaStream_t s,
+                    Profiler *prof);
 void launch_solve(const PairDev *d_pairs, int npairs, float lambda, int mode, double early_eps, int ignore_done,
                   bool chained, cudaStream_t s, Profiler *prof);
 
