@@ -8,12 +8,14 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <string>
 #include <vector>
 
 #include "abi_guard.hpp"
 #include "common.cuh"
+#include "host_copy.hpp"
 #include "host_math.hpp"
 #include "kernels.hpp"
 #include "nicp_gpu.h"
@@ -62,6 +64,7 @@ struct nicp_ctx {
   cudaEvent_t copy_start = nullptr;     // the compute stream's tail when staging begins
   char *pin_down = nullptr;
   size_t pin_down_cap = 0;
+  HostCopier copier;                    // copies into pageable host memory
   size_t cloud_bytes = 0;
   std::vector<GraphEntry> graphs;
   nicp_cloud *scratch_cloud = nullptr;
@@ -208,6 +211,34 @@ static int pin_down(nicp_ctx *ctx, size_t bytes, char **out) {
   return NICP_OK;
 }
 
+// Device -> host copies of a call, complete on return; a few words (counts)
+// take the small pinned buffer.
+constexpr size_t kSmallCopy = 4096;
+static int copy_down(nicp_ctx *ctx, std::initializer_list<HostCopier::Part> parts) {
+  size_t total = 0;
+  for (const HostCopier::Part &p : parts) total += p.dst ? p.bytes : 0;
+  if (total > kSmallCopy) {
+    CK(ctx, ctx->copier.down(parts.begin(), (int)parts.size(), ctx->stream));
+    return NICP_OK;
+  }
+  char *pin;
+  int rc = pin_down(ctx, total, &pin);
+  if (rc) return rc;
+  size_t at = 0;
+  for (const HostCopier::Part &p : parts)
+    if (p.dst && p.bytes) {
+      CK(ctx, cudaMemcpyAsync(pin + at, p.src, p.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+      at += p.bytes;
+    }
+  CK(ctx, cudaStreamSynchronize(ctx->stream));
+  at = 0;
+  for (const HostCopier::Part &p : parts)
+    if (p.dst && p.bytes) {
+      std::memcpy(p.dst, pin + at, p.bytes);
+      at += p.bytes;
+    }
+  return NICP_OK;
+}
 static int cloud_reserve(nicp_cloud *c, int capacity, int rows, int cols, bool eig, bool gauss = false) {
   nicp_ctx *ctx = c->ctx;
   size_t P = (size_t)rows * cols;
@@ -533,9 +564,7 @@ extern "C" int nicp_cloud_size(nicp_cloud *c, int *n) {
   if (!c || !n) return NICP_EINVAL;
   if (!c->mem) { *n = 0; return NICP_OK; }
   nicp_ctx *ctx = c->ctx;
-  CK(ctx, cudaMemcpyAsync(n, c->count, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
-  return NICP_OK;
+  return copy_down(ctx, {{n, c->count, sizeof(int)}});
   NICP_ABI_CATCH
 }
 
@@ -545,9 +574,7 @@ extern "C" int nicp_cloud_normal_count(nicp_cloud *c, int *n) {
   if (!c || !n) return NICP_EINVAL;
   if (!c->mem) { *n = 0; return NICP_OK; }
   nicp_ctx *ctx = c->ctx;
-  CK(ctx, cudaMemcpyAsync(n, c->count + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
-  return NICP_OK;
+  return copy_down(ctx, {{n, c->count + 1, sizeof(int)}});
   NICP_ABI_CATCH
 }
 
@@ -562,35 +589,22 @@ extern "C" int nicp_cloud_download(nicp_cloud *c, float *p4, float *n4, float *c
   if (rc) return rc;
   if (n == 0) return NICP_OK;
   if ((ev3 || U9) && !c->eig_valid) return fail(ctx, NICP_ESTATE, "cloud was built without keep_stats");
-  if ((rc = cloud_ensure_omg(ctx, c))) return rc;
-  std::vector<float4> nrm(n), omg(3 * (size_t)n);
-  std::vector<float> eig;
-  if (p4) CK(ctx, cudaMemcpyAsync(p4, c->pts, 16 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(ctx, cudaMemcpyAsync(nrm.data(), c->nrm, 16 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(ctx, cudaMemcpyAsync(omg.data(), c->omg, 48 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
-  if (ev3 || U9) {
-    eig.resize(kStatsWords * (size_t)n);
-    CK(ctx, cudaMemcpyAsync(eig.data(), c->eig, 4 * kStatsWords * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
-  }
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
-  for (int i = 0; i < n; i++) {
-    if (p4) p4[4 * i + 3] = 1.0f;  // the device keeps a "has a normal" flag in w
-    if (n4) { n4[4 * i] = nrm[i].x; n4[4 * i + 1] = nrm[i].y; n4[4 * i + 2] = nrm[i].z; n4[4 * i + 3] = 0.0f; }
-    if (curv) curv[i] = nrm[i].w;
-    const float *o = reinterpret_cast<const float *>(&omg[3 * (size_t)i]);
-    // (Op00 Op01 Op02 Op11)(Op12 Op22 On00 On01)(On02 On11 On12 On22)
-    if (op9) {
-      float *d = op9 + 9 * (size_t)i;
-      d[0] = o[0]; d[1] = o[1]; d[2] = o[2]; d[3] = o[1]; d[4] = o[3]; d[5] = o[4]; d[6] = o[2]; d[7] = o[4]; d[8] = o[5];
-    }
-    if (on9) {
-      float *d = on9 + 9 * (size_t)i;
-      d[0] = o[6]; d[1] = o[7]; d[2] = o[8]; d[3] = o[7]; d[4] = o[9]; d[5] = o[10]; d[6] = o[8]; d[7] = o[10]; d[8] = o[11];
-    }
-    if (ev3) for (int k = 0; k < 3; k++) ev3[3 * (size_t)i + k] = eig[kStatsWords * (size_t)i + k];
-    if (U9) for (int k = 0; k < 9; k++) U9[9 * (size_t)i + k] = eig[kStatsWords * (size_t)i + 3 + k];
-  }
-  return NICP_OK;
+  if ((op9 || on9) && (rc = cloud_ensure_omg(ctx, c))) return rc;
+  // the caller's layout is written on the device
+  const size_t N = (size_t)n;
+  Layout L;
+  CloudExport x{};
+  const size_t o_p = L.take(16 * N), o_n = L.take(16 * N), o_k = L.take(4 * N), o_op = L.take(36 * N),
+               o_on = L.take(36 * N), o_ev = L.take(12 * N), o_u = L.take(36 * N);
+  if ((rc = ensure_ws(ctx, L.off))) return rc;
+  auto place = [&](const void *wanted, size_t off) { return wanted ? (float *)(ctx->ws + off) : nullptr; };
+  x.pts = c->pts; x.nrm = c->nrm; x.omg = c->omg; x.eig = c->eig;
+  x.p4 = place(p4, o_p); x.n4 = place(n4, o_n); x.curv = place(curv, o_k);
+  x.op9 = place(op9, o_op); x.on9 = place(on9, o_on); x.ev3 = place(ev3, o_ev); x.u9 = place(U9, o_u);
+  launch_cloud_export(x, n, ctx->stream);
+  CK(ctx, cudaGetLastError());
+  return copy_down(ctx, {{p4, x.p4, 16 * N}, {n4, x.n4, 16 * N}, {curv, x.curv, 4 * N}, {op9, x.op9, 36 * N},
+                         {on9, x.on9, 36 * N}, {ev3, x.ev3, 12 * N}, {U9, x.u9, 36 * N}});
   NICP_ABI_CATCH
 }
 
@@ -1071,10 +1085,7 @@ static int build_one(nicp_ctx *ctx, const void *depth, bool u16, int rows, int c
   int rc = build_frames(ctx, 1, &f, cam, prm, &out, false);
   if (rc) return rc;
   if (offset && (rc = nicp_cloud_transform(out, offset))) return rc;
-  if (index_out) {
-    CK(ctx, cudaMemcpyAsync(index_out, out->index, 4 * (size_t)rows * cols, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(ctx, cudaStreamSynchronize(ctx->stream));
-  }
+  if (index_out) return copy_down(ctx, {{index_out, out->index, 4 * (size_t)rows * cols}});
   return NICP_OK;
 }
 
@@ -1136,12 +1147,7 @@ extern "C" int nicp_unproject(nicp_ctx *ctx, const float *depth, int rows, int c
   nicp_cloud *c = ctx->scratch_cloud;
   if ((rc = build_frames(ctx, 1, &f, cam, &prm, &c, true))) return rc;
   if ((rc = nicp_cloud_size(c, n))) return rc;
-  if (points4_out && *n) {
-    CK(ctx, cudaMemcpyAsync(points4_out, c->pts, 16 * (size_t)*n, cudaMemcpyDeviceToHost, ctx->stream));
-  }
-  if (index_out) CK(ctx, cudaMemcpyAsync(index_out, c->index, 4 * (size_t)rows * cols, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
-  return NICP_OK;
+  return copy_down(ctx, {{points4_out, c->pts, 16 * (size_t)*n}, {index_out, c->index, 4 * (size_t)rows * cols}});
   NICP_ABI_CATCH
 }
 
@@ -1164,9 +1170,7 @@ extern "C" int nicp_project_intervals(nicp_ctx *ctx, const float *depth, int row
   launch_intervals((const float *)(ctx->ws + o_d), (int)P, (const float *)(ctx->ws + o_k), cam->min_distance,
                    cam->max_distance, world_radius, (int32_t *)(ctx->ws + o_o), ctx->stream, &ctx->prof);
   CK(ctx, cudaGetLastError());
-  CK(ctx, cudaMemcpyAsync(radius_out, ctx->ws + o_o, 4 * P, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
-  return NICP_OK;
+  return copy_down(ctx, {{radius_out, ctx->ws + o_o, 4 * P}});
   NICP_ABI_CATCH
 }
 
@@ -1304,12 +1308,8 @@ extern "C" int nicp_correspond(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_
   launch_corr_list((const PairDev *)(ctx->ws + pl.o_pairs), 1, pl.total_tiles, corr_params(*prm), 0,
                    (const float *)(ctx->ws + pl.o_krt), s, &ctx->prof);
   CK(ctx, cudaGetLastError());
-  CK(ctx, cudaMemcpyAsync(num_out, ctx->ws + pl.o_np[0], 4, cudaMemcpyDeviceToHost, s));
-  CK(ctx, cudaStreamSynchronize(s));
-  if (pairs_out && *num_out > 0) {
-    CK(ctx, cudaMemcpyAsync(pairs_out, ctx->ws + pl.o_list[0], 8 * (size_t)*num_out, cudaMemcpyDeviceToHost, s));
-    CK(ctx, cudaStreamSynchronize(s));
-  }
+  if ((rc = copy_down(ctx, {{num_out, ctx->ws + pl.o_np[0], 4}}))) return rc;
+  if (pairs_out && *num_out > 0) return copy_down(ctx, {{pairs_out, ctx->ws + pl.o_list[0], 8 * (size_t)*num_out}});
   return NICP_OK;
   NICP_ABI_CATCH
 }
@@ -1425,10 +1425,7 @@ extern "C" int nicp_project(nicp_ctx *ctx, const nicp_cloud *cloud, const nicp_c
   launch_zbuffer(dpd, 1, pl.max_pt_tiles, 0, (const float *)(ctx->ws + pl.o_krt), kZbufDefaultPPT, false, s, &ctx->prof);
   launch_resolve(dpd, 1, pl.max_tiles, 0, (float *)(ctx->ws + o_depth), 0, false, s, &ctx->prof);
   CK(ctx, cudaGetLastError());
-  if (index_out) CK(ctx, cudaMemcpyAsync(index_out, ctx->ws + pl.o_cur[0], 4 * P, cudaMemcpyDeviceToHost, s));
-  if (depth_out) CK(ctx, cudaMemcpyAsync(depth_out, ctx->ws + o_depth, 4 * P, cudaMemcpyDeviceToHost, s));
-  CK(ctx, cudaStreamSynchronize(s));
-  return NICP_OK;
+  return copy_down(ctx, {{index_out, ctx->ws + pl.o_cur[0], 4 * P}, {depth_out, ctx->ws + o_depth, 4 * P}});
   NICP_ABI_CATCH
 }
 
@@ -1640,10 +1637,8 @@ extern "C" int nicp_correspond_nn(nicp_ctx *ctx, const nicp_cloud *ref, const ni
   if (launch_nn_correspond(q, (int32_t *)(ctx->ws + pl.o_pairs), (int *)(ctx->ws + pl.o_np), false, s))
     return fail(ctx, NICP_ECUDA, "nearest-neighbour query failed");
   int K = 0;
-  CK(ctx, cudaMemcpyAsync(&K, ctx->ws + pl.o_np, 4, cudaMemcpyDeviceToHost, s));
-  CK(ctx, cudaStreamSynchronize(s));
-  if (pairs_out && K > 0)
-    CK(ctx, cudaMemcpy(pairs_out, ctx->ws + pl.o_pairs, 8 * (size_t)K, cudaMemcpyDeviceToHost));
+  if ((rc = copy_down(ctx, {{&K, ctx->ws + pl.o_np, 4}}))) return rc;
+  if (pairs_out && K > 0 && (rc = copy_down(ctx, {{pairs_out, ctx->ws + pl.o_pairs, 8 * (size_t)K}}))) return rc;
   *num_pairs = K;
   return NICP_OK;
   NICP_ABI_CATCH

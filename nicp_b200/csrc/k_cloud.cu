@@ -879,6 +879,59 @@ __global__ void k_cloud_transform(float4 *pts, float4 *nrm, float4 *omg, float *
   }
 }
 
+// A cloud in the caller's layout: points with w = 1 (the device keeps its
+// flags there), normals with w = 0, full 3x3 matrices.  256 points per CTA;
+// the nine-word matrices go through shared memory, so that stores are whole
+// lines (it is a pass over 100 bytes a point in and out: the copy engine after
+// it takes ten times as long).
+__global__ void __launch_bounds__(256) k_cloud_export(CloudExport x, int n) {
+  __shared__ float m9[256 * 9];
+  const int t = threadIdx.x, i0 = blockIdx.x * 256, i = i0 + t, here = min(256, n - i0);
+  auto store9 = [&](float *out, const float (&v)[9]) {
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 9; k++) m9[9 * t + k] = v[k];
+    __syncthreads();
+    for (int k = t; k < 9 * here; k += 256) out[9 * (size_t)i0 + k] = m9[k];
+  };
+  const bool in = i < n;
+  if (in) {
+    if (x.p4) {
+      const float4 p = x.pts[i];
+      reinterpret_cast<float4 *>(x.p4)[i] = make_float4(p.x, p.y, p.z, 1.0f);
+    }
+    if (x.n4 || x.curv) {
+      const float4 v = x.nrm[i];
+      if (x.n4) reinterpret_cast<float4 *>(x.n4)[i] = make_float4(v.x, v.y, v.z, 0.0f);
+      if (x.curv) x.curv[i] = v.w;
+    }
+    if (x.ev3)
+#pragma unroll
+      for (int k = 0; k < 3; k++) x.ev3[3 * (size_t)i + k] = x.eig[kStatsWords * (size_t)i + k];
+  }
+  if (x.op9 || x.on9) {
+    float4 a = make_float4(0, 0, 0, 0), b = a, c = a;
+    if (in) {
+      a = x.omg[3 * (size_t)i];
+      b = x.omg[3 * (size_t)i + 1];
+      c = x.omg[3 * (size_t)i + 2];
+    }
+    // (Op00 Op01 Op02 Op11) (Op12 Op22 On00 On01) (On02 On11 On12 On22)
+    if (x.op9) store9(x.op9, {a.x, a.y, a.z, a.y, a.w, b.x, a.z, b.x, b.y});
+    if (x.on9) store9(x.on9, {b.z, b.w, c.x, b.w, c.y, c.z, c.x, c.z, c.w});
+  }
+  if (x.u9) {
+    float u[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) u[k] = in ? x.eig[kStatsWords * (size_t)i + 3 + k] : 0.0f;
+    store9(x.u9, u);
+  }
+}
+
+void launch_cloud_export(const CloudExport &x, int n, cudaStream_t s) {
+  if (n > 0) k_cloud_export<<<(n + 255) / 256, 256, 0, s>>>(x, n);
+}
+
 // PinholePointProjector::projectIntervals (pinholepointprojector.cpp:136-148).
 __global__ void k_intervals(const float *__restrict__ depth, int P, const float *__restrict__ K9, float min_d, float max_d,
                             float R, int32_t *out) {

@@ -128,6 +128,13 @@ void launch_materialize_omg(const float4 *pts, const float4 *nrm, float4 *omg, c
 // omg may be null: an implicit Omega follows the rotated normal by itself.
 void launch_cloud_transform(float4 *pts, float4 *nrm, float4 *omg, float *eig, float4 *gauss, const int *count,
                             int capacity, const float *d_m12, cudaStream_t s, Profiler *prof);
+// A cloud in the layout of nicp_cloud_download; null outputs are not written.
+struct CloudExport {
+  const float4 *pts, *nrm, *omg;
+  const float *eig;
+  float *p4, *n4, *curv, *op9, *on9, *ev3, *u9;
+};
+void launch_cloud_export(const CloudExport &x, int n, cudaStream_t s);
 size_t moment_bytes(int precision);
 void launch_intervals(const float *d_depth, int P, const float *d_K9, float min_d, float max_d, float R, int32_t *d_out,
                       cudaStream_t s, Profiler *prof);
