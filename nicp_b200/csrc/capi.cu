@@ -1048,7 +1048,7 @@ static int build_frames(nicp_ctx *ctx, int n, const FrameIn *fin, const nicp_cam
       const bool lean = !prm->keep_stats && prm->pim_flat[1] == prm->pim_flat[2] &&
                         prm->pim_nonflat[1] == prm->pim_nonflat[2] && prm->nim_flat[1] == prm->nim_flat[2] &&
                         prm->nim_nonflat[1] == prm->nim_nonflat[2];
-      int shape = 0;
+      int shape = stats_default_shape(lean);
       if (ctx->autotune) {
         // the chunk's frame sizes and the moment precision select the shape
         std::map<std::pair<int, int>, int> hist;

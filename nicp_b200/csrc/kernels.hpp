@@ -114,6 +114,7 @@ void launch_moments(int precision, const FrameDev *d_frames, int nframes, int to
 constexpr int kStatsShapes = 4;  // k_stats launch shapes the autotuner chooses from (0: default)
 int stats_shape_threads(int shape);
 int stats_shape_min_ctas(int shape);
+int stats_default_shape(bool lean);
 // lean: no Stats kept and information matrices U diag(d0, d1, d1) U^T (only
 // the smallest eigenpair is computed).
 void launch_stats(int precision, const FrameDev *d_frames, int nframes, int max_pixels, int shape, bool lean,
