@@ -215,16 +215,17 @@ __device__ __forceinline__ float3 xform_point_g(const float *A, float4 p) {
 // transform (the aligner passes _T.inverse()).
 // The transformed reference point and normal are returned in rp / rn (rn
 // only when the normal gates run, i.e. not demoted).
+template <bool kPlain = false>
 __device__ __forceinline__ bool gate_t(const CorrParams &cp, const float *T12, float4 rp0, float4 rn0, float4 cpt,
                                        float4 cn, float3 &rp, float3 &rn) {
-  if (!cp.demoted) {
+  if (kPlain || !cp.demoted) {
     if (normal_is_zero(cn.x, cn.y, cn.z)) return false;
     if (normal_is_zero(rn0.x, rn0.y, rn0.z)) return false;
   }
   rp = xform_point_g2(T12, rp0);
   float dx = fsb(cpt.x, rp.x), dy = fsb(cpt.y, rp.y), dz = fsb(cpt.z, rp.z);
   if (dot3g(dx, dy, dz, dx, dy, dz) > cp.sq_thr) return false;
-  if (!cp.demoted) {
+  if (kPlain || !cp.demoted) {
     rn = xform_normal_g2(T12, rn0);
     if (dot3g(cn.x, cn.y, cn.z, rn.x, rn.y, rn.z) < cp.cos_thr) return false;
     float kr = rn0.w, kc = cn.w;
@@ -344,23 +345,42 @@ struct PixelTerms {
   float en0, en1, en2, le;   // Omega_n times the normal residual, chi2
 };
 
-// False when the pixel adds nothing (an outlier without the robust kernel).
-__device__ __forceinline__ bool pixel_terms(const LinParams &lp, const float *omd, float3 rp, float3 rn, float4 cpt,
-                                            float4 cn, PixelTerms &o) {
-  float alp = 0.0f, bep = 0.0f, aln = 0.0f, ben = 0.0f;
-  if (point_has_normal(cpt.w)) {
-    const int cls = (int)cpt.w - 1;
-    const float *dp = omd + 2 * (cls & 1), *dn = omd + 4 + 2 * ((cls >> 1) & 1);
-    alp = dp[1];
-    bep = dp[0] - dp[1];
-    aln = lp.scale * dn[1];
-    ben = lp.scale * dn[0] - aln;
-  }
-  if (lp.z_scaling) {
+// (alpha, beta) of Omega_p and Omega_n for a class code, scaled as the
+// linearizer scales them.
+__device__ __forceinline__ float4 class_weights(const LinParams &lp, const float *omd, int cls) {
+  const float *dp = omd + 2 * (cls & 1), *dn = omd + 4 + 2 * ((cls >> 1) & 1);
+  float4 w;
+  w.x = dp[1];
+  w.y = dp[0] - dp[1];
+  w.z = lp.scale * dn[1];
+  w.w = lp.scale * dn[0] - w.z;
+  return w;
+}
+// Weights by the code in a point's w (kNoNormalW, 1, 2, 3, 4): entry
+// weight_entry(w) of a table of kWeightEntries, so that the lookup is a shift
+// and one 128-bit read instead of a conversion, four reads and their sums.
+constexpr int kWeightEntries = 7;
+__device__ __forceinline__ int weight_entry(float w) {
+  return (int)min((__float_as_uint(w) >> 22) - 0xFCu, (unsigned)kWeightEntries - 1u);
+}
+// Entry e of that table: the codes' floats lie at 0 (0.5), 2 (1.0), 4 (2.0), 5 (3.0) and 6 (4.0).
+__device__ __forceinline__ float4 table_weights(const LinParams &lp, const float *omd, int e) {
+  const int cls = e == 2 ? 0 : e - 3;
+  return e < 2 || e == 3 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : class_weights(lp, omd, cls);
+}
+
+// w: the point's weights (class_weights; zero without a normal).  kPlain: the
+// defaults (robust kernel, no z scaling, not demoted).  False when the pixel
+// adds nothing (an outlier without the robust kernel).
+template <bool kPlain>
+__device__ __forceinline__ bool pixel_terms(const LinParams &lp, float4 w, float3 rp, float3 rn, float4 cpt, float4 cn,
+                                            PixelTerms &o) {
+  float alp = w.x, bep = w.y, aln = w.z, ben = w.w;
+  if (!kPlain && lp.z_scaling) {
     float f = 1.0f / fabsf(cpt.z);
     alp *= f; bep *= f; aln *= f; ben *= f;
   }
-  if (lp.demoted) { aln = 0.0f; ben = 0.0f; }
+  if (!kPlain && lp.demoted) { aln = 0.0f; ben = 0.0f; }
   const float ux = cn.x, uy = cn.y, uz = cn.z;
   float pe0 = rp.x - cpt.x, pe1 = rp.y - cpt.y, pe2 = rp.z - cpt.z;
   float ne0 = rn.x - cn.x, ne1 = rn.y - cn.y, ne2 = rn.z - cn.z;
@@ -370,7 +390,7 @@ __device__ __forceinline__ bool pixel_terms(const LinParams &lp, const float *om
   float en0 = fmaf(bv, ux, aln * ne0), en1 = fmaf(bv, uy, aln * ne1), en2 = fmaf(bv, uz, aln * ne2);
   float le = fmaf(ne2, en2, fmaf(ne1, en1, fmaf(ne0, en0, fmaf(pe2, ep2, fmaf(pe1, ep1, pe0 * ep0)))));
   if (le > lp.max_chi2) {
-    if (!lp.robust) return false;
+    if (!kPlain && !lp.robust) return false;
     const float ks = lp.max_chi2 / le;
     le *= ks;
     alp *= ks; bep *= ks; aln *= ks; ben *= ks;
@@ -434,18 +454,14 @@ __device__ __forceinline__ void add_rotation_terms(const PixelTerms &p, float *v
   v[20] = fmaf(nw2, wn2, fmaf(pw2, wp2, fmaf(qbn, bn, fmaf(qan, an, fmaf(qb, b, fmaf(qa, a, v[20]))))));
 }
 
-__device__ __forceinline__ void lin_terms_structured_xf(const LinParams &lp, const float *omd, float3 rp, float3 rn,
-                                                       float4 cpt, float4 cn, Acc &acc) {
+template <bool kPlain>
+__device__ __forceinline__ void lin_terms_structured_xf(const LinParams &lp, float4 w, float3 rp, float3 rn, float4 cpt,
+                                                       float4 cn, Acc &acc) {
   PixelTerms p;
-  if (!pixel_terms(lp, omd, rp, rn, cpt, cn, p)) return;
+  if (!pixel_terms<kPlain>(lp, w, rp, rn, cpt, cn, p)) return;
   acc.cnt += Acc::kInlier;
   add_pose_terms(p, acc.v);
   add_rotation_terms(p, acc.v);
-}
-
-__device__ __forceinline__ void lin_terms_structured(const LinParams &lp, const float *T12, const float *omd,
-                                                    float4 rp0, float4 rn0, float4 cpt, float4 cn, Acc &acc) {
-  lin_terms_structured_xf(lp, omd, xform_point_g(T12, rp0), xform_normal_g(T12, rn0), cpt, cn, acc);
 }
 
 // Reduces every thread's Acc to one FP64 partial of the CTA (fixed order).
@@ -518,11 +534,10 @@ constexpr int kConstSlots = 4;
 // words (no bank conflicts).
 struct GatherStageS {  // structured Omega: rebuilt from the current normal
   float4 rp[kSubPix], rn[kSubPix], cp[kSubPix], cn[kSubPix];
-  int valid[kSubPix];
 };
 struct GatherStageG : GatherStageS {  // general Omega: gathered for accepted pixels
   float4 o0[kSubPix], o1[kSubPix], o2[kSubPix];
-  int ci[kSubPix];
+  int valid[kSubPix], ci[kSubPix];
 };
 #ifndef NICP_CORR_S_CTAS
 #define NICP_CORR_S_CTAS 5
@@ -597,8 +612,11 @@ __device__ __forceinline__ void cp_async_wait() {
 // bit1 reset the z-buffer after reading, bit2 keep the resolved reference
 // index image, bit3 statistics pass (gate with Tgate_used; ignores `done`).
 // kStructured: every pair's current cloud has structured information
-// matrices (no Omega gathers, smaller stages).
-template <bool kStructured>
+// matrices (no Omega gathers, smaller stages).  kPlain (structured): the
+// options' defaults, decided on the host; kFirst: bits 0 and 1 of flags.  The
+// pass is bound by the instructions it issues, a good part of which asked for
+// options pixel by pixel.
+template <bool kStructured, bool kPlain, bool kFirst>
 __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS : 3)
     k_corr_lin(const PairDev *__restrict__ pairs, int npairs, const int *__restrict__ tile_pair, int total_tiles,
                CorrParams cp, LinParams lp, int flags) {
@@ -610,12 +628,14 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
   // [0..11] gating T, [12..23] linearizer T, [24..31] the current cloud's
   // Omega parameters, then pair index, skip flag and structured-Omega flag
   __shared__ float sT[kConstSlots][32];
+  __shared__ float4 sW[kConstSlots][kWeightEntries];  // structured: weights by point code
   __shared__ int sPair[kConstSlots], sSkip[kConstSlots], sStruct[kConstSlots], sSame[kConstSlots];
   const bool stats_pass = flags & 8;
   if ((int)blockIdx.x >= total_tiles) return;
   const int ntiles = (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int nsub = ntiles * kSubsPerTile;
-  const bool drop_no_normal = !cp.demoted;
+  const bool drop_no_normal = kPlain || !cp.demoted;
+  const bool first = kPlain ? kFirst : (flags & 1) != 0, reset = kPlain ? kFirst : (flags & 2) != 0;
   auto tile_of = [&](int j) { return (int)blockIdx.x + (j / kSubsPerTile) * (int)gridDim.x; };
   auto stage_of = [&](int j) -> Stage & { return stages[j % corr_stages<kStructured>()]; };
 
@@ -652,9 +672,9 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
     for (int k = 0; k < kFusedPX; k++) {
       const int p = p0 + k * kFusedThreads;
       if (p < P) {
-        if (flags & 1) zI[k] = pd.zbuf[p];
+        if (first) zI[k] = pd.zbuf[p];
         else cI[k] = pd.ref_index[p];  // stashed in cI until phase G1 reads the current index
-        if (flags & 1) cI[k] = pd.cur_index[p];
+        if (first) cI[k] = pd.cur_index[p];
         else zI[k] = (unsigned long long)(unsigned)pd.cur_index[p];
       }
     }
@@ -662,6 +682,7 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
 
   // Phase G1 (two sub-tiles ahead): decode the indices, reset the z-buffer,
   // gather points and normals of both clouds.
+  // Returns the valid pixels (bit k) of a structured pass.
   auto issue_g1 = [&](int j) {
     Stage &g = stage_of(j);
     int ci[kFusedPX], valid[kFusedPX];
@@ -687,7 +708,7 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
           const int p = p0 + k * kFusedThreads, sl = t + k * kFusedThreads;
           if (p < P) {
             int ri;
-            if (flags & 1) {
+            if (first) {
               // an empty word (all ones) decodes to -1 with drop_no_normal
               // and to 2^31 - 1 without, which the bounds test below rejects
               const unsigned lo = (unsigned)zI[k];
@@ -696,14 +717,14 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
               // evict-first: the word is read again only by the next
               // projection, long after it would have left L2, where it
               // would displace the gathered clouds
-              if (flags & 2) __stcs(pd.zbuf + p, ~0ull);
+              if (reset) __stcs(pd.zbuf + p, ~0ull);
               if (flags & 4) pd.ref_index[p] = ri;
             } else {
               ri = cI[k];
               ci[k] = (int)(unsigned)zI[k];
             }
             valid[k] = (unsigned)ri < (unsigned)gt_rc && (unsigned)ci[k] < (unsigned)gt_cc;
-            if (valid[k] && cp.row_limit_threads > 1)
+            if (!kPlain && valid[k] && cp.row_limit_threads > 1)
               valid[k] = p / pd.cols < (pd.rows / cp.row_limit_threads) * cp.row_limit_threads;
             if (valid[k]) {
               cp_async16(&g.rp[sl], pd.ref_pts + ri);
@@ -715,12 +736,18 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
         }
       }
     }
+    unsigned bits = 0;
 #pragma unroll
     for (int k = 0; k < kFusedPX; k++) {
-      if constexpr (!kStructured) g.ci[t + k * kFusedThreads] = ci[k];
-      g.valid[t + k * kFusedThreads] = valid[k];
+      if constexpr (!kStructured) {
+        g.ci[t + k * kFusedThreads] = ci[k];
+        g.valid[t + k * kFusedThreads] = valid[k];
+      } else {
+        bits |= (valid[k] ? 1u : 0u) << k;
+      }
     }
     cp_async_commit();
+    return bits;
   };
 
   // Per-tile constants, written when the tile's first sub-tile enters G1.
@@ -735,6 +762,8 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
                                             : st->Tlin[threadIdx.x - 12];
     else if (threadIdx.x < 32)
       sT[e][threadIdx.x] = pairs[pi].cur_omd[threadIdx.x - 24];
+    else if (threadIdx.x < 32 + kWeightEntries)
+      sW[e][threadIdx.x - 32] = table_weights(lp, pairs[pi].cur_omd, threadIdx.x - 32);
     if (threadIdx.x == 0) {
       sPair[e] = pi;
       sSkip[e] = st->done && !stats_pass;
@@ -783,7 +812,7 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
   acc.zero();
   // Linearizes sub-tile j (its gather -- and, for general Omega, its gate --
   // complete); at a tile's last sub-tile the CTA stores the tile's partial.
-  auto consume = [&](int j) {
+  auto consume = [&](int j, unsigned bits) {
     const int e = (j / kSubsPerTile) % kConstSlots;
     const int sub = j % kSubsPerTile;
     if (sub == 0) {
@@ -794,26 +823,28 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
 #pragma unroll
       for (int k = 0; k < kFusedPX; k++) {
         const int sl = t + k * kFusedThreads;
-        const int v = g.valid[sl];
         if constexpr (kStructured) {
-          if (v) {
+          if ((bits >> k) & 1u) {
             acc.cnt += Acc::kCandidate;
             const float4 rp0 = g.rp[sl], rn0 = g.rn[sl], cpt = g.cp[sl], cn = g.cn[sl];
             float3 rp, rn;
-            if (gate_t(cp, sT[e], rp0, rn0, cpt, cn, rp, rn)) {
+            if (gate_t<kPlain>(cp, sT[e], rp0, rn0, cpt, cn, rp, rn)) {
               acc.cnt += Acc::kAccepted;
-              if (sSame[e] && !cp.demoted)
-                lin_terms_structured_xf(lp, sT[e] + 24, rp, rn, cpt, cn, acc);
-              else
-                lin_terms_structured(lp, sT[e] + 12, sT[e] + 24, rp0, rn0, cpt, cn, acc);
+              if (!sSame[e] || (!kPlain && cp.demoted)) {
+                rp = xform_point_g(sT[e] + 12, rp0);
+                rn = xform_normal_g(sT[e] + 12, rn0);
+              }
+              lin_terms_structured_xf<kPlain>(lp, sW[e][weight_entry(cpt.w)], rp, rn, cpt, cn, acc);
             }
           }
         } else {
+          const int v = g.valid[sl];
           if (v) acc.cnt += Acc::kCandidate;
           if (v == 2) {
             acc.cnt += Acc::kAccepted;
             if (sStruct[e])
-              lin_terms_structured(lp, sT[e] + 12, sT[e] + 24, g.rp[sl], g.rn[sl], g.cp[sl], g.cn[sl], acc);
+              lin_terms_structured_xf<false>(lp, sW[e][weight_entry(g.cp[sl].w)], xform_point_g(sT[e] + 12, g.rp[sl]),
+                                             xform_normal_g(sT[e] + 12, g.rn[sl]), g.cp[sl], g.cn[sl], acc);
             else
               lin_terms(lp, sT[e] + 12, g.rp[sl], g.rn[sl], g.cp[sl], g.cn[sl], g.o0[sl], g.o1[sl], g.o2[sl],
                         acc);
@@ -831,16 +862,17 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
     // two stages: sub-tile j+1 is gathered while j is gated and linearized
     load_indices(0);
     tile_constants(0);
-    issue_g1(0);
+    unsigned bits = issue_g1(0);
     load_indices(1);
     __syncthreads();          // tile 0's constants visible
     for (int j = 0; j < nsub; j++) {
       tile_constants(j + 1);
-      issue_g1(j + 1);        // uses the indices loaded in the previous iteration
+      const unsigned next = issue_g1(j + 1);  // uses the indices loaded in the previous iteration
       load_indices(j + 2);
       if ((j + 1) % kSubsPerTile == 0) __syncthreads();  // the next tile's constants visible
       cp_async_wait<1>();     // G1(j) complete (G1(j+1) may be in flight)
-      consume(j);
+      consume(j, bits);
+      bits = next;
     }
   } else {
     // prologue: sub-tile 0 through G1 and the gate, sub-tile 1 through G1
@@ -862,7 +894,7 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
       cp_async_wait<2>();       // G1(j+1) complete (groups after it: G2(j), G1(j+2))
       gate_g2(j + 1);
       cp_async_wait<2>();       // G2(j) complete (groups after it: G1(j+2), G2(j+1))
-      consume(j);
+      consume(j, 0u);
     }
   }
   cp_async_wait<0>();
@@ -894,7 +926,8 @@ __global__ void __launch_bounds__(kTileThreads, kTileCtas)
     k_corr_tile(const PairDev *__restrict__ pairs, CorrParams cp, LinParams lp, int flags) {
   extern __shared__ __align__(16) unsigned char tile_smem_raw[];
   TileSmem &sm = *reinterpret_cast<TileSmem *>(tile_smem_raw);
-  __shared__ float sT[32];
+  __shared__ float sT[24];
+  __shared__ float4 sW[kWeightEntries];
   __shared__ unsigned counts[kTileThreads / 32];
   __shared__ double wsum[4][32];
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
@@ -915,7 +948,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileCtas)
     const int p = p0 + k * kTileThreads;
     ci[k] = p < P ? pd.cur_index[p] : -1;  // written before the loop
   }
-  if (t >= 32 && t < 40) sT[24 + t - 32] = pd.cur_omd[t - 32];
+  if (t >= 32 && t < 32 + kWeightEntries) sW[t - 32] = table_weights(lp, pd.cur_omd, t - 32);
   chain();
   // one round trip: the pair's flag and transforms, the pixels' indices
   const int done = __ldcg(&st->done);
@@ -984,7 +1017,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileCtas)
             rn = xform_normal_g(sT + 12, rn0);
           }
           PixelTerms q;
-          if (pixel_terms(lp, sT + 24, rp, rn, cpt, cn, q)) {
+          if (pixel_terms<false>(lp, sW[weight_entry(cpt.w)], rp, rn, cpt, cn, q)) {
             cnt += Acc::kInlier;
             o = q;
           }
@@ -1647,7 +1680,7 @@ void launch_resolve(const PairDev *d_pairs, int npairs, int max_tiles, int to_re
 // The shared-memory opt-in holds for the device that was current when it was
 // set, and the occupancy is that device's: both are taken once per device
 // (std::call_once: host threads on other contexts wait rather than race).
-template <bool kStructured>
+template <bool kStructured, bool kPlain, bool kFirst>
 static int corr_lin_grid(int total_tiles, int ctas_per_sm) {
   struct Occupancy {
     int sm_count = 1, per_sm_max = 1;
@@ -1656,11 +1689,11 @@ static int corr_lin_grid(int total_tiles, int ctas_per_sm) {
   static Occupancy occ[kMaxDevices];
   static std::once_flag once[kMaxDevices];
   auto query = [](int dev, Occupancy *o) {
-    cudaFuncSetAttribute(k_corr_lin<kStructured>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_corr_lin<kStructured, kPlain, kFirst>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          corr_smem<kStructured>());
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_corr_lin<kStructured>, kFusedThreads,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_corr_lin<kStructured, kPlain, kFirst>, kFusedThreads,
                                                   corr_smem<kStructured>());
     o->per_sm_max = std::max(1, per_sm);
     o->sm_count = std::max(1, sms);
@@ -1678,6 +1711,14 @@ static int corr_lin_grid(int total_tiles, int ctas_per_sm) {
   const int resident = o->sm_count * o->per_sm_max;
   const int grid = (ctas_per_sm > 0 && ctas_per_sm < o->per_sm_max) ? o->sm_count * ctas_per_sm : resident;
   return std::min(total_tiles, grid);
+}
+
+template <bool kStructured, bool kPlain, bool kFirst>
+static void corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, const CorrParams &cp, const LinParams &lp,
+                     int flags, int ctas_per_sm, const int *tile_pair, cudaStream_t s) {
+  const int grid = corr_lin_grid<kStructured, kPlain, kFirst>(total_tiles, ctas_per_sm);
+  k_corr_lin<kStructured, kPlain, kFirst><<<grid, kFusedThreads, corr_smem<kStructured>(), s>>>(
+      d_pairs, npairs, tile_pair, total_tiles, cp, lp, flags);
 }
 
 // Three CTAs of k_corr_tile fit on an SM.  Up to there the pass takes less
@@ -1701,13 +1742,14 @@ void launch_corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, int ma
   if (structured && few_tiles(npairs, max_tiles)) {
     launch(true, k_corr_tile, dim3(max_tiles, npairs), kTileThreads, sizeof(TileSmem), s, d_pairs, cp, lp, flags);
   } else if (structured) {
-    int grid = corr_lin_grid<true>(total_tiles, ctas_per_sm);
-    k_corr_lin<true><<<grid, kFusedThreads, corr_smem<true>(), s>>>(d_pairs, npairs, tile_pair, total_tiles, cp,
-                                                                    lp, flags);
+    // (the reset goes with the first pass)
+    const bool plain = !cp.demoted && cp.row_limit_threads <= 1 && !lp.demoted && !lp.z_scaling && lp.robust &&
+                       ((flags & 3) == 0 || (flags & 3) == 3);
+    if (plain && (flags & 1)) corr_lin<true, true, true>(d_pairs, npairs, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
+    else if (plain) corr_lin<true, true, false>(d_pairs, npairs, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
+    else corr_lin<true, false, false>(d_pairs, npairs, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
   } else {
-    int grid = corr_lin_grid<false>(total_tiles, ctas_per_sm);
-    k_corr_lin<false><<<grid, kFusedThreads, corr_smem<false>(), s>>>(d_pairs, npairs, tile_pair, total_tiles,
-                                                                      cp, lp, flags);
+    corr_lin<false, false, false>(d_pairs, npairs, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
   }
   prof->end(NICP_K_CORR_LIN, s);
 }
