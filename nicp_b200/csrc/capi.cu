@@ -46,6 +46,8 @@ struct Layout {
 
 }  // namespace
 
+constexpr int kMaxParts = 4;
+
 struct nicp_ctx {
   int device = 0;
   int sm_count = 148;
@@ -62,6 +64,8 @@ struct nicp_ctx {
   cudaStream_t copy_stream = nullptr;   // depth staging copies, overlapped with the build kernels
   std::vector<cudaEvent_t> copy_ev;     // one per build chunk: its frames are staged
   cudaEvent_t copy_start = nullptr;     // the compute stream's tail when staging begins
+  cudaStream_t fork_stream[kMaxParts - 1] = {};  // the other branches of a captured, forked loop
+  cudaEvent_t fork_ev[kMaxParts] = {};
   char *pin_down = nullptr;
   size_t pin_down_cap = 0;
   HostCopier copier;                    // copies into pageable host memory
@@ -432,6 +436,10 @@ extern "C" int nicp_ctx_destroy(nicp_ctx *ctx) {
   for (cudaEvent_t e : ctx->copy_ev) cudaEventDestroy(e);
   if (ctx->copy_start) cudaEventDestroy(ctx->copy_start);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
+  for (cudaStream_t f : ctx->fork_stream)
+    if (f) cudaStreamDestroy(f);
+  for (cudaEvent_t e : ctx->fork_ev)
+    if (e) cudaEventDestroy(e);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return NICP_OK;
@@ -1185,6 +1193,7 @@ struct PairPlan {
   int max_tiles = 0;                      // pixel tiles of the largest pair image
   size_t o_pairs = 0, o_states = 0, o_krt = 0, o_zbuf = 0, zbuf_bytes = 0;
   size_t o_tile_pair = 0;  // int per pixel tile: its pair
+  std::vector<int> part_pair, part_tile;  // a forked loop's parts: first pair, first tile, and the ends
   std::vector<size_t> o_cur, o_ref, o_part, o_list, o_ltc, o_np;
   std::vector<int> P, tiles;
 };
@@ -1958,8 +1967,35 @@ struct AlignCall {
 };
 }  // namespace
 
+// Parts of a forked loop.  A launch over all pairs ends with few CTAs at work,
+// and its solve runs on a few SMs; with the pairs in up to kMaxParts parts, each
+// on a branch of the captured graph, one part's launches fill what another's
+// leave free.  One / two / three / four parts, ms: 9 frames of 640x480 0.97 /
+// 0.91 / 0.92 / 0.92, 20 frames 2.06 / 1.92 / 1.92 / 1.91, 200 frames 17.8 / 17.2
+// / 17.2 / 17.2, 20 of 320x240 0.69 / 0.63 / 0.62 / 0.60, 24 mixed pairs 4.01 /
+// 3.87 / 3.77 / 3.78.  Below kPartTiles tiles a part's own launches are too
+// short (two pairs of 300 tiles: 0.487 whole, 0.494 in two).
+constexpr int kPartTiles = 320;
+static void plan_parts(PairPlan &pl) {
+  const int parts = std::min(std::min(kMaxParts, pl.n), pl.total_tiles / kPartTiles);
+  pl.part_pair.assign(1, 0);
+  pl.part_tile.assign(1, 0);
+  int tile = 0;
+  for (int i = 0; i < pl.n; i++) {
+    // a part ends where its share of the tiles is reached
+    const int g = (int)pl.part_pair.size();
+    if (g < parts && i > pl.part_pair.back() && (long long)tile * parts >= (long long)pl.total_tiles * g) {
+      pl.part_pair.push_back(i);
+      pl.part_tile.push_back(tile);
+    }
+    tile += pl.tiles[i];
+  }
+  pl.part_pair.push_back(pl.n);
+  pl.part_tile.push_back(tile);
+}
+
 // Enqueues the whole Gauss-Newton loop for the planned pairs.
-static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) {
+static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, bool fork) {
   cudaStream_t s = ctx->stream;
   const PairDev *dpd = (const PairDev *)(ctx->ws + pl.o_pairs);
   CorrParams cp = corr_params(*a.corr);
@@ -1986,7 +2022,28 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) 
   // outside list (parity) mode, current pixels whose point has no normal are
   // dropped from the index image: the gates would reject them anyway
   launch_resolve(dpd, pl.n, pl.max_tiles, 0, nullptr, (pl.list_mode || cp.demoted) ? 0 : 1, chained, s, &ctx->prof);
-  for (int i = 0; i < outer; i++) {
+  if (fork) {
+    // each part's iterations on a branch of its own
+    cudaEventRecord(ctx->fork_ev[0], s);
+    const int parts = (int)pl.part_pair.size() - 1;
+    for (int g = 0; g < parts; g++) {
+      cudaStream_t q = g ? ctx->fork_stream[g - 1] : s;
+      if (g) cudaStreamWaitEvent(q, ctx->fork_ev[0], 0);
+      const int p0 = pl.part_pair[g], n = pl.part_pair[g + 1] - p0, t0 = pl.part_tile[g], tn = pl.part_tile[g + 1] - t0;
+      for (int i = 0; i < outer; i++) {
+        launch_zbuffer(dpd + p0, n, pl.max_pt_tiles, 1, nullptr, L.zb_ppt, false, q, &ctx->prof);
+        for (int k = 0; k < inner; k++) {
+          const int flags = (k == 0) ? (1 | 2 | (pl.keep_ref ? 4 : 0)) : 0;
+          launch_corr_lin(dpd, pl.n, t0, tn, pl.max_tiles, cp, lp, flags, true, L.corr_ctas, tile_pair, q, &ctx->prof);
+          launch_solve(dpd + p0, n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, false, q,
+                       &ctx->prof);
+        }
+      }
+      if (g) cudaEventRecord(ctx->fork_ev[g], q);
+    }
+    for (int g = 1; g < parts; g++) cudaStreamWaitEvent(s, ctx->fork_ev[g], 0);
+  }
+  for (int i = 0; i < outer && !fork; i++) {
     launch_zbuffer(dpd, pl.n, pl.max_pt_tiles, 1, nullptr, L.zb_ppt, chained, s, &ctx->prof);
     if (pl.list_mode) {
       launch_resolve(dpd, pl.n, pl.max_tiles, 1, nullptr, 0, false, s, &ctx->prof);
@@ -1998,7 +2055,7 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) 
     } else {
       for (int k = 0; k < inner; k++) {
         int flags = (k == 0) ? (1 | 2 | (pl.keep_ref ? 4 : 0)) : 0;
-        launch_corr_lin(dpd, pl.n, pl.total_tiles, pl.max_tiles, cp, lp, flags, pl.structured, L.corr_ctas, tile_pair, s,
+        launch_corr_lin(dpd, pl.n, 0, pl.total_tiles, pl.max_tiles, cp, lp, flags, pl.structured, L.corr_ctas, tile_pair, s,
                         &ctx->prof);
         launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, chained, s, &ctx->prof);
       }
@@ -2010,7 +2067,7 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) 
     if (pl.list_mode)
       launch_lin_list(dpd, pl.n, pl.total_tiles, lp, std::max(1, a.corr->parity_threads), 2, nullptr, false, s, &ctx->prof);
     else
-      launch_corr_lin(dpd, pl.n, pl.total_tiles, pl.max_tiles, cp, lp, 8, pl.structured, L.corr_ctas, tile_pair, s, &ctx->prof);
+      launch_corr_lin(dpd, pl.n, 0, pl.total_tiles, pl.max_tiles, cp, lp, 8, pl.structured, L.corr_ctas, tile_pair, s, &ctx->prof);
     launch_solve(dpd, pl.n, 0.0f, 4 | xb, 0.0, 1, chained, s, &ctx->prof);
   }
   launch_publish((const PairState *)(ctx->ws + pl.o_states), a.results, pl.n, chained, s, &ctx->prof);
@@ -2030,6 +2087,8 @@ static std::string graph_key(nicp_ctx *ctx, const PairPlan &pl, const AlignCall 
   put(&pl.max_pt_tiles, sizeof(int));
   put(&pl.max_tiles, sizeof(int));
   put(&pl.zbuf_bytes, sizeof(size_t));
+  put(pl.part_pair.data(), sizeof(int) * pl.part_pair.size());
+  put(pl.part_tile.data(), sizeof(int) * pl.part_tile.size());
   put(a.corr, sizeof(*a.corr));
   put(a.lin, sizeof(*a.lin));
   put(a.prm, sizeof(*a.prm));
@@ -2077,7 +2136,7 @@ static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
   auto trial = [&](const nicp_ctx::Launch &c, float *ms) -> int {
     ctx->launch = c;
     CK(ctx, cudaEventRecord(e0, s));
-    enqueue_loop(ctx, pl, a);
+    enqueue_loop(ctx, pl, a, false);
     CK(ctx, cudaEventRecord(e1, s));
     CK(ctx, cudaEventSynchronize(e1));
     CK(ctx, cudaEventElapsedTime(ms, e0, e1));
@@ -2138,6 +2197,7 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
   if ((rc = plan_pairs(ctx, a.n, a.cams, big.data(), keep_ref, list_mode, pl))) return rc;
   pl.structured = !list_mode;
   for (int i = 0; i < a.n && pl.structured; i++) pl.structured = a.curs[i] && a.curs[i]->omega_structured;
+  plan_parts(pl);
   // the list linearizer reads the current clouds' matrices (the fused kernel
   // rebuilds a structured cloud's Omega itself)
   for (int i = 0; i < a.n && list_mode; i++)
@@ -2201,9 +2261,15 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
       size_t rec0 = ctx->prof.recs.size();
       unsigned long long l0 = ctx->prof.launches;
       cudaGraph_t graph;
+      const bool fork = pl.structured && pl.part_pair.size() > 2;
+      for (int k = 0; fork && k < kMaxParts; k++) {
+        if (!ctx->fork_ev[k]) CK(ctx, cudaEventCreateWithFlags(&ctx->fork_ev[k], cudaEventDisableTiming));
+        if (k && !ctx->fork_stream[k - 1])
+          CK(ctx, cudaStreamCreateWithFlags(&ctx->fork_stream[k - 1], cudaStreamNonBlocking));
+      }
       CK(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
       ctx->prof.capturing = true;
-      enqueue_loop(ctx, pl, a);
+      enqueue_loop(ctx, pl, a, fork);
       ctx->prof.capturing = false;
       cudaError_t e = cudaStreamEndCapture(s, &graph);
       if (e != cudaSuccess) return fail(ctx, NICP_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -2225,7 +2291,7 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
     ctx->prof.launches += ge->kernels;
     if (ctx->prof.enabled) ctx->prof.recs.insert(ctx->prof.recs.end(), ge->recs.begin(), ge->recs.end());
   } else {
-    enqueue_loop(ctx, pl, a);
+    enqueue_loop(ctx, pl, a, false);
   }
   CK(ctx, cudaGetLastError());
   CK(ctx, cudaEventRecord(ctx->pin_up_ev, s));  // (the loop reads its input from pinned memory)

@@ -618,8 +618,8 @@ __device__ __forceinline__ void cp_async_wait() {
 // options pixel by pixel.
 template <bool kStructured, bool kPlain, bool kFirst>
 __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS : 3)
-    k_corr_lin(const PairDev *__restrict__ pairs, int npairs, const int *__restrict__ tile_pair, int total_tiles,
-               CorrParams cp, LinParams lp, int flags) {
+    k_corr_lin(const PairDev *__restrict__ pairs, int npairs, const int *__restrict__ tile_pair, int first_tile,
+               int total_tiles, CorrParams cp, LinParams lp, int flags) {
   extern __shared__ __align__(16) unsigned char corr_smem_raw[];
   using Stage = GatherStage<kStructured>;
   Stage *stages = reinterpret_cast<Stage *>(corr_smem_raw);
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
   const int nsub = ntiles * kSubsPerTile;
   const bool drop_no_normal = kPlain || !cp.demoted;
   const bool first = kPlain ? kFirst : (flags & 1) != 0, reset = kPlain ? kFirst : (flags & 2) != 0;
-  auto tile_of = [&](int j) { return (int)blockIdx.x + (j / kSubsPerTile) * (int)gridDim.x; };
+  auto tile_of = [&](int j) { return first_tile + (int)blockIdx.x + (j / kSubsPerTile) * (int)gridDim.x; };
   auto stage_of = [&](int j) -> Stage & { return stages[j % corr_stages<kStructured>()]; };
 
   // Tile -> pair lookups, cached per pipeline stage (a stage's tile changes
@@ -1714,11 +1714,11 @@ static int corr_lin_grid(int total_tiles, int ctas_per_sm) {
 }
 
 template <bool kStructured, bool kPlain, bool kFirst>
-static void corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, const CorrParams &cp, const LinParams &lp,
-                     int flags, int ctas_per_sm, const int *tile_pair, cudaStream_t s) {
+static void corr_lin(const PairDev *d_pairs, int npairs, int first_tile, int total_tiles, const CorrParams &cp,
+                     const LinParams &lp, int flags, int ctas_per_sm, const int *tile_pair, cudaStream_t s) {
   const int grid = corr_lin_grid<kStructured, kPlain, kFirst>(total_tiles, ctas_per_sm);
   k_corr_lin<kStructured, kPlain, kFirst><<<grid, kFusedThreads, corr_smem<kStructured>(), s>>>(
-      d_pairs, npairs, tile_pair, total_tiles, cp, lp, flags);
+      d_pairs, npairs, tile_pair, first_tile, total_tiles, cp, lp, flags);
 }
 
 // Three CTAs of k_corr_tile fit on an SM.  Up to there the pass takes less
@@ -1733,8 +1733,8 @@ bool few_tiles(int npairs, int max_tiles) {
   return npairs <= 65535 && (long long)max_tiles * npairs <= (long long)kTileCtas * sms;
 }
 
-void launch_corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, int max_tiles, const CorrParams &cp,
-                     const LinParams &lp, int flags, bool structured, int ctas_per_sm, const int *tile_pair, cudaStream_t s,
+void launch_corr_lin(const PairDev *d_pairs, int npairs, int first_tile, int total_tiles, int max_tiles,
+                     const CorrParams &cp, const LinParams &lp, int flags, bool structured, int ctas_per_sm, const int *tile_pair, cudaStream_t s,
                      Profiler *prof) {
   if (total_tiles <= 0) return;
   configure_loop();
@@ -1745,11 +1745,11 @@ void launch_corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, int ma
     // (the reset goes with the first pass)
     const bool plain = !cp.demoted && cp.row_limit_threads <= 1 && !lp.demoted && !lp.z_scaling && lp.robust &&
                        ((flags & 3) == 0 || (flags & 3) == 3);
-    if (plain && (flags & 1)) corr_lin<true, true, true>(d_pairs, npairs, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
-    else if (plain) corr_lin<true, true, false>(d_pairs, npairs, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
-    else corr_lin<true, false, false>(d_pairs, npairs, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
+    if (plain && (flags & 1)) corr_lin<true, true, true>(d_pairs, npairs, first_tile, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
+    else if (plain) corr_lin<true, true, false>(d_pairs, npairs, first_tile, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
+    else corr_lin<true, false, false>(d_pairs, npairs, first_tile, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
   } else {
-    corr_lin<false, false, false>(d_pairs, npairs, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
+    corr_lin<false, false, false>(d_pairs, npairs, first_tile, total_tiles, cp, lp, flags, ctas_per_sm, tile_pair, s);
   }
   prof->end(NICP_K_CORR_LIN, s);
 }

@@ -158,8 +158,9 @@ void launch_resolve(const PairDev *d_pairs, int npairs, int max_tiles, int to_re
 // CTA per tile fits on the GPU at once: the fused pass then runs as
 // k_corr_tile and the loop's launches are chained.
 bool few_tiles(int npairs, int max_tiles);
-void launch_corr_lin(const PairDev *d_pairs, int npairs, int total_tiles, int max_tiles, const CorrParams &cp,
-                     const LinParams &lp, int flags, bool structured, int ctas_per_sm, const int *tile_pair, cudaStream_t s,
+// Pixel tiles [first_tile, first_tile + total_tiles) of the npairs pairs' images.
+void launch_corr_lin(const PairDev *d_pairs, int npairs, int first_tile, int total_tiles, int max_tiles,
+                     const CorrParams &cp, const LinParams &lp, int flags, bool structured, int ctas_per_sm, const int *tile_pair, cudaStream_t s,
                      Profiler *prof);
 void launch_corr_list(const PairDev *d_pairs, int npairs, int total_tiles, const CorrParams &cp, int use_state_T,
                       const float *explicit_T, cudaStream_t s, Profiler *prof);
