@@ -1356,7 +1356,7 @@ extern "C" int nicp_linearize(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_c
   const PairDev *dpd = (const PairDev *)(ctx->ws + pl.o_pairs);
   launch_lin_list(dpd, 1, pl.total_tiles, lin_params(*prm), std::max(1, parity_threads), 0,
                   (const float *)(ctx->ws + pl.o_krt), false, s, &ctx->prof);
-  launch_solve(dpd, 1, 0.0f, 2 | (prm->cross_block_f32 ? kSolveCrossF32 : 0), 0.0, 1, false, s, &ctx->prof);
+  launch_solve(dpd, 1, 0.0f, 2 | (prm->cross_block_f32 ? kSolveCrossF32 : 0), 0.0, 1, s, &ctx->prof);
   CK(ctx, cudaGetLastError());
   char *pd_host;
   if ((rc = pin_down(ctx, sizeof(PairState), &pd_host))) return rc;
@@ -1713,13 +1713,13 @@ extern "C" int nicp_align_nn(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cl
     std::swap(q.block_hits, q.next_hits);
     for (int k = 0; k < prm->inner_iterations; k++) {
       launch_lin_list(dpd, 1, pl.tiles, lp, 1, 1, nullptr, true, s, &ctx->prof);
-      launch_solve(dpd, 1, prm->lambda, ((k == prm->inner_iterations - 1) ? 1 : 0) | xb, prm->early_exit_eps, 0, true,
+      launch_solve(dpd, 1, prm->lambda, ((k == prm->inner_iterations - 1) ? 1 : 0) | xb, prm->early_exit_eps, 0,
                    s, &ctx->prof);
     }
   }
   if (prm->compute_statistics) {
     launch_lin_list(dpd, 1, pl.tiles, lp, 1, 2, nullptr, true, s, &ctx->prof);
-    launch_solve(dpd, 1, 0.0f, 4 | xb, 0.0, 1, true, s, &ctx->prof);
+    launch_solve(dpd, 1, 0.0f, 4 | xb, 0.0, 1, s, &ctx->prof);
   }
   char *res;
   if ((rc = pin_down(ctx, sizeof(PairState), &res))) return rc;
@@ -2006,6 +2006,11 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
   const int xb = a.lin->cross_block_f32 ? kSolveCrossF32 : 0;
   // (list mode's kernels and the general fused kernel are not part of a chain)
   const bool chained = pl.structured && few_tiles(pl.n, pl.max_tiles);
+  // After the solve of one or two pairs the projection is chained too: it finds
+  // all SMs but those free (two 640x480 pairs 480 -> 472 us, one 1280x720 600 ->
+  // 590).  More solves upset the placement of its CTAs (three 640x480 pairs 531
+  // -> 537 us, two 1280x720 874 -> 930).
+  const bool chained_projection = chained || (pl.structured && pl.n <= 2);
   int *tile_pair = (int *)(ctx->ws + pl.o_tile_pair);
   BeginArgs begin = a.begin;
   begin.npairs = pl.n;
@@ -2035,8 +2040,7 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
         for (int k = 0; k < inner; k++) {
           const int flags = (k == 0) ? (1 | 2 | (pl.keep_ref ? 4 : 0)) : 0;
           launch_corr_lin(dpd, pl.n, t0, tn, pl.max_tiles, cp, lp, flags, true, L.corr_ctas, tile_pair, q, &ctx->prof);
-          launch_solve(dpd + p0, n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, false, q,
-                       &ctx->prof);
+          launch_solve(dpd + p0, n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, q, &ctx->prof);
         }
       }
       if (g) cudaEventRecord(ctx->fork_ev[g], q);
@@ -2044,20 +2048,20 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
     for (int g = 1; g < parts; g++) cudaStreamWaitEvent(s, ctx->fork_ev[g], 0);
   }
   for (int i = 0; i < outer && !fork; i++) {
-    launch_zbuffer(dpd, pl.n, pl.max_pt_tiles, 1, nullptr, L.zb_ppt, chained, s, &ctx->prof);
+    launch_zbuffer(dpd, pl.n, pl.max_pt_tiles, 1, nullptr, L.zb_ppt, i ? chained_projection : chained, s, &ctx->prof);
     if (pl.list_mode) {
       launch_resolve(dpd, pl.n, pl.max_tiles, 1, nullptr, 0, false, s, &ctx->prof);
       launch_corr_list(dpd, pl.n, pl.total_tiles, cp, 1, nullptr, s, &ctx->prof);
       for (int k = 0; k < inner; k++) {
         launch_lin_list(dpd, pl.n, pl.total_tiles, lp, std::max(1, a.corr->parity_threads), 1, nullptr, false, s, &ctx->prof);
-        launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, chained, s, &ctx->prof);
+        launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, s, &ctx->prof);
       }
     } else {
       for (int k = 0; k < inner; k++) {
         int flags = (k == 0) ? (1 | 2 | (pl.keep_ref ? 4 : 0)) : 0;
         launch_corr_lin(dpd, pl.n, 0, pl.total_tiles, pl.max_tiles, cp, lp, flags, pl.structured, L.corr_ctas, tile_pair, s,
                         &ctx->prof);
-        launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, chained, s, &ctx->prof);
+        launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, s, &ctx->prof);
       }
     }
   }
@@ -2068,9 +2072,10 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
       launch_lin_list(dpd, pl.n, pl.total_tiles, lp, std::max(1, a.corr->parity_threads), 2, nullptr, false, s, &ctx->prof);
     else
       launch_corr_lin(dpd, pl.n, 0, pl.total_tiles, pl.max_tiles, cp, lp, 8, pl.structured, L.corr_ctas, tile_pair, s, &ctx->prof);
-    launch_solve(dpd, pl.n, 0.0f, 4 | xb, 0.0, 1, chained, s, &ctx->prof);
+    launch_solve(dpd, pl.n, 0.0f, 4 | xb, 0.0, 1, s, &ctx->prof);
   }
-  launch_publish((const PairState *)(ctx->ws + pl.o_states), a.results, pl.n, chained, s, &ctx->prof);
+  // (behind the parts' join there is more than one launch to wait for)
+  launch_publish((const PairState *)(ctx->ws + pl.o_states), a.results, pl.n, !fork || stats, s, &ctx->prof);
 }
 
 static std::string graph_key(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) {

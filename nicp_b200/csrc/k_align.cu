@@ -631,6 +631,7 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
   __shared__ float4 sW[kConstSlots][kWeightEntries];  // structured: weights by point code
   __shared__ int sPair[kConstSlots], sSkip[kConstSlots], sStruct[kConstSlots], sSame[kConstSlots];
   const bool stats_pass = flags & 8;
+  chain_next();  // the solve's CTAs
   if ((int)blockIdx.x >= total_tiles) return;
   const int ntiles = (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int nsub = ntiles * kSubsPerTile;
@@ -646,7 +647,7 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
   auto lookup = [&](int tile, int &ctile, int &cpi, bool &cskip) {
     if (tile != ctile) {
       ctile = tile;
-      cpi = tile_pair[tile];  // filled once per alignment by k_tile_pairs
+      cpi = tile_pair[tile];  // filled once per alignment by k_begin_loop
       cskip = !stats_pass && pairs[cpi].state->done;
     }
   };
@@ -1789,10 +1790,10 @@ void launch_publish(const PairState *states, PairState *host, int npairs, bool c
 }
 
 void launch_solve(const PairDev *d_pairs, int npairs, float lambda, int mode, double early_eps, int ignore_done,
-                  bool chained, cudaStream_t s, Profiler *prof) {
+                  cudaStream_t s, Profiler *prof) {
   configure_loop();
   prof->begin(NICP_K_SOLVE, s);
-  launch(chained, k_solve, npairs, kSumThreads, 0, s, d_pairs, npairs, lambda, mode, early_eps, ignore_done);
+  launch(true, k_solve, npairs, kSumThreads, 0, s, d_pairs, npairs, lambda, mode, early_eps, ignore_done);
   prof->end(NICP_K_SOLVE, s);
 }
 
