@@ -88,3 +88,22 @@ def test_tile_partials_add_up(ctx, tiles):
     assert inliers == count
     eps = 300 * 2.0 ** -53
     assert np.all(np.abs(H - Hs) <= 2 * eps * mags) and np.all(np.abs(b - bs) <= 2 * eps * magb)
+
+
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 9])
+def test_parts_of_a_batch(ctx, n):
+    """A batch's loop runs in one to four parts, cut by tiles: each pair's
+    result is what it is alone, wherever the cuts fall."""
+    corr, lin, prm = api.CorrespondenceFinderProjective(ctx).params(), api.Linearizer(ctx).params(), L.AlignParams()
+    ctx.lib.nicp_default_align_params(prm)
+    prm.outer_iterations = 4
+    pairs = [_pair(ctx, rows, cols, 11 + rows) for rows, cols in ((480, 640), (60, 80), (337, 451))]
+    order = [0] * n + [1, 2]  # n of 300 tiles, then 5 and 149
+    order = order[n // 2:] + order[:n // 2]
+    alone = [api.align_batch(ctx, [c[0]], [c[1]], [p.camera()], None, corr, lin, prm)[0] for p, c in pairs]
+    many = api.align_batch(ctx, [pairs[k][1][0] for k in order], [pairs[k][1][1] for k in order],
+                           [pairs[k][0].camera() for k in order], None, corr, lin, prm)
+    for k, r in zip(order, many):
+        assert np.array_equal(np.array(alone[k].T), np.array(r.T), equal_nan=True)
+        assert np.float32(alone[k].error).tobytes() == np.float32(r.error).tobytes()
+        assert (alone[k].inliers, alone[k].num_correspondences) == (r.inliers, r.num_correspondences)
