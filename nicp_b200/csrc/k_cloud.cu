@@ -339,77 +339,39 @@ __device__ __forceinline__ void point_moments(float4 p, bool valid, float m[10])
   m[7] = v * fm(y, y); m[8] = v * fm(y, z); m[9] = v * fm(z, z);
 }
 
-constexpr int kRowThreads = 128;
-constexpr int kRowPix = 5;  // 128 x 5 = 640: one chunk per 640-pixel row
-
-// One chunk of one image row (kRowThreads x kRowPix pixels from x0):
-// inclusive prefix along x of the 10 moments, starting from carry[] (the
-// chunks to its left), which is advanced by the chunk total.  Each thread
-// keeps the points of its kRowPix pixels (depths d[]); the moments are
-// formed twice (for the thread total, then per pixel for emit) to keep
-// register use low.  emit(k, c, acc) receives pixel c = x0 + t kRowPix + k
-// with its 10 prefix values.  [kM0, kM0 + kNM) selects the moments the call
-// scans (the band sweep runs two calls of five, which halves the registers
-// the pixels' moments hold and fits 4 CTAs per SM; every moment's additions
-// are the same either way).  Contains two __syncthreads.
-template <class M, int kM0 = 0, int kNM = 10, class Emit>
-__device__ __forceinline__ void row_chunk_scan(const FrameDev &f, int r, int x0, const float d[kRowPix],
-                                               typename MomAcc<M>::T carry[10],
-                                               typename MomAcc<M>::T (*wtot)[10], Emit &&emit) {
-  typedef typename MomAcc<M>::T A;
-  const int cols = f.cols;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int c0 = x0 + threadIdx.x * kRowPix;
-  float4 pt[kRowPix];
-  unsigned vmask = 0;
-  A acc[10];
-#pragma unroll
-  for (int m = kM0; m < kM0 + kNM; m++) acc[m] = A(0);
-#pragma unroll
-  for (int k = 0; k < kRowPix; k++) {
-    const int c = c0 + k;
-    const bool valid = c < cols && depth_valid(d[k], f.min_d, f.max_d);
-    pt[k] = valid ? unproject_pixel(f.iKRt, c, r, d[k]) : make_float4(0, 0, 0, 0);
-    vmask |= (valid ? 1u : 0u) << k;
-    A mk[10];
-    point_moments(pt[k], valid, mk);
-#pragma unroll
-    for (int m = kM0; m < kM0 + kNM; m++) acc[m] = acc[m] + mk[m];
-  }
-  // warp inclusive scan of the thread totals; acc becomes the exclusive offset
-#pragma unroll
-  for (int m = kM0; m < kM0 + kNM; m++) {
-    A inc = acc[m];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      A y = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc = inc + y;
-    }
-    if (lane == 31) wtot[wid][m] = inc;
-    acc[m] = inc - acc[m];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int m = kM0; m < kM0 + kNM; m++) {
-    A off = carry[m] + acc[m], tot = A(0);
-    for (int w = 0; w < kRowThreads / 32; w++) {
-      A t = wtot[w][m];
-      if (w < wid) off = off + t;
-      tot = tot + t;
-    }
-    acc[m] = off;
-    carry[m] = carry[m] + tot;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < kRowPix; k++) {
-    A mk[10];
-    point_moments(pt[k], (vmask >> k) & 1u, mk);
-#pragma unroll
-    for (int m = kM0; m < kM0 + kNM; m++) acc[m] = acc[m] + mk[m];
-    emit(k, c0 + k, acc);
+// Moment m (a compile-time constant) of a point as point_moments forms it.
+__device__ __forceinline__ double moment_of(int m, float4 p, double v) {
+  const double x = p.x, y = p.y, z = p.z;
+  switch (m) {
+    case 0: return v;
+    case 1: return v * x;
+    case 2: return v * y;
+    case 3: return v * z;
+    case 4: return v * x * x;
+    case 5: return v * x * y;
+    case 6: return v * x * z;
+    case 7: return v * y * y;
+    case 8: return v * y * z;
+    default: return v * z * z;
   }
 }
+__device__ __forceinline__ float moment_of(int m, float4 p, float v) {
+  switch (m) {
+    case 0: return v;
+    case 1: return v * p.x;
+    case 2: return v * p.y;
+    case 3: return v * p.z;
+    case 4: return v * fm(p.x, p.x);
+    case 5: return v * fm(p.x, p.y);
+    case 6: return v * fm(p.x, p.z);
+    case 7: return v * fm(p.y, p.y);
+    case 8: return v * fm(p.y, p.z);
+    default: return v * fm(p.z, p.z);
+  }
+}
+
+constexpr int kRowThreads = 128;
+constexpr int kRowPix = 5;  // 128 x 5 = 640: one chunk per 640-pixel row
 
 // Raw depth words (u16 value or float bits), loaded ahead of use; the
 // conversion happens where the depth is consumed, so that a prefetch does
@@ -436,9 +398,13 @@ __device__ __forceinline__ void load_row_raw(const FrameDev &f, int r, int c0, u
 //                          sum of the band's row prefixes)
 //   k_moments_band_carry   per (plane, column): exclusive prefix of the
 //                          band totals over the bands, in place
-//   k_moments_band_sweep   per band: row prefixes (row_chunk_scan) added
-//                          down the band onto carry_b; every integral value
-//                          is written once, from shared memory, coalesced
+//   k_moments_band_sweep   per band: row prefixes added down the band onto
+//                          carry_b; every integral value is written once,
+//                          coalesced
+// Row prefixes are formed the same way everywhere, so that a frame's planes do
+// not depend on its batch: totals of kRowPix adjacent pixels, an inclusive
+// shuffle scan of 32 of them, then the segments' totals from left to right
+// within a chunk of kRowThreads x kRowPix columns.
 constexpr int kBandRows = 16;
 constexpr int kChunkPix = kRowThreads * kRowPix;
 
@@ -563,78 +529,146 @@ __global__ void __launch_bounds__(128) k_moments_band_carry(const FrameDev *__re
   }
 }
 
-// Grid (band, frame): the frame is blockIdx.y, no search over the frame
-// descriptors; CTAs past a smaller frame's last band return at once.
+// One CTA per band, a warp per image row, 160 columns (a segment) and one plane
+// pair at a time: the warps scan their rows into a shared tile, then a thread
+// per column adds the rows up from registers and writes them.  Bound by the
+// latency of its steps more than by anything else (a step's scan and column
+// sums overlap only with the other CTA's and, as the tiles alternate, with the
+// next step's scan), with 61 % of the DRAM rate at 200 frames of 640x480.  A
+// CTA of four warps that scanned one row at a time, all ten planes, with the
+// running sums in shared memory moved each value through shared memory three
+// times (now twice, 16 bytes at once) behind five barriers per row (now ten per
+// segment) and kept its 128 threads whatever the width: 1717 -> 1191 us for 200
+// frames of 640x480, 112 -> 58 for 9, 2519 -> 1275 for 384 of three sizes down to
+// 160x120.  Half the rows at a time with 3 CTAs of 256 threads: 1287, 74, 1314;
+// a CTA per plane pair: 1759 to 2199 for the 200.
+constexpr int kSweepThreads = 32 * kBandRows;
+constexpr int kSegPix = 32 * kRowPix;    // 160: five adjacent pixels per lane
+constexpr int kSegs = kRowThreads / 32;  // segments per chunk of kChunkPix columns
+template <class A>
+struct __align__(2 * sizeof(A)) MomentPair {
+  A a, b;
+};
 template <class M>
-__global__ void __launch_bounds__(kRowThreads, 4) k_moments_band_sweep(const FrameDev *__restrict__ frames, int nframes) {
+struct SweepSmem {
+  typedef MomentPair<typename MomAcc<M>::T> Pair;
+  Pair tile[2][kBandRows][kSegPix];  // row prefixes
+  Pair total[kBandRows][5][kSegs];   // the rows' segment totals
+  Pair left[kBandRows][5];           // sums left of the chunk (frames wider than a chunk)
+};
+
+// Plane pair K of one segment.  pt, vmask: the lane's points in its warp's row;
+// buf: the tile to write.
+template <class M, int K>
+__device__ __forceinline__ void sweep_pair(SweepSmem<M> &sm, const FrameDev &f, const typename MomAcc<M>::T *carry_b,
+                                           int r0, int nr, int x0, int seg, float4 *pt, unsigned vmask, int &buf) {
+  typedef typename MomAcc<M>::T A;
+  typedef MomentPair<A> Pair;
+  const int t = threadIdx.x, lane = t & 31, row = t >> 5, cols = f.cols;
+  const int c = x0 + seg * kSegPix + t;
+  const bool column = t < kSegPix && c < cols;
+  const size_t P = (size_t)f.rows * cols;
+  A sa = A(0), sb = A(0);  // the column's sums down to the current row
+  if (column) {
+    sa = carry_b[(size_t)(2 * K) * cols + c];
+    sb = carry_b[(size_t)(2 * K + 1) * cols + c];
+  }
+  if (row < nr) {
+    A va[kRowPix], vb[kRowPix], ta = A(0), tb = A(0);
+#pragma unroll
+    for (int k = 0; k < kRowPix; k++) {
+      // (an invalid point is 0: only the count needs the mask)
+      va[k] = K == 0 ? ((vmask >> k) & 1u ? A(1) : A(0)) : moment_of(2 * K, pt[k], A(1));
+      vb[k] = moment_of(2 * K + 1, pt[k], A(1));
+      ta = ta + va[k];
+      tb = tb + vb[k];
+    }
+    A ia = ta, ib = tb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const A ya = __shfl_up_sync(0xffffffffu, ia, o), yb = __shfl_up_sync(0xffffffffu, ib, o);
+      if (lane >= o) {
+        ia = ia + ya;
+        ib = ib + yb;
+      }
+    }
+    Pair l = {A(0), A(0)};
+    if (x0) l = sm.left[row][K];
+    A oa = l.a + (ia - ta), ob = l.b + (ib - tb);
+    A qa = A(0), qb = A(0);
+    for (int w = 0; w < seg; w++) {  // (written by this warp, barriers ago)
+      const Pair q = sm.total[row][K][w];
+      oa = oa + q.a;
+      ob = ob + q.b;
+      qa = qa + q.a;
+      qb = qb + q.b;
+    }
+    if (lane == 31) {
+      sm.total[row][K][seg] = {ia, ib};
+      if (seg == kSegs - 1) sm.left[row][K] = {l.a + (qa + ia), l.b + (qb + ib)};
+    }
+    Pair *out = sm.tile[buf][row] + lane * kRowPix;
+#pragma unroll
+    for (int k = 0; k < kRowPix; k++) {
+      oa = oa + va[k];
+      ob = ob + vb[k];
+      out[k] = {oa, ob};
+    }
+  }
+  // one barrier per step: a tile is written again only after the next step's
+  __syncthreads();
+  if (column) {
+#pragma unroll
+    for (int i = 0; i < kBandRows; i++) {
+      if (i < nr) {
+        const Pair q = sm.tile[buf][i][t];
+        sa = sa + q.a;
+        sb = sb + q.b;
+        M::store2(f.moments, P, K, (size_t)(r0 + i) * cols + c, (double)sa, (double)sb);
+      }
+    }
+  }
+  buf ^= 1;
+}
+
+// Grid (band, frame): the frame is blockIdx.y, no search over the frame
+// descriptors; CTAs past a smaller frame's last band return at once.  only: the
+// plane pair to write, all five if negative -- the launch writes all, but with
+// a condition on each the compiler keeps to 64 registers; five in a row share
+// offsets and conversions and spill 1.3 KB (1330 us instead of 1191).
+template <class M>
+__global__ void __launch_bounds__(kSweepThreads, 2) k_moments_band_sweep(const FrameDev *__restrict__ frames, int only) {
   typedef typename MomAcc<M>::T A;
   extern __shared__ __align__(16) unsigned char band_raw[];
-  A *state = reinterpret_cast<A *>(band_raw);  // [10][kChunkPix]: I(r, c) of the current row
-  __shared__ A wtot[kRowThreads / 32][10];
-  __shared__ A rowc[kBandRows][10];  // row carries across chunks (frames wider than a chunk)
+  SweepSmem<M> &sm = *reinterpret_cast<SweepSmem<M> *>(band_raw);
   const FrameDev &f = frames[blockIdx.y];
-  const int b = blockIdx.x;
   const int cols = f.cols;
-  const size_t P = (size_t)f.rows * cols;
-  if (b * kBandRows >= f.rows) return;
-  const int r0 = b * kBandRows, r1 = min(f.rows, r0 + kBandRows);
-  const A *carry_b = static_cast<const A *>(f.band_tot) + (size_t)b * 10 * cols;
-  const int t = threadIdx.x;
+  const int r0 = (int)blockIdx.x * kBandRows, nr = min(f.rows - r0, kBandRows);
+  if (nr <= 0) return;
+  const A *carry_b = static_cast<const A *>(f.band_tot) + (size_t)blockIdx.x * 10 * cols;
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  int buf = 0;
   for (int x0 = 0; x0 < cols; x0 += kChunkPix) {
-    const int n = min(kChunkPix, cols - x0);
-    const int c0 = x0 + t * kRowPix;
-    // the band's carry row; made visible to the owners of the columns by the
-    // first barrier inside the first scan
+    for (int seg = 0; seg < kSegs && x0 + seg * kSegPix < cols; seg++) {
+      const int c0 = x0 + seg * kSegPix + lane * kRowPix;
+      unsigned raw[kRowPix];
 #pragma unroll
-    for (int m = 0; m < 10; m++)
+      for (int k = 0; k < kRowPix; k++) raw[k] = row < nr && c0 + k < cols ? depth_raw(f, (r0 + row) * cols + c0 + k) : 0u;
+      float4 pt[kRowPix];
+      unsigned vmask = 0;
 #pragma unroll
-      for (int j = 0; j < kRowPix; j++) {
-        const int q = j * kRowThreads + t;
-        state[m * kChunkPix + q] = q < n ? carry_b[(size_t)m * cols + x0 + q] : A(0);
+      for (int k = 0; k < kRowPix; k++) {
+        const float d = depth_from_raw(f, raw[k]);
+        const bool valid = c0 + k < cols && depth_valid(d, f.min_d, f.max_d);
+        pt[k] = valid ? unproject_pixel(f.iKRt, c0 + k, r0 + row, d) : make_float4(0, 0, 0, 0);
+        vmask |= (valid ? 1u : 0u) << k;
       }
-    unsigned wn[kRowPix];
-    load_row_raw(f, r0, c0, wn);
-    for (int r = r0; r < r1; r++) {
-      float d[kRowPix];
-#pragma unroll
-      for (int k = 0; k < kRowPix; k++) d[k] = depth_from_raw(f, wn[k]);
-      if (r + 1 < r1) load_row_raw(f, r + 1, c0, wn);
-      A carry[10];
-#pragma unroll
-      for (int m = 0; m < 10; m++) carry[m] = x0 ? rowc[r - r0][m] : A(0);
-      // every thread has finished the previous row's copy-out once it has
-      // passed the first barrier inside the scan
-      row_chunk_scan<M, 0, 5>(f, r, x0, d, carry, wtot, [&](int, int c, const A *acc) {
-        if (c < cols) {
-#pragma unroll
-          for (int m = 0; m < 5; m++)
-            state[m * kChunkPix + (c - x0)] = state[m * kChunkPix + (c - x0)] + acc[m];
-        }
-      });
-      row_chunk_scan<M, 5, 5>(f, r, x0, d, carry, wtot, [&](int, int c, const A *acc) {
-        if (c < cols) {
-#pragma unroll
-          for (int m = 5; m < 10; m++)
-            state[m * kChunkPix + (c - x0)] = state[m * kChunkPix + (c - x0)] + acc[m];
-        }
-      });
-      if (t == 0 && x0 + kChunkPix < cols) {
-#pragma unroll
-        for (int m = 0; m < 10; m++) rowc[r - r0][m] = carry[m];
-      }
-      __syncthreads();
-      const size_t row0 = (size_t)r * cols + x0;
-#pragma unroll
-      for (int k = 0; k < 5; k++)
-#pragma unroll
-        for (int j = 0; j < kRowPix; j++) {
-          const int q = j * kRowThreads + t;
-          if (q < n)
-            M::store2(f.moments, P, k, row0 + q, (double)state[2 * k * kChunkPix + q],
-                      (double)state[(2 * k + 1) * kChunkPix + q]);
-        }
+      if (only < 0 || only == 0) sweep_pair<M, 0>(sm, f, carry_b, r0, nr, x0, seg, pt, vmask, buf);
+      if (only < 0 || only == 1) sweep_pair<M, 1>(sm, f, carry_b, r0, nr, x0, seg, pt, vmask, buf);
+      if (only < 0 || only == 2) sweep_pair<M, 2>(sm, f, carry_b, r0, nr, x0, seg, pt, vmask, buf);
+      if (only < 0 || only == 3) sweep_pair<M, 3>(sm, f, carry_b, r0, nr, x0, seg, pt, vmask, buf);
+      if (only < 0 || only == 4) sweep_pair<M, 4>(sm, f, carry_b, r0, nr, x0, seg, pt, vmask, buf);
     }
-    __syncthreads();  // the last copy-out has read the state before the next chunk's carry row
   }
 }
 
@@ -1030,37 +1064,6 @@ constexpr int kFewThreads = kFewRows * kRowThreads;      // 640: also a column e
 static_assert(kFewThreads == kChunkPix, "a band CTA has a thread per column of a chunk");
 static_assert(2 * kFewRows == 10, "two moments per 128 threads");
 
-// Moment m (a compile-time constant) of a point as point_moments forms it.
-__device__ __forceinline__ double moment_of(int m, float4 p, double v) {
-  const double x = p.x, y = p.y, z = p.z;
-  switch (m) {
-    case 0: return v;
-    case 1: return v * x;
-    case 2: return v * y;
-    case 3: return v * z;
-    case 4: return v * x * x;
-    case 5: return v * x * y;
-    case 6: return v * x * z;
-    case 7: return v * y * y;
-    case 8: return v * y * z;
-    default: return v * z * z;
-  }
-}
-__device__ __forceinline__ float moment_of(int m, float4 p, float v) {
-  switch (m) {
-    case 0: return v;
-    case 1: return v * p.x;
-    case 2: return v * p.y;
-    case 3: return v * p.z;
-    case 4: return v * fm(p.x, p.x);
-    case 5: return v * fm(p.x, p.y);
-    case 6: return v * fm(p.x, p.z);
-    case 7: return v * fm(p.y, p.y);
-    case 8: return v * fm(p.y, p.z);
-    default: return v * fm(p.z, p.z);
-  }
-}
-
 // Row prefix of the image row r by 128 threads (their barrier: `bar`).
 template <class M>
 __device__ __forceinline__ void row_prefix(const FrameDev &f, int r, int bar, typename MomAcc<M>::T (*stage)[kChunkPix],
@@ -1308,7 +1311,7 @@ static void configure_bands() {
   cudaGetDevice(&dev);
   auto set = [] {
     cudaFuncSetAttribute(k_moments_band_totals<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, band_smem_bytes<M>());
-    cudaFuncSetAttribute(k_moments_band_sweep<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, band_smem_bytes<M>());
+    cudaFuncSetAttribute(k_moments_band_sweep<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SweepSmem<M>));
     cudaFuncSetAttribute(k_build_rows<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, band_smem_bytes<M>());
   };
   if (dev >= 0 && dev < kMaxDevices)
@@ -1326,7 +1329,7 @@ static void launch_bands(const FrameDev *d_frames, int nframes, int total_bands,
   k_moments_band_carry<M><<<total_carry_ctas, 128, 0, s>>>(d_frames, frame_of_carry);
   prof->end(NICP_K_MOMENTS_BANDS, s, 2);
   prof->begin(NICP_K_MOMENTS_SWEEP, s);
-  k_moments_band_sweep<M><<<dim3(max_bands, nframes), kRowThreads, band_smem_bytes<M>(), s>>>(d_frames, nframes);
+  k_moments_band_sweep<M><<<dim3(max_bands, nframes), kSweepThreads, sizeof(SweepSmem<M>), s>>>(d_frames, -1);
   prof->end(NICP_K_MOMENTS_SWEEP, s);
 }
 
@@ -1374,7 +1377,7 @@ template <class M>
 static int sweep_occupancy() {
   configure_bands<M>();
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_moments_band_sweep<M>, kRowThreads, band_smem_bytes<M>()) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_moments_band_sweep<M>, kSweepThreads, sizeof(SweepSmem<M>)) !=
       cudaSuccess) {
     cudaGetLastError();
     n = 0;
