@@ -10,13 +10,18 @@
 //                (correspondencefinderprojective.cpp:23-115) and Linearizer::update
 //                (linearizer.cpp:21-134): per pixel, gate the pair, and if accepted
 //                add its 21 H + 6 b + chi2 + inlier terms.  Per-thread sums in FP32
-//                over 4 pixels, then FP64: warp butterfly reduce-scatter, shared
-//                memory, one partial per CTA tile (fixed tile -> partial mapping).
+//                over 8 pixels, then FP64: transposed through shared memory, one
+//                partial per 1024-pixel tile (fixed tile -> partial mapping).
+//   k_corr_tile  the same pass, the same sums in the same order, one CTA per
+//                tile: loops of few tiles.
 //   k_corr_count / k_corr_write
 //                the same gates with ordered compaction into the reference's
 //                row-major correspondence list (parity / list mode).
 //   k_lin_list   Linearizer::update over a correspondence list (with the
 //                reference's K % T drop when T > 1).
+//   k_begin_loop / k_publish
+//                descriptors and poses from pinned host memory, states, tables and
+//                empty z-buffers; the states back to pinned host memory.
 //   k_solve      per pair: fixed-order FP64 sum of the tile partials, H + lambda I,
 //                6x6 LDL^T, pose update and renormalisation (alignerprojective.cpp:
 //                72-100), early exit, and the float matrices of the next iteration.

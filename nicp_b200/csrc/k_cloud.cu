@@ -13,6 +13,10 @@
 //       planes, over bands of 16 image rows: band column totals, their
 //       prefix over the bands, then one sweep per band that writes every
 //       value once.
+//   k_build_rows / k_build_planes
+//       the unprojection and the same planes for launches of one or two
+//       frames: every row prefix in parallel, then the points and the sums
+//       down the columns.
 //   k_stats
 //       one thread per pixel: interval radius, 4-corner box query, FP64 3x3
 //       covariance and eigensolve, curvature, oriented normal, and both
@@ -20,6 +24,8 @@
 //       informationmatrixcalculator.cpp:9-57).
 //   k_cloud_transform
 //       Cloud::transformInPlace (cloud.cpp:191-204).
+//   k_cloud_export
+//       a cloud in the layout of a download.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -603,6 +609,7 @@ __device__ __forceinline__ void sweep_pair(SweepSmem<M> &sm, const FrameDev &f, 
       qa = qa + q.a;
       qb = qb + q.b;
     }
+    __syncwarp();  // all lanes have read the row's sums to the left
     if (lane == 31) {
       sm.total[row][K][seg] = {ia, ib};
       if (seg == kSegs - 1) sm.left[row][K] = {l.a + (qa + ia), l.b + (qb + ib)};
