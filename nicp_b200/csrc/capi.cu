@@ -1878,7 +1878,7 @@ extern "C" int nicp_merge(nicp_ctx *ctx, nicp_cloud *cloud, const nicp_camera *c
   for (int k = 0; k < 7; k++) o_int[k] = E.take(4 * N);
   size_t scan_bytes = merge_scan_temp_bytes(n);
   size_t o_scan = E.take(scan_bytes);
-  size_t o_pts = E.take(16 * N), o_nrm = E.take(16 * N), o_omg = E.take(48 * N);
+  size_t o_pts = E.take(16 * N), o_nrm = E.take(16 * N), o_omg = E.take(cloud->omg_valid ? 48 * N : 16);
   size_t o_eig = E.take(cloud->eig_valid ? 4 * kStatsWords * N : 16), o_gauss = E.take(48 * N), o_cnt = E.take(8);
   PairPlan pl;
   const nicp_cloud *cc = cloud;
@@ -1905,7 +1905,7 @@ extern "C" int nicp_merge(nicp_ctx *ctx, nicp_cloud *cloud, const nicp_camera *c
   a.count = cloud->count;
   a.pts = cloud->pts;
   a.nrm = cloud->nrm;
-  a.omg = cloud->omg;
+  a.omg = cloud->omg_valid ? cloud->omg : nullptr;
   a.eig = cloud->eig_valid ? cloud->eig : nullptr;
   a.gauss = cloud->gauss;
   a.KRt12 = (const float *)(ctx->ws + pl.o_krt);
@@ -1929,17 +1929,15 @@ extern "C" int nicp_merge(nicp_ctx *ctx, nicp_cloud *cloud, const nicp_camera *c
   a.o_eig = cloud->eig_valid ? (float *)(ex + o_eig) : nullptr;
   a.o_gauss = (float4 *)(ex + o_gauss);
   a.out_count = (int *)(ex + o_cnt);
+  a.back = {{a.o_pts, a.o_nrm, a.o_omg, (const float4 *)a.o_eig, a.o_gauss},
+            {cloud->pts, cloud->nrm, a.omg ? cloud->omg : nullptr, a.o_eig ? (float4 *)cloud->eig : nullptr,
+             cloud->gauss},
+            a.out_count,
+            cloud->count};
   if (launch_merge(a, s)) {
     cudaError_t e = cudaGetLastError();
     return fail(ctx, NICP_ECUDA, std::string("merge: ") + cudaGetErrorString(e));
   }
-  // the compacted cloud back in place
-  CK(ctx, cudaMemcpyAsync(cloud->pts, a.o_pts, 16 * N, cudaMemcpyDeviceToDevice, s));
-  CK(ctx, cudaMemcpyAsync(cloud->nrm, a.o_nrm, 16 * N, cudaMemcpyDeviceToDevice, s));
-  CK(ctx, cudaMemcpyAsync(cloud->omg, a.o_omg, 48 * N, cudaMemcpyDeviceToDevice, s));
-  if (a.o_eig) CK(ctx, cudaMemcpyAsync(cloud->eig, a.o_eig, 4 * kStatsWords * N, cudaMemcpyDeviceToDevice, s));
-  CK(ctx, cudaMemcpyAsync(cloud->gauss, a.o_gauss, 48 * N, cudaMemcpyDeviceToDevice, s));
-  CK(ctx, cudaMemcpyAsync(cloud->count, a.out_count, 2 * sizeof(int), cudaMemcpyDeviceToDevice, s));
   int after[2];
   if ((rc = cloud_counts2(cloud, after))) return rc;
   if (removed) *removed = n - after[0];

@@ -210,10 +210,19 @@ int lin_noalloc(const NoAllocLinArgs &args, double *out_dev, cudaStream_t s);
 // Merger::merge on the device (k_merge.cu).  n points (host copy of *count);
 // every per-point array below holds n ints; the o_* staging arrays receive the
 // compacted cloud, out_count its counts (points, points with a normal).
+struct MergeBack {
+  const float4 *src[5];  // points, normals, information matrices, eigen, Gaussians
+  float4 *dst[5];        // (null: not kept)
+  const int *out_count;
+  int *count;
+  // float4 words per point
+  __host__ __device__ static constexpr int words(int q) { return q < 2 ? 1 : q == 3 ? kStatsWords / 4 : 3; }
+};
 struct MergeArgs {
   int n;
   const int *count;
-  const float4 *pts, *nrm, *omg;
+  const float4 *pts, *nrm;
+  const float4 *omg;      // or null (implicit)
   const float *eig;       // or null
   float4 *gauss;          // fused in place
   const float *KRt12;     // device, the projector's KRt for the merge transform
@@ -228,6 +237,7 @@ struct MergeArgs {
   float *o_eig;
   float4 *o_gauss;
   int *out_count;
+  MergeBack back;
 };
 // Uniform grid over the current cloud's xyz (k_nn.cu).
 struct NNGrid {
