@@ -143,3 +143,32 @@ def test_merge_keeps_implicit_omega_consistent(ctx):
     (da, ra), (db, rb) = out
     assert ra == rb
     _check_same_omega(da, db, 1e-6)
+
+
+def test_merge_moves_every_array(ctx):
+    """A merge keeps its survivors in order: their rows of every array that it
+    does not change (normals, curvature, eigenpairs, Omega) are a subsequence
+    of the rows before it."""
+    d1, _, _, cam = synth.render_pair(37, "320x240")
+    _, conv = converter(cam, ctx, keep_stats=True)
+    conv.keepGaussians = True
+    a, b = api.Cloud(ctx), api.Cloud(ctx)
+    conv.compute(a, d1)
+    conv.compute(b, d1)
+    a.add(b, np.eye(4))
+
+    def rows():
+        d = a.download(stats=True)
+        n = len(d["points"])
+        keys = ("normals", "curvature", "omega_p", "omega_n", "eigenvalues", "eigenvectors")
+        return [r.tobytes() for r in np.concatenate([np.float32(d[k]).reshape(n, -1) for k in keys], axis=1)]
+
+    before = rows()
+    m = api.Merger(ctx)
+    m.setDepthImageConverter(conv)
+    m.setImageSize(cam["rows"], cam["cols"])
+    m.merge(a, np.eye(4))
+    after = rows()
+    assert len(after) == len(before) - m.removed and 0 < m.removed < len(before)
+    rest = iter(before)
+    assert all(r in rest for r in after)
