@@ -19,6 +19,7 @@
 #include "host_math.hpp"
 #include "kernels.hpp"
 #include "nicp_gpu.h"
+#include "pair_plan.hpp"
 
 using namespace nicp;
 
@@ -31,22 +32,7 @@ struct GraphEntry {
   std::vector<Profiler::Rec> recs;
 };
 
-size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
-
-// Offsets into one device allocation, assigned in two passes (size, then place).
-struct Layout {
-  size_t off = 0;
-  size_t take(size_t bytes) {
-    off = align_up(off, 256);
-    size_t r = off;
-    off += bytes;
-    return r;
-  }
-};
-
 }  // namespace
-
-constexpr int kMaxParts = 4;
 
 struct nicp_ctx {
   int device = 0;
@@ -1188,65 +1174,24 @@ extern "C" int nicp_project_intervals(nicp_ctx *ctx, const float *depth, int row
 }
 
 // ------------------------------------------------------------------ pair workspace
-namespace {
-struct PairPlan {
-  int n = 0;
-  size_t o_extra = 0;
-  bool keep_ref = false, list_mode = false;
-  bool structured = false;  // every current cloud has structured Omegas (k_corr_lin<true>)
-  int total_tiles = 0, max_pt_tiles = 0;  // max_pt_tiles: 1024-point tiles of the largest projected cloud
-  int max_tiles = 0;                      // pixel tiles of the largest pair image
-  size_t o_pairs = 0, o_states = 0, o_krt = 0, o_zbuf = 0, zbuf_bytes = 0;
-  size_t o_tile_pair = 0;  // int per pixel tile: its pair
-  std::vector<int> part_pair, part_tile;  // a forked loop's parts: first pair, first tile, and the ends
-  std::vector<size_t> o_cur, o_ref, o_part, o_list, o_ltc, o_np;
-  std::vector<int> P, tiles;
-};
-}  // namespace
-
 // Lays out per-pair buffers; cams[i] gives the projection image of pair i.
 static int plan_pairs(nicp_ctx *ctx, int n, const nicp_camera *cams, const nicp_cloud *const *refs, bool keep_ref,
                       bool list_mode, PairPlan &pl, size_t extra_bytes = 0) {
   pl.n = n;
   pl.keep_ref = keep_ref;
   pl.list_mode = list_mode;
-  Layout L;
-  pl.o_pairs = L.take(sizeof(PairDev) * n);
-  pl.o_states = L.take(sizeof(PairState) * n);
-  pl.o_krt = L.take(48 * (size_t)n);
-  size_t ztot = 0;
   pl.P.resize(n);
-  pl.tiles.resize(n);
+  std::vector<int> capacity(n);
   for (int i = 0; i < n; i++) {
     if (!valid_camera(&cams[i])) return fail(ctx, NICP_EINVAL, "bad camera for pair " + std::to_string(i));
     size_t P = (size_t)cam_rows(cams[i]) * cam_cols(cams[i]);
     if (P > (1u << 30)) return fail(ctx, NICP_EINVAL, "projection image too large");
     pl.P[i] = (int)P;
-    pl.tiles[i] = (int)((P + kCorrTilePixels - 1) / kCorrTilePixels);
-    pl.max_tiles = std::max(pl.max_tiles, pl.tiles[i]);
-    ztot += align_up(8 * P, 256);
+    capacity[i] = refs[i] ? refs[i]->capacity : 0;
   }
-  pl.o_zbuf = L.take(ztot);
-  pl.zbuf_bytes = ztot;
-  pl.o_cur.resize(n); pl.o_ref.resize(n); pl.o_part.resize(n);
-  pl.o_list.resize(n); pl.o_ltc.resize(n); pl.o_np.resize(n);
-  pl.total_tiles = 0;
-  pl.max_pt_tiles = 0;
-  for (int i = 0; i < n; i++) {
-    size_t P = pl.P[i];
-    pl.o_cur[i] = L.take(4 * P);
-    pl.o_ref[i] = (keep_ref || list_mode) ? L.take(4 * P) : 0;
-    pl.o_part[i] = L.take(8 * kPartialWords * (size_t)pl.tiles[i]);
-    pl.o_list[i] = list_mode ? L.take(8 * P) : 0;
-    pl.o_ltc[i] = list_mode ? L.take(4 * (size_t)pl.tiles[i]) : 0;
-    pl.o_np[i] = L.take(4);
-    pl.total_tiles += pl.tiles[i];
-    int cap = std::max(refs[i] ? refs[i]->capacity : 0, 1);
-    pl.max_pt_tiles = std::max(pl.max_pt_tiles, (cap + kPointsPerCta - 1) / kPointsPerCta);
-  }
-  pl.o_tile_pair = L.take(4 * (size_t)std::max(pl.total_tiles, 1));
-  pl.o_extra = L.take(std::max<size_t>(extra_bytes, 1));
-  return ensure_ws(ctx, L.off);
+  const PairSizes sizes = {sizeof(PairDev), sizeof(PairState), 8 * kPartialWords, kCorrTilePixels, kPointsPerCta};
+  lay_out_pairs(pl, sizes, capacity, extra_bytes);
+  return ensure_ws(ctx, pl.bytes);
 }
 
 // Fills the PairDev descriptors in host memory.
@@ -1970,35 +1915,8 @@ struct AlignCall {
 };
 }  // namespace
 
-// Parts of a forked loop.  A launch over all pairs ends with few CTAs at work,
-// and its solve runs on a few SMs; with the pairs in up to kMaxParts parts, each
-// on a branch of the captured graph, one part's launches fill what another's
-// leave free.  One / two / three / four parts, ms: 9 frames of 640x480 0.97 /
-// 0.91 / 0.92 / 0.92, 20 frames 2.06 / 1.92 / 1.92 / 1.91, 200 frames 17.8 / 17.2
-// / 17.2 / 17.2, 20 of 320x240 0.69 / 0.63 / 0.62 / 0.60, 24 mixed pairs 4.01 /
-// 3.87 / 3.77 / 3.78.  Below kPartTiles tiles a part's own launches are too
-// short (two pairs of 300 tiles: 0.487 whole, 0.494 in two).
-constexpr int kPartTiles = 320;
-static void plan_parts(PairPlan &pl) {
-  const int parts = std::min(std::min(kMaxParts, pl.n), pl.total_tiles / kPartTiles);
-  pl.part_pair.assign(1, 0);
-  pl.part_tile.assign(1, 0);
-  int tile = 0;
-  for (int i = 0; i < pl.n; i++) {
-    // a part ends where its share of the tiles is reached
-    const int g = (int)pl.part_pair.size();
-    if (g < parts && i > pl.part_pair.back() && (long long)tile * parts >= (long long)pl.total_tiles * g) {
-      pl.part_pair.push_back(i);
-      pl.part_tile.push_back(tile);
-    }
-    tile += pl.tiles[i];
-  }
-  pl.part_pair.push_back(pl.n);
-  pl.part_tile.push_back(tile);
-}
-
 // Enqueues the whole Gauss-Newton loop for the planned pairs.
-static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, bool fork) {
+static void enqueue_loop(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall &a, bool fork) {
   cudaStream_t s = ctx->stream;
   const PairDev *dpd = (const PairDev *)(ctx->ws + pl.o_pairs);
   CorrParams cp = corr_params(*a.corr);
@@ -2081,22 +1999,16 @@ static void enqueue_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
   launch_publish((const PairState *)(ctx->ws + pl.o_states), a.results, pl.n, !fork || stats, s, &ctx->prof);
 }
 
-static std::string graph_key(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a) {
+// What enqueue_loop bakes into a captured graph: the plan (offsets into ws,
+// grids), the pinned addresses of the input and the results, the options.
+static std::string graph_key(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall &a) {
   std::string k;
   auto put = [&](const void *p, size_t n) { k.append((const char *)p, n); };
   put(&ctx->ws, sizeof(ctx->ws));
-  put(&a.begin, sizeof(a.begin));  // (baked into the graph)
-  put(&a.results, sizeof(a.results));
-  put(&pl.n, sizeof(int));
-  put(&pl.keep_ref, 1);
-  put(&pl.list_mode, 1);
-  put(&pl.structured, 1);
-  put(&pl.total_tiles, sizeof(int));
-  put(&pl.max_pt_tiles, sizeof(int));
-  put(&pl.max_tiles, sizeof(int));
-  put(&pl.zbuf_bytes, sizeof(size_t));
-  put(pl.part_pair.data(), sizeof(int) * pl.part_pair.size());
-  put(pl.part_tile.data(), sizeof(int) * pl.part_tile.size());
+  for (const void *p : {(const void *)a.begin.pairs, (const void *)a.begin.krt, (const void *)a.begin.guess,
+                        (const void *)a.begin.roff, (const void *)a.results})
+    put(&p, sizeof(p));
+  pl.put(k);
   put(a.corr, sizeof(*a.corr));
   put(a.lin, sizeof(*a.lin));
   put(a.prm, sizeof(*a.prm));
