@@ -1436,6 +1436,16 @@ extern "C" int nicp_depth_scale(nicp_ctx *ctx, const void *depth, int is_u16, in
 static int cloud_counts2(nicp_cloud *c, int out[2]);
 
 namespace {
+// The statistics pass linearizes the last iteration's correspondences
+// (Aligner::_computeStatistics).  Without an iteration there are none -- the
+// index images and the list hold whatever the workspace held -- and the system
+// is zero, as the reference's is over an empty list.
+bool statistics_pass(const nicp_align_params &p) { return p.compute_statistics && p.outer_iterations > 0; }
+const double *statistics_system(const nicp_align_params &p, const PairState &st) {
+  static const double none[36] = {};
+  return statistics_pass(p) ? st.Hstat : none;
+}
+
 // Workspace of one NN alignment: the grid over the current cloud, the match
 // and candidate arrays over the reference points, the pair list, FP64
 // partials, the pair descriptor and state.
@@ -1667,7 +1677,7 @@ extern "C" int nicp_align_nn(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cl
                    s, &ctx->prof);
     }
   }
-  if (prm->compute_statistics) {
+  if (statistics_pass(*prm)) {
     launch_lin_list(dpd, 1, pl.tiles, lp, 1, 2, nullptr, true, s, &ctx->prof);
     launch_solve(dpd, 1, 0.0f, 4 | xb, 0.0, 1, s, &ctx->prof);
   }
@@ -1688,7 +1698,7 @@ extern "C" int nicp_align_nn(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cl
   std::memset(out->omega, 0, sizeof(out->omega));
   std::memset(out->mean, 0, sizeof(out->mean));
   if (prm->compute_statistics) {
-    solution_statistics(st.Hstat, st.T, &out->translational_ratio, &out->rotational_ratio, out->omega, out->mean);
+    solution_statistics(statistics_system(*prm, st), st.T, &out->translational_ratio, &out->rotational_ratio, out->omega, out->mean);
     out->solution_valid = !(out->rotational_ratio > prm->rotational_min_eigen_ratio ||
                             out->translational_ratio > prm->translational_min_eigen_ratio);
   }
@@ -1923,7 +1933,7 @@ static void enqueue_loop(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall &a, 
   LinParams lp = lin_params(*a.lin);
   const nicp_align_params &p = *a.prm;
   int outer = p.outer_iterations, inner = p.inner_iterations;
-  bool stats = p.compute_statistics != 0;
+  const bool stats = statistics_pass(p);
   const int xb = a.lin->cross_block_f32 ? kSolveCrossF32 : 0;
   // (list mode's kernels and the general fused kernel are not part of a chain)
   const bool chained = pl.structured && few_tiles(pl.n, pl.max_tiles);
@@ -2231,7 +2241,7 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
     std::memset(r.omega, 0, sizeof(r.omega));
     std::memset(r.mean, 0, sizeof(r.mean));
     if (p.compute_statistics) {
-      solution_statistics(st[i].Hstat, st[i].T, &r.translational_ratio, &r.rotational_ratio, r.omega, r.mean);
+      solution_statistics(statistics_system(p, st[i]), st[i].T, &r.translational_ratio, &r.rotational_ratio, r.omega, r.mean);
       r.solution_valid = !(r.rotational_ratio > p.rotational_min_eigen_ratio ||
                            r.translational_ratio > p.translational_min_eigen_ratio);
     }
