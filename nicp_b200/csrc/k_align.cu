@@ -1617,8 +1617,9 @@ __global__ void __launch_bounds__(256) k_begin_loop(BeginArgs a) {
   for (size_t k = (size_t)blockIdx.x * 256 + t; k < a.zbuf16; k += (size_t)gridDim.x * 256) a.zbuf[k] = ones;
 }
 
-// The pairs' states to the host (pinned memory), chained to the loop's last solve.
-__global__ void __launch_bounds__(256) k_publish(const uint4 *__restrict__ states, uint4 *__restrict__ host, size_t n) {
+// The pairs' states to the host (pinned memory), chained to the loop's last
+// solve, which still writes them when this starts (no __restrict__).
+__global__ void __launch_bounds__(256) k_publish(const uint4 *states, uint4 *host, size_t n) {
   chain();
   for (size_t k = (size_t)blockIdx.x * 256 + threadIdx.x; k < n; k += (size_t)gridDim.x * 256)
     host[k] = __ldcg(states + k);

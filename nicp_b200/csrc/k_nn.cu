@@ -362,10 +362,11 @@ __global__ void __launch_bounds__(kNNThreads) k_nn_far(NNQuery a) {
 
 // (ref, cur) pairs in reference-index order: a CTA adds the hits of the query
 // CTAs before its own, then places its matches by ballots.
-__global__ void __launch_bounds__(kNNBlock) k_nn_pairs(const int *__restrict__ match, int n,
-                                                         const int *__restrict__ block_hits,
-                                                         int32_t *__restrict__ pairs, int *__restrict__ num_pairs,
-                                                         int *far_count, int *__restrict__ next_hits) {
+// (match and block_hits are written by k_nn_far while this chained kernel
+// waits for it: no __restrict__, which would promise the compiler that they
+// do not change and let it load them early, or through the read-only path.)
+__global__ void __launch_bounds__(kNNBlock) k_nn_pairs(const int *match, int n, const int *block_hits, int32_t *pairs,
+                                                       int *num_pairs, int *far_count, int *next_hits) {
   constexpr int kWarps = kNNBlock / 32;
   __shared__ int part[kWarps], hits[kWarps];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
