@@ -2098,6 +2098,14 @@ static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
   return rc;
 }
 
+// The loop reads its input from the pinned upload block.  However a call ends
+// -- a failed launch or an error that an earlier call left behind returns with
+// launches in flight -- the block is not filled again before they are done.
+struct PinUpInUse {
+  nicp_ctx *ctx;
+  ~PinUpInUse() { cudaEventRecord(ctx->pin_up_ev, ctx->stream); }
+};
+
 static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
   if (!ctx || a.n < 0 || !a.cams || !a.corr || !a.lin || !a.prm || (a.n > 0 && (!a.refs || !a.curs || !out)))
     return NICP_EINVAL;
@@ -2135,6 +2143,7 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
   size_t up = sizeof(PairDev) * a.n + 48 * (size_t)a.n + 256 * (size_t)a.n;
   char *pin;
   if ((rc = pin_up(ctx, up, &pin))) return rc;
+  const PinUpInUse in_use{ctx};
   PairDev *pd = (PairDev *)pin;
   fill_pairs(ctx, pl, a.cams, big.data(), a.curs, pd);
   for (int i = 0; i < a.n; i++) {
@@ -2224,7 +2233,6 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
     enqueue_loop(ctx, pl, a, false);
   }
   CK(ctx, cudaGetLastError());
-  CK(ctx, cudaEventRecord(ctx->pin_up_ev, s));  // (the loop reads its input from pinned memory)
   ctx->d2h_bytes += sizeof(PairState) * (unsigned long long)a.n;
   CK(ctx, cudaStreamSynchronize(s));
   const PairState *st = (const PairState *)res;
