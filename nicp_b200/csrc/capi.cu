@@ -1936,7 +1936,7 @@ static void enqueue_loop(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall &a, 
   const bool stats = statistics_pass(p);
   const int xb = a.lin->cross_block_f32 ? kSolveCrossF32 : 0;
   // (list mode's kernels and the general fused kernel are not part of a chain)
-  const bool chained = pl.structured && few_tiles(pl.n, pl.max_tiles);
+  const bool chained = pl.few;
   // After the solve of one or two pairs the projection is chained too: it finds
   // all SMs but those free (two 640x480 pairs 480 -> 472 us, one 1280x720 600 ->
   // 590).  More solves upset the placement of its CTAs (three 640x480 pairs 531
@@ -1958,6 +1958,13 @@ static void enqueue_loop(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall &a, 
   // outside list (parity) mode, current pixels whose point has no normal are
   // dropped from the index image: the gates would reject them anyway
   launch_resolve(dpd, pl.n, pl.max_tiles, 0, nullptr, (pl.list_mode || cp.demoted) ? 0 : 1, chained, s, &ctx->prof);
+  // the fused pass over all pairs
+  auto fused_pass = [&](int flags) {
+    if (pl.few)
+      launch_corr_tile(dpd, pl.n, pl.max_tiles, cp, lp, flags, s, &ctx->prof);
+    else
+      launch_corr_lin(dpd, pl.n, 0, pl.total_tiles, cp, lp, flags, pl.structured, L.corr_ctas, tile_pair, s, &ctx->prof);
+  };
   if (fork) {
     // each part's iterations on a branch of its own
     cudaEventRecord(ctx->fork_ev[0], s);
@@ -1970,7 +1977,7 @@ static void enqueue_loop(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall &a, 
         launch_zbuffer(dpd + p0, n, pl.max_pt_tiles, 1, nullptr, L.zb_ppt, false, q, &ctx->prof);
         for (int k = 0; k < inner; k++) {
           const int flags = (k == 0) ? (1 | 2 | (pl.keep_ref ? 4 : 0)) : 0;
-          launch_corr_lin(dpd, pl.n, t0, tn, pl.max_tiles, cp, lp, flags, true, L.corr_ctas, tile_pair, q, &ctx->prof);
+          launch_corr_lin(dpd, pl.n, t0, tn, cp, lp, flags, true, L.corr_ctas, tile_pair, q, &ctx->prof);
           launch_solve(dpd + p0, n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, q, &ctx->prof);
         }
       }
@@ -1990,8 +1997,7 @@ static void enqueue_loop(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall &a, 
     } else {
       for (int k = 0; k < inner; k++) {
         int flags = (k == 0) ? (1 | 2 | (pl.keep_ref ? 4 : 0)) : 0;
-        launch_corr_lin(dpd, pl.n, 0, pl.total_tiles, pl.max_tiles, cp, lp, flags, pl.structured, L.corr_ctas, tile_pair, s,
-                        &ctx->prof);
+        fused_pass(flags);
         launch_solve(dpd, pl.n, p.lambda, ((k == inner - 1) ? 1 : 0) | xb, p.early_exit_eps, 0, s, &ctx->prof);
       }
     }
@@ -2002,7 +2008,7 @@ static void enqueue_loop(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall &a, 
     if (pl.list_mode)
       launch_lin_list(dpd, pl.n, pl.total_tiles, lp, std::max(1, a.corr->parity_threads), 2, nullptr, false, s, &ctx->prof);
     else
-      launch_corr_lin(dpd, pl.n, 0, pl.total_tiles, pl.max_tiles, cp, lp, 8, pl.structured, L.corr_ctas, tile_pair, s, &ctx->prof);
+      fused_pass(8);
     launch_solve(dpd, pl.n, 0.0f, 4 | xb, 0.0, 1, s, &ctx->prof);
   }
   // (behind the parts' join there is more than one launch to wait for)
@@ -2135,6 +2141,7 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
   if ((rc = plan_pairs(ctx, a.n, a.cams, big.data(), keep_ref, list_mode, pl))) return rc;
   pl.structured = !list_mode;
   for (int i = 0; i < a.n && pl.structured; i++) pl.structured = a.curs[i] && a.curs[i]->omega_structured;
+  pl.few = pl.structured && few_tiles(pl.n, pl.max_tiles);
   plan_parts(pl);
   // the list linearizer reads the current clouds' matrices (the fused kernel
   // rebuilds a structured cloud's Omega itself)

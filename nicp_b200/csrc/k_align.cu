@@ -1740,15 +1740,22 @@ bool few_tiles(int npairs, int max_tiles) {
   return npairs <= 65535 && (long long)max_tiles * npairs <= (long long)kTileCtas * sms;
 }
 
-void launch_corr_lin(const PairDev *d_pairs, int npairs, int first_tile, int total_tiles, int max_tiles,
-                     const CorrParams &cp, const LinParams &lp, int flags, bool structured, int ctas_per_sm, const int *tile_pair, cudaStream_t s,
-                     Profiler *prof) {
+void launch_corr_tile(const PairDev *d_pairs, int npairs, int max_tiles, const CorrParams &cp, const LinParams &lp,
+                      int flags, cudaStream_t s, Profiler *prof) {
+  if (max_tiles <= 0 || npairs <= 0) return;
+  configure_loop();
+  prof->begin(NICP_K_CORR_LIN, s);
+  launch(true, k_corr_tile, dim3(max_tiles, npairs), kTileThreads, sizeof(TileSmem), s, d_pairs, cp, lp, flags);
+  prof->end(NICP_K_CORR_LIN, s);
+}
+
+void launch_corr_lin(const PairDev *d_pairs, int npairs, int first_tile, int total_tiles, const CorrParams &cp,
+                     const LinParams &lp, int flags, bool structured, int ctas_per_sm, const int *tile_pair,
+                     cudaStream_t s, Profiler *prof) {
   if (total_tiles <= 0) return;
   configure_loop();
   prof->begin(NICP_K_CORR_LIN, s);
-  if (structured && few_tiles(npairs, max_tiles)) {
-    launch(true, k_corr_tile, dim3(max_tiles, npairs), kTileThreads, sizeof(TileSmem), s, d_pairs, cp, lp, flags);
-  } else if (structured) {
+  if (structured) {
     // (the reset goes with the first pass)
     const bool plain = !cp.demoted && cp.row_limit_threads <= 1 && !lp.demoted && !lp.z_scaling && lp.robust &&
                        ((flags & 3) == 0 || (flags & 3) == 3);

@@ -155,13 +155,16 @@ void launch_zbuffer(const PairDev *d_pairs, int npairs, int max_pt_tiles, int mo
 void launch_resolve(const PairDev *d_pairs, int npairs, int max_tiles, int to_ref, float *depth_out,
                     int drop_no_normal, bool chained, cudaStream_t s, Profiler *prof);
 // A loop over so few pixel tiles (max_tiles of each of npairs pairs) that one
-// CTA per tile fits on the GPU at once: the fused pass then runs as
-// k_corr_tile and the loop's launches are chained.
+// CTA per tile fits on the GPU at once: if all its current clouds have
+// structured Omegas, the fused pass runs as launch_corr_tile, over all pairs,
+// and the loop's launches are chained.
 bool few_tiles(int npairs, int max_tiles);
+void launch_corr_tile(const PairDev *d_pairs, int npairs, int max_tiles, const CorrParams &cp, const LinParams &lp,
+                      int flags, cudaStream_t s, Profiler *prof);
 // Pixel tiles [first_tile, first_tile + total_tiles) of the npairs pairs' images.
-void launch_corr_lin(const PairDev *d_pairs, int npairs, int first_tile, int total_tiles, int max_tiles,
-                     const CorrParams &cp, const LinParams &lp, int flags, bool structured, int ctas_per_sm, const int *tile_pair, cudaStream_t s,
-                     Profiler *prof);
+void launch_corr_lin(const PairDev *d_pairs, int npairs, int first_tile, int total_tiles, const CorrParams &cp,
+                     const LinParams &lp, int flags, bool structured, int ctas_per_sm, const int *tile_pair,
+                     cudaStream_t s, Profiler *prof);
 void launch_corr_list(const PairDev *d_pairs, int npairs, int total_tiles, const CorrParams &cp, int use_state_T,
                       const float *explicit_T, cudaStream_t s, Profiler *prof);
 void launch_lin_list(const PairDev *d_pairs, int npairs, int total_tiles, const LinParams &lp, int parity_threads,

@@ -33,6 +33,9 @@ struct LoopPlan {
   bool structured = false;  // every current cloud has structured Omegas (k_corr_lin<true>)
   int total_tiles = 0, max_pt_tiles = 0;  // max_pt_tiles: 1024-point tiles of the largest projected cloud
   int max_tiles = 0;                      // pixel tiles of the largest pair image
+  // one CTA per pixel tile of every pair at once (k_corr_tile): the loop's
+  // launches are chained, and cover all pairs -- such a loop has one part
+  bool few = false;
   size_t o_pairs = 0, o_states = 0, o_krt = 0, o_zbuf = 0, zbuf_bytes = 0;
   size_t o_tile_pair = 0;  // int per pixel tile: its pair
   std::vector<int> part_pair, part_tile;  // a forked loop's parts: first pair, first tile, and the ends
@@ -46,6 +49,7 @@ struct LoopPlan {
     one(total_tiles);
     one(max_pt_tiles);
     one(max_tiles);
+    one(few);
     for (size_t o : {o_pairs, o_states, o_krt, o_zbuf, zbuf_bytes, o_tile_pair}) one(o);
     one(part_pair.size());
     for (int v : part_pair) one(v);
@@ -113,7 +117,7 @@ inline void lay_out_pairs(PairPlan &pl, const PairSizes &z, const std::vector<in
 constexpr int kMaxParts = 4;
 constexpr int kPartTiles = 320;
 inline void plan_parts(PairPlan &pl) {
-  const int parts = std::min(std::min(kMaxParts, pl.n), pl.total_tiles / kPartTiles);
+  const int parts = pl.few ? 1 : std::min(std::min(kMaxParts, pl.n), pl.total_tiles / kPartTiles);
   pl.part_pair.assign(1, 0);
   pl.part_tile.assign(1, 0);
   int tile = 0;

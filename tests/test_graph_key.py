@@ -1,8 +1,13 @@
-"""A captured loop is replayed for a call with the same key, so the key has to
+"""What a captured alignment loop is made from (host arithmetic, no GPU).
+
+A captured loop is replayed for a call with the same key, so the key has to
 fix every offset that the loop holds.  Batches whose images differ in a few
 rows or columns can share their count, tiles, parts and z-buffer bytes and
 still lay the tile -> pair table elsewhere: over a neighbourhood of sizes, plans
-with one key have one set of offsets (host arithmetic, no GPU)."""
+with one key have one set of offsets.
+
+A loop whose fused pass is one CTA per tile of all pairs has one part, whatever
+its tiles: the parts would each process all pairs, at the same time."""
 import os
 import subprocess
 
@@ -52,7 +57,13 @@ int main() {
           plans++;
           ambiguous += seen.emplace(key(pl), at).first->second != at;
         }
-  std::printf("%ld %ld\n", plans, ambiguous);
+  // parts of eight pairs of 900 tiles, forked or with one CTA per tile
+  PairPlan few = plan(std::vector<int>(8, 720 * 1280), true);
+  std::printf("%ld %ld %d ", plans, ambiguous, (int)few.part_pair.size() - 1);
+  const std::string forked = key(few);
+  few.few = true;
+  plan_parts(few);
+  std::printf("%d %d\n", (int)few.part_pair.size() - 1, key(few) != forked);
 }
 """
 
@@ -62,7 +73,8 @@ def test_equal_keys_have_equal_offsets(tmp_path):
     src.write_text(PROBE)
     subprocess.run([os.environ.get("NICP_CXX", "g++"), "-std=c++17", "-O1", "-I", os.path.join(ROOT, "nicp_b200", "csrc"),
                     str(src), "-o", str(exe)], check=True, capture_output=True, text=True)
-    same_zbuf, same_tiles, moved, told_apart, plans, ambiguous = map(
+    same_zbuf, same_tiles, moved, told_apart, plans, ambiguous, parts, few_parts, few_told = map(
         int, subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split())
     assert (same_zbuf, same_tiles, moved) == (1, 1, 1)  # the sizes at which the table moves alone
     assert told_apart and plans > 10000 and ambiguous == 0
+    assert parts == 4 and few_parts == 1 and few_told
