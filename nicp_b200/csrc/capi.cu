@@ -201,8 +201,8 @@ static int pin_down(nicp_ctx *ctx, size_t bytes, char **out) {
   return NICP_OK;
 }
 
-// Device -> host copies of a call, complete on return; a few words (counts)
-// take the small pinned buffer.
+// Device -> host copies of a call, complete on return; a few words (counts,
+// small images) take the small pinned buffer.
 constexpr size_t kSmallCopy = 4096;
 static int copy_down(nicp_ctx *ctx, std::initializer_list<HostCopier::Part> parts) {
   size_t total = 0;
@@ -211,6 +211,9 @@ static int copy_down(nicp_ctx *ctx, std::initializer_list<HostCopier::Part> part
     CK(ctx, ctx->copier.down(parts.begin(), (int)parts.size(), ctx->stream));
     return NICP_OK;
   }
+  for (const HostCopier::Part &p : parts)  // (a count is the caller's own variable)
+    if (p.dst && p.bytes > sizeof(int) && HostCopier::kind(p.dst, p.bytes) == HostCopier::kDevice)
+      return fail(ctx, NICP_ECUDA, "the destination of a copy to the host is device memory");
   char *pin;
   int rc = pin_down(ctx, total, &pin);
   if (rc) return rc;

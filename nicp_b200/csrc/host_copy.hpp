@@ -1,5 +1,5 @@
-// host_copy.hpp -- device -> host copies into pageable memory through a
-// context's own pinned slots.
+// host_copy.hpp -- device -> host copies: straight into page-locked memory, into
+// pageable memory through a context's own pinned slots.
 //
 // A copy into pageable memory that is handed to the driver waits for each of
 // its staging transfers, and memory that the caller has just allocated is first
@@ -11,6 +11,10 @@
 // (2.4 MB: 0.92 ms alone, 1.09 shared).  Uploads stay with the driver: through
 // the slots they were no faster from one thread, and slower shared.
 //
+// A page-locked destination takes one transfer and no copy after it: a 640x480
+// projection's two images 213 us through the slots, 90 direct, a whole cloud of
+// that size (32 MB) 2.2 ms through the slots, 0.63 direct.
+//
 // The slots (kSlots x kSlotBytes, allocated on first use) and the workers
 // (started by the first copy of kShareBytes or more) belong to one context,
 // are used by the one host thread that uses the context, and end with it.
@@ -21,6 +25,7 @@
 #include <condition_variable>
 #include <cstring>
 #include <deque>
+#include <initializer_list>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -51,18 +56,51 @@ class HostCopier {
     if (mem_) cudaFreeHost(mem_);
   }
 
+  // What a destination is.  (Both ends are looked up: a buffer of which only a
+  // part is page-locked is pageable.)
+  enum Kind { kPageable, kLocked, kDevice };
+  static Kind kind(const void *dst, size_t bytes) {
+    Kind k = kLocked;
+    for (const char *p : {(const char *)dst, (const char *)dst + (bytes ? bytes - 1 : 0)}) {
+      cudaPointerAttributes at = {};
+      if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return kPageable;
+      }
+      if (at.type == cudaMemoryTypeUnregistered) return kPageable;
+      if (at.type == cudaMemoryTypeDevice) k = kDevice;
+    }
+    return k;
+  }
+
   // Device -> host, complete on return.  The stream's earlier work is waited for.
   struct Part {
     void *dst;
     const void *src;
     size_t bytes;
   };
-  cudaError_t down(const Part *parts, int n, cudaStream_t s) {
-    size_t total = 0;
-    for (int i = 0; i < n; i++) total += parts[i].dst ? parts[i].bytes : 0;
-    if (!total) return cudaStreamSynchronize(s);
-    cudaError_t e = ready();
-    if (e != cudaSuccess) return e;
+  cudaError_t down(const Part *parts, int n, cudaStream_t s) {  // n <= 64
+    size_t total = 0;         // bytes for the slots
+    unsigned long long slow = 0;  // their parts
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < n; i++) {
+      const Part &p = parts[i];
+      if (!p.dst || !p.bytes) continue;
+      const Kind k = kind(p.dst, p.bytes);
+      if (k == kDevice) e = cudaErrorInvalidValue;  // (not host memory: refused)
+      if (k == kLocked && e == cudaSuccess) {
+        // one transfer, no copy after it; where the runtime refuses (a range
+        // that was page-locked in pieces) the slots do it
+        if (cudaMemcpyAsync(p.dst, p.src, p.bytes, cudaMemcpyDeviceToHost, s) == cudaSuccess) continue;
+        cudaGetLastError();
+      }
+      total += p.bytes;
+      slow |= 1ull << i;
+    }
+    if (!total || e != cudaSuccess || (e = ready()) != cudaSuccess) {
+      const cudaError_t err = cudaStreamSynchronize(s);
+      return e != cudaSuccess ? e : err;
+    }
     const bool share = total >= kShareBytes && start();
     std::deque<Piece> flight;  // transfers on their way, in stream order
     auto land = [&] {          // the oldest transfer: wait, then copy out
@@ -77,7 +115,7 @@ class HostCopier {
     };
     int next = 0;
     for (int i = 0; i < n && e == cudaSuccess; i++) {
-      if (!parts[i].dst) continue;
+      if (!((slow >> i) & 1)) continue;
       for (size_t at = 0; at < parts[i].bytes && e == cudaSuccess;) {
         const size_t bytes = std::min(kSlotBytes, parts[i].bytes - at);
         if ((int)flight.size() == kSlots) e = land();

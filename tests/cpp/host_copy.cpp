@@ -1,0 +1,58 @@
+// Drives HostCopier over the stand-in runtime: one scenario per run, "ok" when
+// it holds.
+#include <cstdio>
+#include <memory>
+#include <string>
+
+#include "host_copy.hpp"
+
+using nicp::HostCopier;
+using Bytes = std::vector<char>;
+
+static int failures = 0;
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); failures++; } } while (0)
+
+static Bytes source(size_t n, unsigned seed) {
+  Bytes b(n);
+  for (size_t i = 0; i < n; i++) b[i] = (char)((i * 2654435761u + seed * 97u) >> 13);
+  return b;
+}
+
+// Page-locked destinations are copied into directly, beside pageable ones.
+static void locked() {
+  const size_t big = ((size_t)3 << 20) + 17;
+  const Bytes a = source(big, 1), b = source(big, 2);
+  Bytes da(big), db(big);
+  fake.locked[da.data()] = big;
+  {
+    HostCopier c;
+    const HostCopier::Part one[] = {{da.data(), a.data(), big}};
+    CHECK(c.down(one, 1, nullptr) == cudaSuccess);
+    CHECK(da == a && fake.copies.size() == 1 && fake.copies[0].dst == da.data() && fake.allocated == 0);
+    da.assign(big, 0);
+    const HostCopier::Part two[] = {{db.data(), b.data(), big}, {nullptr, a.data(), 5}, {da.data(), a.data(), big}};
+    CHECK(c.down(two, 3, nullptr) == cudaSuccess);
+    CHECK(da == a && db == b);
+    int direct = 0;
+    for (const Fake::Copy &k : fake.copies) direct += k.dst == da.data();
+    CHECK(direct == 2);
+  }
+  // only the front half page-locked: not taken for a page-locked buffer
+  fake.locked[da.data()] = big / 2;
+  fake.copies.clear();
+  da.assign(big, 0);
+  HostCopier c;
+  const HostCopier::Part one[] = {{da.data(), a.data(), big}};
+  CHECK(c.down(one, 1, nullptr) == cudaSuccess && da == a);
+  for (const Fake::Copy &k : fake.copies) CHECK(k.dst != da.data());
+  fake.locked.erase(da.data());
+}
+
+int main(int, char **argv) {
+  const std::string what = argv[1];
+  if (what == "locked") locked();
+  else CHECK(!"a scenario");
+  CHECK(fake.allocated == fake.freed && fake.events == 0);
+  std::puts(failures ? "failed" : "ok");
+  return failures != 0;
+}
