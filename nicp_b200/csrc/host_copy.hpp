@@ -97,7 +97,14 @@ class HostCopier {
       total += p.bytes;
       slow |= 1ull << i;
     }
-    if (!total || e != cudaSuccess || (e = ready()) != cudaSuccess) {
+    if (total && e == cudaSuccess && ready() != cudaSuccess) {
+      // no page-locked memory for the slots: the driver's own staging
+      cudaGetLastError();
+      for (int i = 0; i < n && e == cudaSuccess; i++)
+        if ((slow >> i) & 1) e = cudaMemcpyAsync(parts[i].dst, parts[i].src, parts[i].bytes, cudaMemcpyDeviceToHost, s);
+      total = 0;
+    }
+    if (!total || e != cudaSuccess) {
       const cudaError_t err = cudaStreamSynchronize(s);
       return e != cudaSuccess ? e : err;
     }

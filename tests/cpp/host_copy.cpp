@@ -48,9 +48,29 @@ static void locked() {
   fake.locked.erase(da.data());
 }
 
+// Without page-locked memory for the slots (or their events) a copy still
+// arrives, and the slots are used once they can be had.
+static void no_slots() {
+  const size_t big = ((size_t)9 << 20) + 5;
+  const Bytes a = source(big, 3);
+  Bytes da(big), db(100);
+  HostCopier c;
+  const HostCopier::Part parts[] = {{da.data(), a.data(), big}, {db.data(), a.data(), 100}};
+  for (int k = 0; k < 4; k++) {
+    fake.lock_fails = k == 0;
+    fake.event_fails = k == 1;
+    da.assign(big, 0);
+    db.assign(100, 0);
+    CHECK(c.down(parts, 2, nullptr) == cudaSuccess && cudaGetLastError() == cudaSuccess);
+    CHECK(da == a && std::equal(db.begin(), db.end(), a.begin()));
+  }
+  CHECK(fake.allocated == 1);
+}
+
 int main(int, char **argv) {
   const std::string what = argv[1];
   if (what == "locked") locked();
+  else if (what == "no_slots") no_slots();
   else CHECK(!"a scenario");
   CHECK(fake.allocated == fake.freed && fake.events == 0);
   std::puts(failures ? "failed" : "ok");
