@@ -24,7 +24,6 @@
 #include <algorithm>
 #include <condition_variable>
 #include <cstring>
-#include <deque>
 #include <initializer_list>
 #include <mutex>
 #include <thread>
@@ -109,10 +108,9 @@ class HostCopier {
       return e != cudaSuccess ? e : err;
     }
     const bool share = total >= kShareBytes && start();
-    std::deque<Piece> flight;  // transfers on their way, in stream order
-    auto land = [&] {          // the oldest transfer: wait, then copy out
-      const Piece p = flight.front();
-      flight.pop_front();
+    Ring<Piece> flight;  // transfers on their way, in stream order
+    auto land = [&] {    // the oldest transfer: wait, then copy out
+      const Piece p = flight.pop();
       const cudaError_t err = cudaEventSynchronize(slots_[p.slot].ev);
       if (err == cudaSuccess) {
         if (share) submit(Job{p.host, slots_[p.slot].p, p.bytes, p.slot});
@@ -125,18 +123,18 @@ class HostCopier {
       if (!((slow >> i) & 1)) continue;
       for (size_t at = 0; at < parts[i].bytes && e == cudaSuccess;) {
         const size_t bytes = std::min(kSlotBytes, parts[i].bytes - at);
-        if ((int)flight.size() == kSlots) e = land();
+        if (flight.size == kSlots) e = land();
         if (e != cudaSuccess) break;
         const int k = next;
         next = (next + 1) % kSlots;
         if (share) wait_job(k);
         e = cudaMemcpyAsync(slots_[k].p, (const char *)parts[i].src + at, bytes, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaEventRecord(slots_[k].ev, s);
-        if (e == cudaSuccess) flight.push_back(Piece{(char *)parts[i].dst + at, bytes, k});
+        if (e == cudaSuccess) flight.push(Piece{(char *)parts[i].dst + at, bytes, k});
         at += bytes;
       }
     }
-    while (!flight.empty()) {
+    while (flight.size) {
       const cudaError_t err = land();
       if (e == cudaSuccess) e = err;
     }
@@ -150,6 +148,21 @@ class HostCopier {
     char *p = nullptr;
     cudaEvent_t ev = nullptr;
     bool job = false;  // a worker copies from it (under m_)
+  };
+  // At most kSlots of anything: a slot has one transfer, then one job.  (Nothing
+  // here allocates once the slots and workers exist, so a copy under way cannot
+  // end in an exception that leaves jobs writing to the caller's memory.)
+  template <class T>
+  struct Ring {
+    T at[kSlots];
+    int first = 0, size = 0;
+    void push(const T &v) { at[(first + size++) % kSlots] = v; }
+    T pop() {
+      const T v = at[first];
+      first = (first + 1) % kSlots;
+      size--;
+      return v;
+    }
   };
   struct Piece {
     char *host;
@@ -181,6 +194,7 @@ class HostCopier {
     if (!workers_.empty()) return true;
     const int n = std::min<int>(kWorkers, (int)std::thread::hardware_concurrency() - 1);
     try {
+      workers_.reserve(std::max(n, 0));
       for (int k = 0; k < n; k++) workers_.emplace_back([this] { work(); });
     } catch (...) {
     }
@@ -189,14 +203,13 @@ class HostCopier {
   void work() {
     std::unique_lock<std::mutex> l(m_);
     for (;;) {
-      work_.wait(l, [&] { return stop_ || !jobs_.empty(); });
-      if (jobs_.empty()) return;
+      work_.wait(l, [&] { return stop_ || jobs_.size; });
+      if (!jobs_.size) return;
       one(l);
     }
   }
   void one(std::unique_lock<std::mutex> &l) {
-    const Job j = jobs_.front();
-    jobs_.pop_front();
+    const Job j = jobs_.pop();
     l.unlock();
     std::memcpy(j.dst, j.src, j.bytes);
     l.lock();
@@ -209,7 +222,7 @@ class HostCopier {
       std::lock_guard<std::mutex> l(m_);
       slots_[j.slot].job = true;
       pending_++;
-      jobs_.push_back(j);
+      jobs_.push(j);
     }
     work_.notify_one();
   }
@@ -217,15 +230,15 @@ class HostCopier {
   void wait_job(int slot) {
     std::unique_lock<std::mutex> l(m_);
     while (slots_[slot].job) {
-      if (!jobs_.empty()) one(l);
-      else done_.wait(l, [&] { return !slots_[slot].job || !jobs_.empty(); });
+      if (jobs_.size) one(l);
+      else done_.wait(l, [&] { return !slots_[slot].job || jobs_.size; });
     }
   }
   void drain() {
     std::unique_lock<std::mutex> l(m_);
     while (pending_) {
-      if (!jobs_.empty()) one(l);
-      else done_.wait(l, [&] { return !pending_ || !jobs_.empty(); });
+      if (jobs_.size) one(l);
+      else done_.wait(l, [&] { return !pending_ || jobs_.size; });
     }
   }
   char *mem_ = nullptr;
@@ -234,7 +247,7 @@ class HostCopier {
   std::vector<std::thread> workers_;
   std::mutex m_;
   std::condition_variable work_, done_;
-  std::deque<Job> jobs_;
+  Ring<Job> jobs_;
   int pending_ = 0;
   bool stop_ = false;
 };

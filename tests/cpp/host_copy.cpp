@@ -1,13 +1,23 @@
 // Drives HostCopier over the stand-in runtime: one scenario per run, "ok" when
 // it holds.
+#include <atomic>
 #include <cstdio>
-#include <memory>
+#include <new>
 #include <string>
 
 #include "host_copy.hpp"
 
 using nicp::HostCopier;
 using Bytes = std::vector<char>;
+
+static std::atomic<bool> no_new{false};
+void *operator new(size_t n) {
+  void *p = no_new ? nullptr : std::malloc(n);
+  if (!p) throw std::bad_alloc();
+  return p;
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 static int failures = 0;
 #define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); failures++; } } while (0)
@@ -48,6 +58,38 @@ static void locked() {
   fake.locked.erase(da.data());
 }
 
+// A copy that has its slots and workers allocates nothing (an exception on the
+// way would leave the workers writing into memory that the caller takes back);
+// a failing transfer is reported, and the copier works on.
+static void no_memory() {
+  const size_t big = ((size_t)40 << 20) + 9;
+  const Bytes a = source(big, 4);
+  Bytes da(big);
+  HostCopier c;
+  const HostCopier::Part one[] = {{da.data(), a.data(), big}};
+  CHECK(c.down(one, 1, nullptr) == cudaSuccess && da == a);
+  fake.copies.clear();
+  fake.copies.reserve(1000);
+  da.assign(big, 0);
+  no_new = true;
+  bool thrown = false;
+  cudaError_t e = cudaSuccess;
+  try {
+    e = c.down(one, 1, nullptr);
+  } catch (const std::bad_alloc &) {
+    thrown = true;
+  }
+  no_new = false;
+  CHECK(!thrown && e == cudaSuccess && da == a);
+  fake.copies.clear();
+  fake.fail_copy = 20;
+  CHECK(c.down(one, 1, nullptr) == cudaErrorInvalidValue);
+  fake.fail_copy = -1;
+  cudaGetLastError();
+  da.assign(big, 0);
+  CHECK(c.down(one, 1, nullptr) == cudaSuccess && da == a);
+}
+
 // Without page-locked memory for the slots (or their events) a copy still
 // arrives, and the slots are used once they can be had.
 static void no_slots() {
@@ -71,6 +113,7 @@ int main(int, char **argv) {
   const std::string what = argv[1];
   if (what == "locked") locked();
   else if (what == "no_slots") no_slots();
+  else if (what == "no_memory") no_memory();
   else CHECK(!"a scenario");
   CHECK(fake.allocated == fake.freed && fake.events == 0);
   std::puts(failures ? "failed" : "ok");

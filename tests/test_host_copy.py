@@ -1,5 +1,6 @@
 """Copies into host memory (host_copy.hpp) over a stand-in for the CUDA runtime,
-no GPU: page-locked destinations, no page-locked memory for the slots."""
+no GPU: page-locked destinations, no page-locked memory for the slots, no
+memory at all."""
 import os
 import subprocess
 
@@ -19,7 +20,7 @@ def program(tmp_path_factory):
     return str(exe)
 
 
-@pytest.mark.parametrize("scenario", ["locked", "no_slots"])
+@pytest.mark.parametrize("scenario", ["locked", "no_slots", "no_memory"])
 def test_host_copier(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
