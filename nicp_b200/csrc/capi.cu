@@ -204,34 +204,39 @@ static int pin_down(nicp_ctx *ctx, size_t bytes, char **out) {
 // Device -> host copies of a call, complete on return; a few words (counts,
 // small images) take the small pinned buffer.
 constexpr size_t kSmallCopy = 4096;
-static int copy_down(nicp_ctx *ctx, std::initializer_list<HostCopier::Part> parts) {
+static int copy_down(nicp_ctx *ctx, const HostCopier::Part *parts, int n) {
   size_t total = 0;
-  for (const HostCopier::Part &p : parts) total += p.dst ? p.bytes : 0;
+  for (int i = 0; i < n; i++) total += parts[i].dst ? parts[i].bytes : 0;
   if (total > kSmallCopy) {
-    CK(ctx, ctx->copier.down(parts.begin(), (int)parts.size(), ctx->stream));
+    CK(ctx, ctx->copier.down(parts, n, ctx->stream));
     return NICP_OK;
   }
-  for (const HostCopier::Part &p : parts)  // (a count is the caller's own variable)
-    if (p.dst && p.bytes > sizeof(int) && HostCopier::kind(p.dst, p.bytes) == HostCopier::kDevice)
+  for (int i = 0; i < n; i++)  // (a count is the caller's own variable)
+    if (parts[i].dst && parts[i].bytes > sizeof(int) &&
+        HostCopier::kind(parts[i].dst, parts[i].bytes) == HostCopier::kDevice)
       return fail(ctx, NICP_ECUDA, "the destination of a copy to the host is device memory");
   char *pin;
   int rc = pin_down(ctx, total, &pin);
   if (rc) return rc;
   size_t at = 0;
-  for (const HostCopier::Part &p : parts)
-    if (p.dst && p.bytes) {
-      CK(ctx, cudaMemcpyAsync(pin + at, p.src, p.bytes, cudaMemcpyDeviceToHost, ctx->stream));
-      at += p.bytes;
+  for (int i = 0; i < n; i++)
+    if (parts[i].dst && parts[i].bytes) {
+      CK(ctx, cudaMemcpyAsync(pin + at, parts[i].src, parts[i].bytes, cudaMemcpyDeviceToHost, ctx->stream));
+      at += parts[i].bytes;
     }
   CK(ctx, cudaStreamSynchronize(ctx->stream));
   at = 0;
-  for (const HostCopier::Part &p : parts)
-    if (p.dst && p.bytes) {
-      std::memcpy(p.dst, pin + at, p.bytes);
-      at += p.bytes;
+  for (int i = 0; i < n; i++)
+    if (parts[i].dst && parts[i].bytes) {
+      std::memcpy(parts[i].dst, pin + at, parts[i].bytes);
+      at += parts[i].bytes;
     }
   return NICP_OK;
 }
+static int copy_down(nicp_ctx *ctx, std::initializer_list<HostCopier::Part> parts) {
+  return copy_down(ctx, parts.begin(), (int)parts.size());
+}
+
 static int cloud_reserve(nicp_cloud *c, int capacity, int rows, int cols, bool eig, bool gauss = false) {
   nicp_ctx *ctx = c->ctx;
   size_t P = (size_t)rows * cols;
@@ -587,21 +592,37 @@ extern "C" int nicp_cloud_download(nicp_cloud *c, float *p4, float *n4, float *c
   if (n == 0) return NICP_OK;
   if ((ev3 || U9) && !c->eig_valid) return fail(ctx, NICP_ESTATE, "cloud was built without keep_stats");
   if ((op9 || on9) && (rc = cloud_ensure_omg(ctx, c))) return rc;
-  // the caller's layout is written on the device
-  const size_t N = (size_t)n;
-  Layout L;
-  CloudExport x{};
-  const size_t o_p = L.take(16 * N), o_n = L.take(16 * N), o_k = L.take(4 * N), o_op = L.take(36 * N),
-               o_on = L.take(36 * N), o_ev = L.take(12 * N), o_u = L.take(36 * N);
-  if ((rc = ensure_ws(ctx, L.off))) return rc;
-  auto place = [&](const void *wanted, size_t off) { return wanted ? (float *)(ctx->ws + off) : nullptr; };
-  x.pts = c->pts; x.nrm = c->nrm; x.omg = c->omg; x.eig = c->eig;
-  x.p4 = place(p4, o_p); x.n4 = place(n4, o_n); x.curv = place(curv, o_k);
-  x.op9 = place(op9, o_op); x.on9 = place(on9, o_on); x.ev3 = place(ev3, o_ev); x.u9 = place(U9, o_u);
-  launch_cloud_export(x, n, ctx->stream);
-  CK(ctx, cudaGetLastError());
-  return copy_down(ctx, {{p4, x.p4, 16 * N}, {n4, x.n4, 16 * N}, {curv, x.curv, 4 * N}, {op9, x.op9, 36 * N},
-                         {on9, x.on9, 36 * N}, {ev3, x.ev3, 12 * N}, {U9, x.u9, 36 * N}});
+  // the caller's layout is written on the device, the outputs asked for and in
+  // pieces that fit the workspace as it is: a download does not make it grow
+  // with the cloud (a context that has built or aligned anything has the room
+  // of a piece already)
+  float *const dst[7] = {p4, n4, curv, op9, on9, ev3, U9};
+  constexpr size_t kWords[7] = {4, 4, 1, 9, 9, 3, 9};
+  size_t words = 0;
+  for (int k = 0; k < 7; k++) words += dst[k] ? kWords[k] : 0;
+  if (!words) return NICP_OK;
+  constexpr size_t kPieceFloor = (size_t)16 << 20, kPad = 7 * 256;  // (Layout's alignment of seven arrays)
+  const size_t room = std::min(std::max(ctx->ws_cap, kPieceFloor), 4 * words * n + kPad);
+  if ((rc = ensure_ws(ctx, room))) return rc;
+  const int piece = (int)std::min<size_t>(n, (room - kPad) / (4 * words));
+  for (int i0 = 0; i0 < n; i0 += piece) {
+    const size_t N = (size_t)std::min(piece, n - i0);
+    Layout L;
+    float *ws[7];
+    HostCopier::Part part[7];
+    for (int k = 0; k < 7; k++) {
+      const size_t bytes = 4 * kWords[k] * N;
+      ws[k] = dst[k] ? (float *)(ctx->ws + L.take(bytes)) : nullptr;
+      part[k] = {dst[k] ? dst[k] + kWords[k] * i0 : nullptr, ws[k], bytes};
+    }
+    const CloudExport x = {c->pts + i0, c->nrm + i0, c->omg + 3 * (size_t)i0,
+                           c->eig ? c->eig + kStatsWords * (size_t)i0 : nullptr,
+                           ws[0], ws[1], ws[2], ws[3], ws[4], ws[5], ws[6]};
+    launch_cloud_export(x, (int)N, ctx->stream);
+    CK(ctx, cudaGetLastError());
+    if ((rc = copy_down(ctx, part, 7))) return rc;
+  }
+  return NICP_OK;
   NICP_ABI_CATCH
 }
 
