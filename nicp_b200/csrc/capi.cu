@@ -20,6 +20,7 @@
 #include "kernels.hpp"
 #include "nicp_gpu.h"
 #include "pair_plan.hpp"
+#include "pinned_block.hpp"
 
 using namespace nicp;
 
@@ -44,16 +45,14 @@ struct nicp_ctx {
   Profiler prof;
   char *ws = nullptr;
   size_t ws_cap = 0;
-  char *pin_up = nullptr;
-  size_t pin_up_cap = 0;
+  PinnedBlock pin_up;
   cudaEvent_t pin_up_ev = nullptr;
   cudaStream_t copy_stream = nullptr;   // depth staging copies, overlapped with the build kernels
   std::vector<cudaEvent_t> copy_ev;     // one per build chunk: its frames are staged
   cudaEvent_t copy_start = nullptr;     // the compute stream's tail when staging begins
   cudaStream_t fork_stream[kMaxParts - 1] = {};  // the other branches of a captured, forked loop
   cudaEvent_t fork_ev[kMaxParts] = {};
-  char *pin_down = nullptr;
-  size_t pin_down_cap = 0;
+  PinnedBlock pin_down;
   HostCopier copier;                    // copies into pageable host memory
   size_t cloud_bytes = 0;
   std::vector<GraphEntry> graphs;
@@ -174,31 +173,25 @@ static int ensure_ws(nicp_ctx *ctx, size_t bytes) {
   return NICP_OK;
 }
 
-// Pinned upload staging: waits until the previous upload has been consumed.
-static int pin_up(nicp_ctx *ctx, size_t bytes, char **out) {
-  CK(ctx, cudaEventSynchronize(ctx->pin_up_ev));
-  if (bytes > ctx->pin_up_cap) {
-    if (ctx->pin_up) cudaFreeHost(ctx->pin_up);
-    ctx->pin_up = nullptr;
-    size_t cap = align_up(bytes + bytes / 4, 1 << 16);
-    CK(ctx, cudaMallocHost(&ctx->pin_up, cap));
-    ctx->pin_up_cap = cap;
+static int pin_reserve(nicp_ctx *ctx, PinnedBlock &block, size_t bytes, char **out) {
+  const cudaError_t e = block.reserve(bytes);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // (reported here, not by the next launch that is checked)
+    return fail(ctx, NICP_ECUDA, std::string("page-locked staging: ") + cudaGetErrorString(e));
   }
-  *out = ctx->pin_up;
+  *out = block.p;
   return NICP_OK;
 }
 
+// Pinned upload staging: waits until the previous upload has been consumed.
+static int pin_up(nicp_ctx *ctx, size_t bytes, char **out) {
+  CK(ctx, cudaEventSynchronize(ctx->pin_up_ev));
+  return pin_reserve(ctx, ctx->pin_up, bytes, out);
+}
+
 static int pin_down(nicp_ctx *ctx, size_t bytes, char **out) {
-  if (bytes > ctx->pin_down_cap) {
-    CK(ctx, cudaStreamSynchronize(ctx->stream));
-    if (ctx->pin_down) cudaFreeHost(ctx->pin_down);
-    ctx->pin_down = nullptr;
-    size_t cap = align_up(bytes + bytes / 4, 1 << 16);
-    CK(ctx, cudaMallocHost(&ctx->pin_down, cap));
-    ctx->pin_down_cap = cap;
-  }
-  *out = ctx->pin_down;
-  return NICP_OK;
+  if (bytes > ctx->pin_down.cap) CK(ctx, cudaStreamSynchronize(ctx->stream));
+  return pin_reserve(ctx, ctx->pin_down, bytes, out);
 }
 
 // Device -> host copies of a call, complete on return; a few words (counts,
@@ -424,8 +417,8 @@ extern "C" int nicp_ctx_destroy(nicp_ctx *ctx) {
   if (ctx->scratch_cloud) nicp_cloud_destroy(ctx->scratch_cloud);
   for (auto &g : ctx->graphs) cudaGraphExecDestroy(g.exec);
   if (ctx->ws) cudaFree(ctx->ws);
-  if (ctx->pin_up) cudaFreeHost(ctx->pin_up);
-  if (ctx->pin_down) cudaFreeHost(ctx->pin_down);
+  ctx->pin_up.release();
+  ctx->pin_down.release();
   cudaEventDestroy(ctx->pin_up_ev);
   for (cudaEvent_t e : ctx->copy_ev) cudaEventDestroy(e);
   if (ctx->copy_start) cudaEventDestroy(ctx->copy_start);
