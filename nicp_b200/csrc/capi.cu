@@ -156,11 +156,15 @@ static int cloud_ensure_omg(nicp_ctx *ctx, const nicp_cloud *c) {
   return NICP_OK;
 }
 
+static void drop_graphs(nicp_ctx *ctx) {
+  for (auto &g : ctx->graphs) cudaGraphExecDestroy(g.exec);
+  ctx->graphs.clear();
+}
+
 static int ensure_ws(nicp_ctx *ctx, size_t bytes) {
   if (bytes <= ctx->ws_cap) return NICP_OK;
   CK(ctx, cudaStreamSynchronize(ctx->stream));
-  for (auto &g : ctx->graphs) cudaGraphExecDestroy(g.exec);
-  ctx->graphs.clear();
+  drop_graphs(ctx);
   if (ctx->ws) cudaFree(ctx->ws);
   ctx->ws = nullptr;
   ctx->ws_cap = 0;
@@ -174,6 +178,11 @@ static int ensure_ws(nicp_ctx *ctx, size_t bytes) {
 }
 
 static int pin_reserve(nicp_ctx *ctx, PinnedBlock &block, size_t bytes, char **out) {
+  if (bytes > block.cap && !ctx->graphs.empty()) {
+    // (captured loops hold the address of the block that goes)
+    CK(ctx, cudaStreamSynchronize(ctx->stream));
+    drop_graphs(ctx);
+  }
   const cudaError_t e = block.reserve(bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();  // (reported here, not by the next launch that is checked)
@@ -415,7 +424,7 @@ extern "C" int nicp_ctx_destroy(nicp_ctx *ctx) {
   cudaStreamSynchronize(ctx->stream);
   if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);  // staging copies write into ws
   if (ctx->scratch_cloud) nicp_cloud_destroy(ctx->scratch_cloud);
-  for (auto &g : ctx->graphs) cudaGraphExecDestroy(g.exec);
+  drop_graphs(ctx);
   if (ctx->ws) cudaFree(ctx->ws);
   ctx->pin_up.release();
   ctx->pin_down.release();

@@ -8,6 +8,10 @@
 namespace nicp {
 
 struct PinnedBlock {
+  // Captured loops hold the block's address, so each move costs them: the first
+  // block has room for loops of 700 pairs and builds of a thousand frames of
+  // 640x480, and from there a larger one is at least twice as large.
+  static constexpr size_t kFirst = (size_t)1 << 20;
   char *p = nullptr;
   size_t cap = 0;
   // Room for `bytes`.  The old block is freed where it is too small: whoever
@@ -15,8 +19,9 @@ struct PinnedBlock {
   // tries again.
   cudaError_t reserve(size_t bytes) {
     if (bytes <= cap) return cudaSuccess;
+    size_t want = cap ? cap : kFirst / 2;
+    while (want *= 2, want < bytes) {}
     release();
-    const size_t want = (bytes + bytes / 4 + 0xffff) & ~(size_t)0xffff;
     const cudaError_t e = cudaMallocHost(&p, want);
     if (e != cudaSuccess) {
       p = nullptr;
