@@ -1075,10 +1075,10 @@ static int build_frames(nicp_ctx *ctx, int n, const FrameIn *fin, const nicp_cam
                         prm->nim_nonflat[1] == prm->nim_nonflat[2];
       int shape = stats_default_shape(lean);
       if (ctx->autotune) {
-        // the chunk's frame sizes and the moment precision select the shape
+        // the chunk's frame sizes, the moment precision and the kernel's form select the shape
         std::map<std::pair<int, int>, int> hist;
         for (int i = i0; i < i0 + nf; i++) hist[{fin[i].rows, fin[i].cols}]++;
-        std::string key = std::to_string(prm->moments_precision) + ":";
+        std::string key = std::to_string(prm->moments_precision) + (lean ? "lean:" : "full:");
         for (auto &h : hist)
           key += std::to_string(h.first.first) + "x" + std::to_string(h.first.second) + "*" +
                  std::to_string(h.second) + " ";
