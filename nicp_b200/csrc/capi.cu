@@ -2062,14 +2062,14 @@ static std::string graph_key(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall 
 
 // The resolution mix of a batch: sorted (rows, cols, count) plus the loop
 // shape; the autotuner keeps one choice per key.
-static std::string tune_key(const PairPlan &pl, const AlignCall &a) {
+static std::string tune_key(const PairPlan &pl, const AlignCall &a, bool fork) {
   std::map<std::pair<int, int>, int> hist;
   for (int i = 0; i < a.n; i++) hist[{cam_rows(a.cams[i]), cam_cols(a.cams[i])}]++;
   std::string k;
   for (auto &h : hist) k += std::to_string(h.first.first) + "x" + std::to_string(h.first.second) + ":" +
                            std::to_string(h.second) + " ";
   k += "o" + std::to_string(a.prm->outer_iterations) + "i" + std::to_string(a.prm->inner_iterations) +
-       (pl.structured ? "s" : "g") + (a.prm->compute_statistics ? "t" : "");
+       (pl.structured ? "s" : "g") + (a.prm->compute_statistics ? "t" : "") + (fork ? "f" : "");
   return k;
 }
 
@@ -2077,17 +2077,33 @@ static std::string tune_key(const PairPlan &pl, const AlignCall &a) {
 // projection grid spans about two waves of its 128-thread CTAs (16 per SM),
 // more independent loads and atomics per thread pay (the 199-pair 640x480
 // sequence: 8 points per thread, 3 % faster than 4); below that (one or a
-// few pairs) more threads do.
+// few pairs) more threads do.  A forked loop launches a part of the pairs at a
+// time, but its parts share the GPU, and the line lies at all their CTAs as
+// well (4 / 8 points per thread, forked, us: 1425 CTAs of 320x240 354 / 378,
+// 1500 of 640x480 396 / 412, 2400 of 640x480 574 / 547, 2925 of 320x240 658 /
+// 635, 3600 of 1280x720 820 / 799).
 static int default_zb_ppt(const nicp_ctx *ctx, const PairPlan &pl) {
   const long long ctas = (long long)pl.max_pt_tiles * pl.n;
   return ctas >= 16ll * ctx->sm_count ? kZbufWidePPT : kZbufDefaultPPT;
 }
 
+// The streams and events of a forked loop.
+static int fork_ready(nicp_ctx *ctx) {
+  for (int k = 0; k < kMaxParts; k++) {
+    if (!ctx->fork_ev[k]) CK(ctx, cudaEventCreateWithFlags(&ctx->fork_ev[k], cudaEventDisableTiming));
+    if (k && !ctx->fork_stream[k - 1])
+      CK(ctx, cudaStreamCreateWithFlags(&ctx->fork_stream[k - 1], cudaStreamNonBlocking));
+  }
+  return NICP_OK;
+}
+
 // Times the loop with each candidate launch shape (direct launches, CUDA
 // events on the context stream) and keeps the fastest: z-buffer points per
-// thread first, then the fused kernel's CTAs per SM.  The loop re-initialises
-// every pair from its guess, so trials leave no trace in the results.
-static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, nicp_ctx::Launch *best) {
+// thread first, then the fused kernel's CTAs per SM.  The trials run in the
+// form -- forked or not -- in which the loop then runs.  The loop
+// re-initialises every pair from its guess, so trials leave no trace in the
+// results.
+static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, bool fork, nicp_ctx::Launch *best) {
   cudaStream_t s = ctx->stream;
   cudaEvent_t e0, e1;
   CK(ctx, cudaEventCreate(&e0));
@@ -2098,7 +2114,7 @@ static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
   auto trial = [&](const nicp_ctx::Launch &c, float *ms) -> int {
     ctx->launch = c;
     CK(ctx, cudaEventRecord(e0, s));
-    enqueue_loop(ctx, pl, a, false);
+    enqueue_loop(ctx, pl, a, fork);
     CK(ctx, cudaEventRecord(e1, s));
     CK(ctx, cudaEventSynchronize(e1));
     CK(ctx, cudaEventElapsedTime(ms, e0, e1));
@@ -2126,7 +2142,7 @@ static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
   ctx->prof.enabled = prof;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  ctx->tune_ms[tune_key(pl, a)] = times;
+  ctx->tune_ms[tune_key(pl, a, fork)] = times;
   return rc;
 }
 
@@ -2209,20 +2225,23 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
   ctx->h2d_bytes += (sizeof(PairDev) + 48 + 256) * (unsigned long long)a.n;
   ctx->launch = nicp_ctx::Launch();
   ctx->launch.zb_ppt = default_zb_ppt(ctx, pl);
+  // Events recorded while a stream is captured are capture-internal and
+  // cannot be timed after a replay, so a profiled call launches the same
+  // kernels directly, in one chain (a server's too).
+  const bool replay = a.graph && !ctx->prof.enabled;
+  const bool fork = replay && pl.structured && pl.part_pair.size() > 2;
+  if (fork && (rc = fork_ready(ctx))) return rc;
   if (ctx->autotune && !list_mode) {
-    std::string tk = tune_key(pl, a);
+    std::string tk = tune_key(pl, a, fork);
     auto it = ctx->tuned.find(tk);
     if (it == ctx->tuned.end()) {
       nicp_ctx::Launch best;
-      if ((rc = autotune_loop(ctx, pl, a, &best))) return rc;
+      if ((rc = autotune_loop(ctx, pl, a, fork, &best))) return rc;
       it = ctx->tuned.emplace(tk, best).first;
     }
     ctx->launch = it->second;
   }
-  // Events recorded while a stream is captured are capture-internal and
-  // cannot be timed after a replay, so a profiled call launches the same
-  // kernels directly.
-  if (a.graph && !ctx->prof.enabled) {
+  if (replay) {
     std::string key = graph_key(ctx, pl, a);
     GraphEntry *ge = nullptr;
     for (auto &g : ctx->graphs)
@@ -2233,12 +2252,6 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
       size_t rec0 = ctx->prof.recs.size();
       unsigned long long l0 = ctx->prof.launches;
       cudaGraph_t graph;
-      const bool fork = pl.structured && pl.part_pair.size() > 2;
-      for (int k = 0; fork && k < kMaxParts; k++) {
-        if (!ctx->fork_ev[k]) CK(ctx, cudaEventCreateWithFlags(&ctx->fork_ev[k], cudaEventDisableTiming));
-        if (k && !ctx->fork_stream[k - 1])
-          CK(ctx, cudaStreamCreateWithFlags(&ctx->fork_stream[k - 1], cudaStreamNonBlocking));
-      }
       CK(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
       ctx->prof.capturing = true;
       enqueue_loop(ctx, pl, a, fork);
