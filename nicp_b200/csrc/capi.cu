@@ -71,7 +71,6 @@ struct nicp_ctx {
   // and the shape of the last build
   std::map<std::string, int> stats_tuned;
   int stats_shape = 0;
-  std::map<std::string, std::vector<float>> tune_ms;  // trial times per resolution mix
 };
 
 struct nicp_cloud {
@@ -2110,7 +2109,6 @@ static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
   CK(ctx, cudaEventCreate(&e1));
   bool prof = ctx->prof.enabled;
   ctx->prof.enabled = false;
-  std::vector<float> times;
   auto trial = [&](const nicp_ctx::Launch &c, float *ms) -> int {
     ctx->launch = c;
     CK(ctx, cudaEventRecord(e0, s));
@@ -2118,7 +2116,6 @@ static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
     CK(ctx, cudaEventRecord(e1, s));
     CK(ctx, cudaEventSynchronize(e1));
     CK(ctx, cudaEventElapsedTime(ms, e0, e1));
-    times.push_back(*ms);
     return NICP_OK;
   };
   const nicp_ctx::Launch cur = ctx->launch;  // the default shape for this call
@@ -2142,7 +2139,6 @@ static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
   ctx->prof.enabled = prof;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  ctx->tune_ms[tune_key(pl, a, fork)] = times;
   return rc;
 }
 

@@ -26,7 +26,6 @@ namespace nicp {
 constexpr int kCorrTilePixels = 1024;   // pixels per CTA in the pair-image kernels
 constexpr int kCorrThreads = 256;       // 4 pixels per thread
 constexpr int kUnprojTilePixels = 4096; // 16 pixels per thread, 256 threads
-constexpr int kStatsThreads = 256;
 constexpr int kPartialWords = 32;       // doubles per CTA partial (21 H + 6 b + chi2 + inliers + C + K + pad)
 constexpr int kSolveCrossF32 = 32;      // k_solve mode bit: FP32 sum of the tile partials
 constexpr int kPointsPerCta = 1024;     // z-buffer kernel tile (points per CTA; threads = 1024 / points per thread)

@@ -32,19 +32,6 @@ struct HM4 {
   }
 };
 
-inline HM4 hm_mul(const HM4 &A, const HM4 &B) {
-  HM4 C;
-  for (int i = 0; i < 4; i++)
-    for (int j = 0; j < 4; j++) {
-      float s = A(i, 0) * B(0, j);
-      s = s + A(i, 1) * B(1, j);
-      s = s + A(i, 2) * B(2, j);
-      s = s + A(i, 3) * B(3, j);
-      C(i, j) = s;
-    }
-  return C;
-}
-
 inline HM4 hm_iso_inverse(const HM4 &T) {
   HM4 r = HM4::identity();
   for (int i = 0; i < 3; i++)

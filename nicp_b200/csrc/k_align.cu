@@ -630,10 +630,10 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
   Stage *stages = reinterpret_cast<Stage *>(corr_smem_raw);
   const int t = threadIdx.x;
   // per-tile constants for the two tiles the pipeline can span:
-  // [0..11] gating T, [12..23] linearizer T, [24..31] the current cloud's
-  // Omega parameters, then pair index, skip flag and structured-Omega flag
-  __shared__ float sT[kConstSlots][32];
-  __shared__ float4 sW[kConstSlots][kWeightEntries];  // structured: weights by point code
+  // [0..11] gating T, [12..23] linearizer T, the Omega weights by point code,
+  // then pair index, skip flag and structured-Omega flag
+  __shared__ float sT[kConstSlots][24];
+  __shared__ float4 sW[kConstSlots][kWeightEntries];
   __shared__ int sPair[kConstSlots], sSkip[kConstSlots], sStruct[kConstSlots], sSame[kConstSlots];
   const bool stats_pass = flags & 8;
   chain_next();  // the solve's CTAs
@@ -766,9 +766,7 @@ __global__ void __launch_bounds__(kFusedThreads, kStructured ? NICP_CORR_S_CTAS 
     if (threadIdx.x < 24)
       sT[e][threadIdx.x] = threadIdx.x < 12 ? (stats_pass ? st->Tgate_used : st->Tgate)[threadIdx.x]
                                             : st->Tlin[threadIdx.x - 12];
-    else if (threadIdx.x < 32)
-      sT[e][threadIdx.x] = pairs[pi].cur_omd[threadIdx.x - 24];
-    else if (threadIdx.x < 32 + kWeightEntries)
+    else if (threadIdx.x >= 32 && threadIdx.x < 32 + kWeightEntries)
       sW[e][threadIdx.x - 32] = table_weights(lp, pairs[pi].cur_omd, threadIdx.x - 32);
     if (threadIdx.x == 0) {
       sPair[e] = pi;
@@ -1578,7 +1576,6 @@ __global__ void __launch_bounds__(kSumThreads) k_solve(const PairDev *__restrict
 __global__ void __launch_bounds__(256) k_begin_loop(BeginArgs a) {
   __shared__ SolveScratch sc;
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  chain_next();
   for (int pi = blockIdx.x; pi < a.npairs; pi += gridDim.x) {
     const PairDev &src = a.pairs[pi];
     if (wid == 0) {

@@ -272,11 +272,6 @@ __global__ void __launch_bounds__(256) k_unproject_write(const FrameDev *__restr
 // kernel reads a corner's ten sums with five paired loads and the sweep
 // writes them with five paired stores.
 struct MomF64 {
-  typedef double T;
-  __device__ static double val(double v) { return v; }
-  __device__ static void store(void *base, size_t P, int m, size_t i, double v) {
-    static_cast<double *>(base)[2 * ((size_t)(m >> 1) * P + i) + (m & 1)] = v;
-  }
   __device__ static void store2(void *base, size_t P, int k, size_t i, double a, double b) {
     static_cast<double2 *>(base)[(size_t)k * P + i] = make_double2(a, b);
   }
@@ -287,11 +282,6 @@ struct MomF64 {
   }
 };
 struct MomF32 {
-  typedef float T;
-  __device__ static double val(float v) { return (double)v; }
-  __device__ static void store(void *base, size_t P, int m, size_t i, double v) {
-    static_cast<float *>(base)[2 * ((size_t)(m >> 1) * P + i) + (m & 1)] = (float)v;
-  }
   __device__ static void store2(void *base, size_t P, int k, size_t i, double a, double b) {
     static_cast<float2 *>(base)[(size_t)k * P + i] = make_float2((float)a, (float)b);
   }
@@ -304,14 +294,9 @@ struct MomF32 {
 // Two-float: an unevaluated sum hi + lo of two floats (about 48 significant
 // bits); values travel as double inside the kernels and are split on store.
 struct MomTwoFloat {
-  typedef float2 T;
-  __device__ static double val(float2 v) { return (double)v.x + (double)v.y; }
   __device__ static float2 split(double v) {
     const float hi = (float)v;
     return make_float2(hi, (float)(v - (double)hi));
-  }
-  __device__ static void store(void *base, size_t P, int m, size_t i, double v) {
-    static_cast<float2 *>(base)[2 * ((size_t)(m >> 1) * P + i) + (m & 1)] = split(v);
   }
   __device__ static void store2(void *base, size_t P, int k, size_t i, double a, double b) {
     const float2 x = split(a), y = split(b);
