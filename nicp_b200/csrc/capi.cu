@@ -844,66 +844,78 @@ static int build_frames(nicp_ctx *ctx, int n, const FrameIn *fin, const nicp_cam
     any_host |= !f.on_device;
     any_staged |= staged[i] != 0;
   }
-  std::vector<std::pair<int, int>> chunks;
-  for (int i0 = 0; i0 < n;) {
-    // with host frames the first chunk is short, so the kernels start after
-    // a few frames' copies
-    // (frames per launch are the grids' y dimension: at most 65535)
-    const int max_frames = std::min(65535, !any_host ? n : stream_chunk(i0, i0 == 0));
-    int i1 = i0;
-    size_t mom = 0;
-    while (i1 < n && i1 - i0 < max_frames) {
-      size_t m = (size_t)fin[i1].rows * fin[i1].cols * 10 * msz;
-      if (i1 > i0 && mom + m > kChunkMoments) break;
-      mom += m;
-      i1++;
-    }
-    chunks.push_back({i0, i1});
-    i0 = i1;
-  }
-  // one layout for the call: staging region, descriptors, then the scratch
-  // of the largest chunk (reused chunk after chunk, in stream order)
   const int nb_rows = moment_band_rows();
-  Layout L;
-  std::vector<size_t> o_stage(n, 0);
-  for (int i = 0; i < n; i++)
-    if (staged[i]) o_stage[i] = L.take((size_t)fin[i].rows * fin[i].cols * (fin[i].u16 ? 2 : 4)) + 1;  // +1: "staged"
-  // descriptors of every frame, then per chunk the frame of each CTA of the
-  // 1-D build grids: unprojection tiles, 16-row bands, band-carry CTAs
-  std::vector<size_t> tab_off(chunks.size() + 1, 0);
-  std::vector<int> tab_tiles(chunks.size(), 0), tab_bands(chunks.size(), 0);
-  for (size_t ci = 0; ci < chunks.size(); ci++) {
-    size_t t = 0, b = 0, k = 0;
-    for (int i = chunks[ci].first; i < chunks[ci].second; i++) {
-      const size_t P = (size_t)fin[i].rows * fin[i].cols;
-      t += (P + kUnprojTilePixels - 1) / kUnprojTilePixels;
-      b += (fin[i].rows + nb_rows - 1) / nb_rows;
-      k += (10 * (size_t)fin[i].cols + 127) / 128;
-    }
-    tab_tiles[ci] = (int)t;
-    tab_bands[ci] = (int)b;
-    tab_off[ci + 1] = tab_off[ci] + t + b + k;
-  }
-  const size_t frames_bytes = sizeof(FrameDev) * n + 4 * tab_off[chunks.size()];
-  const size_t o_frames_all = L.take(frames_bytes);
-  const size_t scratch0 = L.off;
-  size_t scratch_max = scratch0;
-  for (auto &c : chunks) {
-    Layout C;
-    C.off = scratch0;
-    const bool rowpath = moments_row_path(c.second - c.first);
-    for (int i = c.first; i < c.second; i++) {
-      const size_t P = (size_t)fin[i].rows * fin[i].cols;
-      C.take(4 * ((P + kUnprojTilePixels - 1) / kUnprojTilePixels));
-      if (!unproject_only) {
-        C.take(P * 10 * msz);
-        C.take((size_t)((fin[i].rows + nb_rows - 1) / nb_rows) * 10 * fin[i].cols * msz);
-        if (rowpath) C.take(P * 10 * moment_acc_bytes(prm->moments_precision));
+  std::vector<std::pair<int, int>> chunks;
+  std::vector<size_t> o_stage, tab_off;
+  std::vector<int> tab_tiles, tab_bands;
+  size_t frames_bytes = 0, o_frames_all = 0, scratch0 = 0, scratch_max = 0, largest = 0;
+  auto plan = [&](size_t chunk_moments) {
+    chunks.clear();
+    largest = 0;
+    for (int i0 = 0; i0 < n;) {
+      // with host frames the first chunk is short, so the kernels start after
+      // a few frames' copies
+      // (frames per launch are the grids' y dimension: at most 65535)
+      const int max_frames = std::min(65535, !any_host ? n : stream_chunk(i0, i0 == 0));
+      int i1 = i0;
+      size_t mom = 0;
+      while (i1 < n && i1 - i0 < max_frames) {
+        size_t m = (size_t)fin[i1].rows * fin[i1].cols * 10 * msz;
+        if (i1 > i0 && mom + m > chunk_moments) break;
+        mom += m;
+        i1++;
       }
+      largest = std::max(largest, mom);
+      chunks.push_back({i0, i1});
+      i0 = i1;
     }
-    scratch_max = std::max(scratch_max, C.off);
-  }
-  if ((rc = ensure_ws(ctx, scratch_max))) return rc;
+    // one layout for the call: staging region, descriptors, then the scratch
+    // of the largest chunk (reused chunk after chunk, in stream order)
+    Layout L;
+    o_stage.assign(n, 0);
+    for (int i = 0; i < n; i++)
+      if (staged[i]) o_stage[i] = L.take((size_t)fin[i].rows * fin[i].cols * (fin[i].u16 ? 2 : 4)) + 1;  // +1: "staged"
+    // descriptors of every frame, then per chunk the frame of each CTA of the
+    // 1-D build grids: unprojection tiles, 16-row bands, band-carry CTAs
+    tab_off.assign(chunks.size() + 1, 0);
+    tab_tiles.assign(chunks.size(), 0);
+    tab_bands.assign(chunks.size(), 0);
+    for (size_t ci = 0; ci < chunks.size(); ci++) {
+      size_t t = 0, b = 0, k = 0;
+      for (int i = chunks[ci].first; i < chunks[ci].second; i++) {
+        const size_t P = (size_t)fin[i].rows * fin[i].cols;
+        t += (P + kUnprojTilePixels - 1) / kUnprojTilePixels;
+        b += (fin[i].rows + nb_rows - 1) / nb_rows;
+        k += (10 * (size_t)fin[i].cols + 127) / 128;
+      }
+      tab_tiles[ci] = (int)t;
+      tab_bands[ci] = (int)b;
+      tab_off[ci + 1] = tab_off[ci] + t + b + k;
+    }
+    frames_bytes = sizeof(FrameDev) * n + 4 * tab_off[chunks.size()];
+    o_frames_all = L.take(frames_bytes);
+    scratch0 = scratch_max = L.off;
+    for (auto &c : chunks) {
+      Layout C;
+      C.off = scratch0;
+      const bool rowpath = moments_row_path(c.second - c.first);
+      for (int i = c.first; i < c.second; i++) {
+        const size_t P = (size_t)fin[i].rows * fin[i].cols;
+        C.take(4 * ((P + kUnprojTilePixels - 1) / kUnprojTilePixels));
+        if (!unproject_only) {
+          C.take(P * 10 * msz);
+          C.take((size_t)((fin[i].rows + nb_rows - 1) / nb_rows) * 10 * fin[i].cols * msz);
+          if (rowpath) C.take(P * 10 * moment_acc_bytes(prm->moments_precision));
+        }
+      }
+      scratch_max = std::max(scratch_max, C.off);
+    }
+  };
+  // (where the scratch of the largest chunk cannot be had, smaller chunks do)
+  size_t limit = kChunkMoments;
+  for (plan(limit); (rc = ensure_ws(ctx, scratch_max)) == NICP_ENOMEM && (int)chunks.size() < n;)
+    plan(limit = std::min(limit, largest) / 2);
+  if (rc) return rc;
   char *pin;
   if ((rc = pin_up(ctx, frames_bytes, &pin))) return rc;
   int *tab_all = reinterpret_cast<int *>(pin + sizeof(FrameDev) * n);

@@ -1,0 +1,40 @@
+"""A build of many host frames on a GPU that is nearly full: the chunks shrink
+to the scratch that can be had, and the clouds are the same."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import converter
+from nicp_b200 import api, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def test_chunks_shrink_to_the_memory_there_is(built):
+    d1, _, _, cam = synth.render_pair(61, "640x480")
+    n = 140
+    ctx = api.Context(0)
+    proj, conv = converter(cam, ctx)
+    want = api.Cloud(ctx)
+    conv.compute(want, d1)
+    w = want.download()
+    clouds = [api.Cloud(ctx) for _ in range(n)]
+    # room for the clouds (84 bytes a pixel) and 1.7 GB: 59 frames' planes with
+    # their share take 2.06 GB, 39 frames' 1.4
+    left = n * (84 * 307200 + (1 << 21)) + int(1.7e9)
+    torch.cuda.empty_cache()
+    fill = torch.cuda.mem_get_info()[0] - left
+    assert fill > 0
+    held = torch.empty(fill, dtype=torch.uint8, device="cuda")
+    try:
+        api.build_batch(ctx, [d1] * n, [proj.camera()] * n, conv.params(), clouds)
+        ctx.synchronize()
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    for k in (0, 8, 9, 66, 67, 139):
+        got = clouds[k].download()
+        for key in ("points", "normals", "curvature"):
+            assert np.array_equal(got[key], w[key]), (k, key)
+    del clouds, want
+    ctx.close()
