@@ -53,7 +53,7 @@ struct nicp_ctx {
   cudaStream_t fork_stream[kMaxParts - 1] = {};  // the other branches of a captured, forked loop
   cudaEvent_t fork_ev[kMaxParts] = {};
   PinnedBlock pin_down;
-  HostCopier copier;                    // copies into pageable host memory
+  HostCopier copier;                    // copies into the caller's host memory
   size_t cloud_bytes = 0;
   std::vector<GraphEntry> graphs;
   nicp_cloud *scratch_cloud = nullptr;
@@ -1497,7 +1497,10 @@ struct NNPlan {
 // read-back), then the grid: cell h = kNNCell cbrt(volume / points), at least
 // 1 mm, at most 2^24 cells.  The points lie on surfaces: at 320x240 a point's
 // cell holds about 20.  0.35 / 0.5 / 0.7 / 1.0 / 1.4 measured 1.31 / 1.19 /
-// 1.10 / 1.37 / 1.49 ms per 10-iteration alignment there.
+// 1.10 / 1.37 / 1.49 ms per 10-iteration alignment there.  (Volumes and planes
+// of 300 to 40 k points, and a plane with one point 500 m away, whose cells then
+// hold thousands, take 0.2 to 0.7 of what one thread per point over cells of the
+// mean spacing took.)
 constexpr double kNNCell = 0.7;
 int nn_plan(nicp_ctx *ctx, const nicp_cloud *ref, const nicp_cloud *cur, NNPlan &pl) {
   int rc;

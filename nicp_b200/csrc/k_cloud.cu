@@ -529,8 +529,8 @@ __global__ void __launch_bounds__(128) k_moments_band_carry(const FrameDev *__re
 // CTA of four warps that scanned one row at a time, all ten planes, with the
 // running sums in shared memory moved each value through shared memory three
 // times (now twice, 16 bytes at once) behind five barriers per row (now ten per
-// segment) and kept its 128 threads whatever the width: 1717 -> 1191 us for 200
-// frames of 640x480, 112 -> 58 for 9, 2519 -> 1275 for 384 of three sizes down to
+// segment) and kept its 128 threads whatever the width: 1717 -> 1194 us for 200
+// frames of 640x480, 112 -> 62 for 9, 2519 -> 1186 for 384 of three sizes down to
 // 160x120.  Half the rows at a time with 3 CTAs of 256 threads: 1287, 74, 1314;
 // a CTA per plane pair: 1759 to 2199 for the 200.
 constexpr int kSweepThreads = 32 * kBandRows;
@@ -627,7 +627,7 @@ __device__ __forceinline__ void sweep_pair(SweepSmem<M> &sm, const FrameDev &f, 
 // descriptors; CTAs past a smaller frame's last band return at once.  only: the
 // plane pair to write, all five if negative -- the launch writes all, but with
 // a condition on each the compiler keeps to 64 registers; five in a row share
-// offsets and conversions and spill 1.3 KB (1330 us instead of 1191).
+// offsets and conversions and spill 1.3 KB (1330 us instead of 1194).
 template <class M>
 __global__ void __launch_bounds__(kSweepThreads, 2) k_moments_band_sweep(const FrameDev *__restrict__ frames, int only) {
   typedef typename MomAcc<M>::T A;

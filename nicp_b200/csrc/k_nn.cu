@@ -4,19 +4,21 @@
 // The reference asks FLANN's randomized kd-tree (approximate, 16 checks) for
 // the nearest current point within the squared radius in the 6-D space
 // (p, s n).  Here the search is exact: the current cloud is bucketed in a
-// uniform grid over xyz (cell h); a query scans Chebyshev shells of cells
-// around its own cell and stops once the shell's lower bound on the xyz
-// distance -- a lower bound of the 6-D distance -- exceeds the best squared
-// distance found (or the radius).  Ties keep the lowest current index, as the
-// oracle's exhaustive scan does, so the order of a cell's points is free.
+// uniform grid over xyz (cell h); a query searches a box of cells around its
+// own whose half-width doubles (1, 2, 4, ... cells) and stops once the lower
+// bound on the xyz distance to anything outside the box -- a lower bound of the
+// 6-D distance -- exceeds the best squared distance found (or the radius).  Ties
+// keep the lowest current index, as the oracle's exhaustive scan does, so the
+// order of a cell's points is free.
 //
 //   k_nn_bounds    bounding box of the current cloud
 //   k_nn_count     per current point: its cell, its rank in the cell
 //   (CUB scan of the cell counts: the first point of every cell)
 //   k_nn_scatter   positions, scaled normals and indices in cell order
-//   k_nn_query     per reference point: transform, shell search, the
-//                  reference's gates; match[i] = current index or -1
-//   k_nn_far       the points that need a wide search, a warp each
+//   k_nn_query     eight lanes per reference point: transform, the boxes up to
+//                  kNNNear cells, the reference's gates; match[i] = current
+//                  index or -1
+//   k_nn_far       the points that need a wider search, a CTA each
 //   k_nn_pairs     ordered compaction into (ref, cur) pairs
 #include <cuda_runtime.h>
 
@@ -34,7 +36,8 @@ namespace nicp {
 constexpr int kNNThreads = 256;
 // Box half-width (cells, a power of two) up to which eight lanes search before
 // a CTA takes over: 2 against 4 measured 1.10 / 1.41 ms per 10-iteration
-// alignment at 320x240 (cells of 0.7 of the mean spacing, see nn_plan).
+// alignment at 320x240 (cells of 0.7 of the mean spacing, see nn_plan).  Both
+// are from rooms of that size; the result does not depend on them.
 constexpr int kNNNear = 2;
 constexpr int kNNFarBlocks = 4 * 148;  // CTAs of the wide search: about what fits at once
 constexpr int kRuns = 4;               // runs of points in flight per group of lanes
