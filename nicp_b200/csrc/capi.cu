@@ -2059,6 +2059,7 @@ static void enqueue_loop(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall &a, 
 // grids), the pinned addresses of the input and the results, the options.
 static std::string graph_key(nicp_ctx *ctx, const LoopPlan &pl, const AlignCall &a) {
   std::string k;
+  k.reserve(512);
   auto put = [&](const void *p, size_t n) { k.append((const char *)p, n); };
   put(&ctx->ws, sizeof(ctx->ws));
   for (const void *p : {(const void *)a.begin.pairs, (const void *)a.begin.krt, (const void *)a.begin.guess,
@@ -2162,7 +2163,14 @@ static int autotune_loop(nicp_ctx *ctx, const PairPlan &pl, const AlignCall &a, 
 // launches in flight -- the block is not filled again before they are done.
 struct PinUpInUse {
   nicp_ctx *ctx;
-  ~PinUpInUse() { cudaEventRecord(ctx->pin_up_ev, ctx->stream); }
+  cudaError_t release() {  // (behind the loop, before the host waits for it)
+    nicp_ctx *c = ctx;
+    ctx = nullptr;
+    return cudaEventRecord(c->pin_up_ev, c->stream);
+  }
+  ~PinUpInUse() {
+    if (ctx) release();
+  }
 };
 
 static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
@@ -2203,7 +2211,7 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
   size_t up = sizeof(PairDev) * a.n + 48 * (size_t)a.n + 256 * (size_t)a.n;
   char *pin;
   if ((rc = pin_up(ctx, up, &pin))) return rc;
-  const PinUpInUse in_use{ctx};
+  PinUpInUse in_use{ctx};
   PairDev *pd = (PairDev *)pin;
   fill_pairs(ctx, pl, a.cams, big.data(), a.curs, pd);
   for (int i = 0; i < a.n; i++) {
@@ -2290,6 +2298,7 @@ static int align_impl(nicp_ctx *ctx, AlignCall a, nicp_align_result *out) {
     enqueue_loop(ctx, pl, a, false);
   }
   CK(ctx, cudaGetLastError());
+  CK(ctx, in_use.release());
   ctx->d2h_bytes += sizeof(PairState) * (unsigned long long)a.n;
   CK(ctx, cudaStreamSynchronize(s));
   const PairState *st = (const PairState *)res;
