@@ -39,7 +39,9 @@
  *     forced to (0 0 0 1) as the reference does.
  *   - Host buffers are caller-owned; device buffers (clouds, scratch) are
  *     owned by the library.  Calls on one context are ordered on its CUDA
- *     stream; functions that return data in host memory synchronize it.
+ *     stream; functions that return data in host memory synchronize it.  A
+ *     destination in page-locked memory is written by one transfer; one in
+ *     device memory is refused (NICP_ECUDA).
  *   - Cloud builds from host depth (nicp_cloud_from_depth_*, nicp_build_batch
  *     with on_device 0) return before the frames are copied when nothing is
  *     returned in host memory: keep pinned host frames valid until the
@@ -160,7 +162,7 @@ typedef struct {
 
 /* Aligner (aligner.cpp:21-41) plus the device-loop controls. */
 typedef struct {
-  int outer_iterations, inner_iterations;
+  int outer_iterations, inner_iterations; /* 0 outer: T is the guess, the statistics those of an empty list */
   float lambda;
   int min_inliers;
   float translational_min_eigen_ratio, rotational_min_eigen_ratio;
@@ -263,7 +265,8 @@ int nicp_cloud_download_stats(nicp_cloud *cloud, float *eigval3, float *eigvec9,
 
 /* Any output may be NULL.  points4/normals4: n*4 floats (w = 1 / 0);
  * curvature: n; omega_p9/omega_n9: n*9 (3x3 blocks); eigval3: n*3;
- * eigvec9: n*9 (columns are eigenvectors; needs keep_stats).
+ * eigvec9: n*9 (columns are eigenvectors; needs keep_stats).  Large clouds
+ * come in pieces: the context's workspace does not grow with them.
  * A cloud built with information matrices of the form U diag(d0, d1, d1) U^T
  * and without keep_stats holds them implicitly (d1 I + (d0 - d1) n n^T from
  * its float normal, evaluated in double and rounded once); the first call
