@@ -25,7 +25,10 @@ def test_chunks_shrink_to_the_memory_there_is(built):
     torch.cuda.empty_cache()
     fill = torch.cuda.mem_get_info()[0] - left
     assert fill > 0
-    held = torch.empty(fill, dtype=torch.uint8, device="cuda")
+    try:
+        held = torch.empty(fill, dtype=torch.uint8, device="cuda")
+    except torch.OutOfMemoryError:
+        pytest.skip("the free memory cannot be had in one block")
     try:
         api.build_batch(ctx, [d1] * n, [proj.camera()] * n, conv.params(), clouds)
         ctx.synchronize()
